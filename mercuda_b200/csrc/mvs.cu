@@ -8,9 +8,10 @@
 #include "mvs_device.cuh"
 
 // Minimum resident CTAs per SM requested from ptxas for the particle kernel
-// (bounds its registers per thread at 65536 / (128 * this)).
+// (bounds its registers per thread at 65536 / (128 * this)). 1M particles, 16
+// steps: 0.90 ms a launch with 5 (96 registers), 0.885 with 6 (80), 0.89 with 7.
 #ifndef MB200_PARTICLE_MIN_BLOCKS
-#define MB200_PARTICLE_MIN_BLOCKS 5
+#define MB200_PARTICLE_MIN_BLOCKS 6
 #endif
 
 namespace mb200 {
@@ -27,6 +28,13 @@ __device__ __forceinline__ void st3(double* p, int stride, int k, double3 v) {
     p[k] = v.x;
     p[stride + k] = v.y;
     p[2 * stride + k] = v.z;
+}
+
+// The order of doubles on integers: a >= b implies order_key(a) >= order_key(b)
+// - 1 (only the high words count; the 1 is for -0 >= +0).
+__device__ __forceinline__ int order_key(double x) {
+    const int hi = __double2hiint(x);
+    return hi ^ ((hi >> 31) & 0x7fffffff);
 }
 
 // ------------------------------------------------------------ Big bodies
@@ -341,6 +349,8 @@ __device__ void big_run(const MvsBigArgs& A, double* smem) {
             box_extent(S.X0[N + k], S.X[N + k], S.V0[N + k], S.V[N + k], h, lo, hi);
             b[6] = lo - pad;
             b[7] = hi + pad;
+            reinterpret_cast<int4*>(row + TAB_HEAD + TAB_BODY * nb)[k - 1] =
+                make_int4(order_key(b[4]) - 1, order_key(b[5]), order_key(b[6]) - 1, order_key(b[7]));
             double* d = det + (k - 1) * TAB_DETAIL;
             for (int c = 0; c < 3; ++c) {
                 d[c] = S.X0[c * N + k];
@@ -459,222 +469,320 @@ __device__ __forceinline__ int claim_slot(bool has, int cap, DeviceStatus* st, i
     return slot;
 }
 
-// Thread-private shared-memory columns of the particle kernel, one double per
+// Thread-private shared-memory columns of the particle kernels, one double per
 // thread per column (column-major, so the lanes of a warp hit distinct banks).
-// Only x, v and the cached acceleration of the particle being advanced live in
-// registers; its constants, its pre-drift state and the second particle of the
-// thread's pair wait here, which keeps the drift's register footprint small.
-struct Cols {
-    static constexpr int PARK = 0;     // 9: x, v, acc of the waiting particle
-    static constexpr int RCE = 9;      // 2: per particle of the pair
-    static constexpr int RPHYS = 11;   // 2
-    static constexpr int MASS = 13;    // 2
-    static constexpr int X0 = 15;      // 3: state after the first kick
-    static constexpr int V0 = 18;      // 3
-    static constexpr int CEN = 21;     // 4: mce_cent start quantities
-    static constexpr int NGF = 25;     // 10: five coefficients per particle
-    static constexpr int count(bool ngf) { return ngf ? 35 : 25; }
+// Only x, v, the cached acceleration and |x|^2 live in registers; what a step
+// needs again after the drift waits here, which keeps the drift's register
+// footprint small.
+template <int STRIDE_> struct ColsOf {
+    static constexpr int X0 = 0;       // 3: state after the first kick
+    static constexpr int V0 = 3;       // 3
+    static constexpr int VS = 6;       // 3: velocity at the start of the step (mce_cent)
+    static constexpr int PAD = 9;      // 1.2 rce, mce_stat's margin
+    static constexpr int NGF = 10;     // 5 coefficients
+    __host__ __device__ static constexpr int count(bool ngf) { return ngf ? 15 : 10; }
     // column stride: the kernel's largest CTA, so that a column offset is a
     // constant (base already points at the thread's own entry)
-    static constexpr int STRIDE = 128;
+    static constexpr int STRIDE = STRIDE_;
     volatile double* base;
     __device__ volatile double& at(int c) const { return base[c * STRIDE]; }
     __device__ double3 ld3(int c) const { return make_double3(at(c), at(c + 1), at(c + 2)); }
     __device__ void st3(int c, double3 v) const { at(c) = v.x; at(c + 1) = v.y; at(c + 2) = v.z; }
 };
 
-// small_body_force with the coefficients of pair member u in the columns.
-template <bool NGF, bool OBL>
-__device__ __forceinline__ double3 particle_force(const double3 x, const double3 v_ngf, const Cols& cols, int u,
-                                                  const double* T, int nb, const double* jcen, double mu,
-                                                  DeviceStatus* st) {
-    return small_body_force<NGF, OBL>(x, v_ngf, [&](int c) -> double { return cols.at(Cols::NGF + 5 * u + c); }, T,
-                                      nb, jcen, mu, st);
+using Cols = ColsOf<128>;
+
+// A particle between steps: what the next step takes from the one before.
+struct Particle {
+    double3 x, v, acc;
+    double rr;          // |x|^2
+    int kx, ky;         // order_key of x.x and x.y
+    int rv;             // high word of x.v
+    bool padded;        // rce != 0
+    __device__ void derive() {
+        rr = x.x * x.x + x.y * x.y + x.z * x.z;
+        kx = order_key(x.x);
+        ky = order_key(x.y);
+        rv = __double2hiint(v.x * x.x + v.y * x.y + v.z * x.z);
+    }
+};
+
+// What a step needs of its system.
+struct StepEnv {
+    double mu, rmu, h, hby2, rcen;
+    int nb;
+};
+
+// Keys of a coordinate's extent over the step when the velocity turns within
+// it (mce_box then adds the interpolated turning point) or the body has a
+// margin of its own: an interval that contains mce_box's. The turning point is
+// within |a1 - a0| + |h| min(|u0|, |u1|) / 2 of an end, without the division
+// (1/16 more covers the roundings).
+__device__ __forceinline__ void wide_keys(double a0, double a1, double u0, double u1, double h, double pad, int& klo,
+                                          int& khi) {
+    double e = pad;
+    if ((__double2hiint(u0) ^ __double2hiint(u1)) < 0)
+        e = e + 1.0625 * (fabs(a1 - a0) + 0.5 * fabs(h) * fmin(fabs(u0), fabs(u1)));
+    klo = order_key(fmin(a0, a1) - e) - 1;
+    khi = order_key(fmax(a0, a1) + e);
 }
 
-// One mdt_mvs step of one Small body (slot p, pair member u) against the staged
-// table T of step s.
-template <bool NGF, bool OBL, bool CENTRAL>
-__device__ __forceinline__ void particle_step(double3& x, double3& v, double3& acc, bool ok, int p, int u,
-                                              const Cols& cols, const double* T, int s, const MvsParticleArgs& A,
-                                              double hby2, double hm1) {
-    const int nb = A.nb;
-    const double h = A.h;
-    double bxlo = 0.0, bxhi = 0.0, bylo = 0.0, byhi = 0.0;
+// The bodies of keys[0 .. n), n <= 32, whose box may overlap [kxlo, kxhi] x
+// [kylo, kyhi], as a bit mask. Four compares chained through one predicate and
+// one predicated OR a body.
+__device__ __forceinline__ unsigned overlap_mask(const int4* keys, int n, int kxlo, int kxhi, int kylo, int kyhi) {
+    unsigned mask = 0;
+    auto test = [&](int b, unsigned bit) {
+        const int4 k = keys[b];
+        asm("{\n\t.reg .pred p;\n\t"
+            "setp.ge.s32 p, %1, %2;\n\t"
+            "setp.ge.and.s32 p, %3, %4, p;\n\t"
+            "setp.ge.and.s32 p, %5, %6, p;\n\t"
+            "setp.ge.and.s32 p, %7, %8, p;\n\t"
+            "@p or.b32 %0, %0, %9;\n\t}"
+            : "+r"(mask)
+            : "r"(k.y), "r"(kxlo), "r"(kxhi), "r"(k.x), "r"(k.w), "r"(kylo), "r"(kyhi), "r"(k.z), "r"(bit));
+    };
+    if (n == 8) {   // the usual planetary system, without a loop
+#pragma unroll
+        for (int b = 0; b < 8; ++b) test(b, 1u << b);
+    } else {
+#pragma unroll 1
+        for (int b = 0; b < n; ++b) test(b, 1u << b);
+    }
+    return mask;
+}
+
+// One mdt_mvs step of one Small body: kick, Kepler drift, mce_stat's box
+// screen, interaction force, kick, mce_cent. T holds the step's head, the
+// bodies' force rows (ROW doubles apart) and their box keys; G the table row
+// with the exact boxes. found(b, P, x0, v0) is called by the whole warp for
+// each body with the lanes whose exact boxes overlap, struck(hit, time) once a
+// step.
+//
+// The screens run in two passes. The first compares integers: order_key()
+// keeps the order of doubles by their high words (a >= b implies key(a) >=
+// key(b) - 1), and x at the step's start, |x|^2 and x.v come from the step
+// before. What passes is tested with mce_box's and mce_cent's own statements.
+// The kernel issues an FP64 instruction every other cycle and another kind in
+// between (on particles that all take drift_kepmd's path it fits 1.8 cycles
+// for each FP64 instruction and 1.4 for any other), so both kinds count. Per
+// warp-step, 8 planets: 563 FP64 of 1,138 instructions with exact boxes
+// compared on the FP64 pipe and IEEE division calls, 497 of 944 so; 1M
+// particles, 16 steps: 1.19 ms a launch before, 0.75 now, and with the
+// benchmark's mixture of orbits 1.52 ms and 0.89.
+template <bool NGF, bool OBL, bool CENTRAL, int ROW, class Cols, class Found, class Struck>
+__device__ __forceinline__ void particle_step(Particle& P, bool ok, const Cols& cols, const double* T,
+                                              const double* G, const StepEnv& E, const double* jcen,
+                                              DeviceStatus* status, double mass, Found&& found, Struck&& struck) {
+    double3& x = P.x;
+    double3& v = P.v;
+    const int nb = E.nb;
+    const double h = E.h;
+    int kxlo = 0, kxhi = 0, kylo = 0, kyhi = 0;
+    const int rr0 = __double2hiint(P.rr), rv0 = P.rv;
     if (ok) {
-        if (CENTRAL) {
-            const CentralStart c = central_start(x, v);
-            cols.at(Cols::CEN) = c.rr0;
-            cols.at(Cols::CEN + 1) = c.rv0;
-            cols.at(Cols::CEN + 2) = c.h2;
-            cols.at(Cols::CEN + 3) = c.v2;
-        }
-        v.x = v.x + hby2 * acc.x;
-        v.y = v.y + hby2 * acc.y;
-        v.z = v.z + hby2 * acc.z;
+        if (CENTRAL) cols.st3(Cols::VS, v);
+        v.x = v.x + E.hby2 * P.acc.x;
+        v.y = v.y + E.hby2 * P.acc.y;
+        v.z = v.z + E.hby2 * P.acc.z;
+        const int ux = __double2hiint(v.x), uy = __double2hiint(v.y);
         cols.st3(Cols::X0, x);
         cols.st3(Cols::V0, v);
-        drift_one(A.mu, x, v, h);
-        box_extent(cols.at(Cols::X0), x.x, cols.at(Cols::V0), v.x, h, bxlo, bxhi);
-        box_extent(cols.at(Cols::X0 + 1), x.y, cols.at(Cols::V0 + 1), v.y, h, bylo, byhi);
-        const double pad = cols.at(Cols::RCE + u) * 1.2;
-        bxlo = bxlo - pad;
-        bxhi = bxhi + pad;
-        bylo = bylo - pad;
-        byhi = byhi + pad;
+        drift_one(E.mu, E.rmu, x, v, h, P.rr);
+        P.rr = x.x * x.x + x.y * x.y + x.z * x.z;
+        const int kx = order_key(x.x), ky = order_key(x.y);
+        kxlo = min(P.kx, kx) - 1;
+        kxhi = max(P.kx, kx);
+        kylo = min(P.ky, ky) - 1;
+        kyhi = max(P.ky, ky);
+        P.kx = kx;
+        P.ky = ky;
+        if ((ux ^ __double2hiint(v.x)) < 0 || P.padded)
+            wide_keys(cols.at(Cols::X0), x.x, cols.at(Cols::V0), v.x, h, cols.at(Cols::PAD), kxlo, kxhi);
+        if ((uy ^ __double2hiint(v.y)) < 0 || P.padded)
+            wide_keys(cols.at(Cols::X0 + 1), x.y, cols.at(Cols::V0 + 1), v.y, h, cols.at(Cols::PAD), kylo, kyhi);
     }
-    // mce_stat against each Big body; the loop is uniform across the warp.
-#pragma unroll 1
-    for (int b = 0; b < nb; ++b) {
-        const double* row = T + TAB_HEAD + b * TAB_BODY;
-        const bool cand = ok && row[5] >= bxlo && bxhi >= row[4] && row[7] >= bylo && byhi >= row[6];
-        if (__any_sync(FULL, cand)) {
-            const int slot = claim_slot(cand, A.cand_cap, A.status, &A.status->cands, 2);
-            if (slot >= 0) {
-                EncounterCandidate* c = A.cands + slot;
-                *reinterpret_cast<int4*>(c) = make_int4(p, b, A.step0 + s, A.nbig + A.perm[p] + 1);
-                double2* w = reinterpret_cast<double2*>(c);
-                w[1] = make_double2(cols.at(Cols::RCE + u), cols.at(Cols::RPHYS + u));
-                w[2] = make_double2(cols.at(Cols::X0), cols.at(Cols::X0 + 1));
-                w[3] = make_double2(cols.at(Cols::X0 + 2), cols.at(Cols::V0));
-                w[4] = make_double2(cols.at(Cols::V0 + 1), cols.at(Cols::V0 + 2));
-                w[5] = make_double2(x.x, x.y);
-                w[6] = make_double2(x.z, v.x);
-                w[7] = make_double2(v.y, v.z);
-            }
+    for (int b0 = 0; b0 < nb; b0 += 32) {
+        const int4* keys = reinterpret_cast<const int4*>(T + TAB_HEAD + ROW * nb) + b0;
+        unsigned maybe = overlap_mask(keys, min(32, nb - b0), kxlo, kxhi, kylo, kyhi);
+        if (!ok) maybe = 0;
+        unsigned any = __reduce_or_sync(FULL, maybe);
+        if (any == 0) continue;
+        double bxlo = 0.0, bxhi = 0.0, bylo = 0.0, byhi = 0.0;
+        const double3 x0 = cols.ld3(Cols::X0), v0 = cols.ld3(Cols::V0);
+        if (maybe) {
+            box_extent(x0.x, x.x, v0.x, v.x, h, bxlo, bxhi);
+            box_extent(x0.y, x.y, v0.y, v.y, h, bylo, byhi);
+            const double pad = cols.at(Cols::PAD);
+            bxlo = bxlo - pad;
+            bxhi = bxhi + pad;
+            bylo = bylo - pad;
+            byhi = byhi + pad;
         }
+        do {
+            const int b = __ffs(any) - 1;
+            any &= any - 1;
+            const double* row = G + TAB_HEAD + (b0 + b) * TAB_BODY;
+            found(((maybe >> b) & 1u) && row[5] >= bxlo && bxhi >= row[4] && row[7] >= bylo && byhi >= row[6], b0 + b,
+                  x0, v0);
+        } while (any);
     }
     if (ok) {
-        acc = particle_force<NGF, OBL>(x, v, cols, u, T, nb, A.jcen, A.mu, A.status);
-        v.x = v.x + hby2 * acc.x;
-        v.y = v.y + hby2 * acc.y;
-        v.z = v.z + hby2 * acc.z;
+        P.acc = small_body_force<NGF, OBL, ROW>(
+            x, v, [&](int c) -> double { return cols.at(Cols::NGF + c); }, T, nb, jcen, E.mu, status);
+        v.x = v.x + E.hby2 * P.acc.x;
+        v.y = v.y + E.hby2 * P.acc.y;
+        v.z = v.z + E.hby2 * P.acc.z;
     }
     if (CENTRAL) {
+        // mce_cent's first test, (rv0 h <= 0 and rv1 h >= 0) or min |x|^2 <=
+        // rcen^2, on high words: signs, with numbers that a product with h
+        // could flush to zero (below 2^-767) counted as both
+        P.rv = __double2hiint(v.x * x.x + v.y * x.y + v.z * x.z);
+        const int hs = __double2hiint(h) & 0x80000000;
         double temp = 0.0;
         bool hit = false;
-        if (ok) {
-            const CentralStart c{cols.at(Cols::CEN), cols.at(Cols::CEN + 1), cols.at(Cols::CEN + 2),
-                                 cols.at(Cols::CEN + 3)};
-            hit = central_finish(c, x, v, A.mu, cols.at(Cols::MASS + u), h, A.rcen, temp);
+        if (ok && (((rv0 ^ hs) < 0x10000000 && (unsigned)(P.rv ^ hs) < 0x90000000u) ||
+                   min(rr0, __double2hiint(P.rr)) <= __double2hiint(E.rcen * E.rcen) || fabs(h) < 1e-60)) {
+            // a pericentre inside rcen needs |x0 x v0|^2 <= rcen^2 (v0^2 - 2 M
+            // / r0) + 2 M rcen (the speed an orbit has at rcen): most passages
+            // end here, without the square roots and divisions of the rest
+            const CentralStart c = central_start(cols.ld3(Cols::X0), cols.ld3(Cols::VS));
+            const double rcen2 = E.rcen * E.rcen;
+            if (c.rr0 <= rcen2 || c.h2 <= 1.001 * (rcen2 * c.v2 + 2.0 * (E.mu + mass) * E.rcen))
+                hit = central_finish(c, x, v, E.mu, mass, h, E.rcen, temp);
         }
-        const int slot = claim_slot(hit, A.event_cap, A.status, &A.status->events, 1);
-        if (slot >= 0) {
-            MercuryEvent* e = A.events + slot;
-            *reinterpret_cast<int4*>(e) = make_int4(1, A.nbig + A.perm[p] + 1, EV_CENTRAL, 0);
-            reinterpret_cast<double2*>(e)[1] = make_double2(A.rcen, temp);
-            // a central-body record carries no states (xi = xj = 0)
-            for (int k = 2; k < 8; ++k) reinterpret_cast<double2*>(e)[k] = make_double2(0.0, 0.0);
-            A.event_step[slot] = A.step0 + s;
-        }
+        struck(hit, temp);
     }
 }
 
-// Test-particle kernel: each thread owns a pair of adjacent particle slots (one
-// double2 per state component), advances the first through all K steps while
-// the second waits in shared memory, then the second; the Big-body tables of
-// the K steps are staged in shared memory once per CTA.
+// A central-body record (it carries no states: xi = xj = 0).
+__device__ __forceinline__ void central_record(MercuryEvent* e, int id, double rcen, double temp) {
+    *reinterpret_cast<int4*>(e) = make_int4(1, id, EV_CENTRAL, 0);
+    reinterpret_cast<double2*>(e)[1] = make_double2(rcen, temp);
+    for (int k = 2; k < 8; ++k) reinterpret_cast<double2*>(e)[k] = make_double2(0.0, 0.0);
+}
+__device__ __forceinline__ void candidate_record(EncounterCandidate* c, int4 head, double rce, double rphys,
+                                                 double3 x0, double3 v0, double3 x, double3 v) {
+    *reinterpret_cast<int4*>(c) = head;
+    double2* w = reinterpret_cast<double2*>(c);
+    w[1] = make_double2(rce, rphys);
+    w[2] = make_double2(x0.x, x0.y);
+    w[3] = make_double2(x0.z, v0.x);
+    w[4] = make_double2(v0.y, v0.z);
+    w[5] = make_double2(x.x, x.y);
+    w[6] = make_double2(x.z, v.x);
+    w[7] = make_double2(v.y, v.z);
+}
+
+// Rows of the Big bodies staged in shared memory: a table row without the
+// exact boxes, {head, x y z m per body, box keys}.
+constexpr int SROW_BODY = 4;
+__host__ __device__ constexpr int srow_stride(int nb) { return TAB_HEAD + (SROW_BODY + TAB_KEYS) * nb; }
+
+// Test-particle kernel: one particle slot per thread through all K steps; the
+// Big-body rows of the K steps are staged in shared memory once per CTA.
+//
+// One slot per thread, not two: a warp's time on a tile is the time of its
+// slowest particle, and a tile of particles that need the universal-variable
+// drift takes several times an ordinary one. With two particles in turn in
+// each thread such a tile alone took the whole launch (1M particles, 16 steps: 1.52 ms of a
+// 1.52 ms launch; one slot a thread, 0.97 ms).
 template <bool NGF, bool OBL, bool CENTRAL>
 __global__ void __launch_bounds__(128, MB200_PARTICLE_MIN_BLOCKS) mvs_particle_kernel(MvsParticleArgs A) {
     extern __shared__ double smem[];
-    const int nb = A.nb, stride = tab_stride(nb);
+    const int nb = A.nb, gstride = tab_stride(nb), stride = srow_stride(nb);
     const int rows = A.nsteps + (A.reset ? 1 : 0);
     double* stab = smem;
     const Cols cols{smem + (size_t)rows * stride + threadIdx.x};
-    const double* gtab = A.tab + (A.reset ? 0 : stride);
-    for (int k = threadIdx.x; k < rows * stride; k += blockDim.x) stab[k] = gtab[k];
+    const double* gtab = A.tab + (A.reset ? 0 : gstride);
+    {
+        // 16 bytes at a time: unit u of a staged row is the head's, a body's
+        // half force row or a body's keys
+        const int units = stride / 2, gunits = gstride / 2;
+        const double2* src = reinterpret_cast<const double2*>(gtab);
+        double2* dst = reinterpret_cast<double2*>(stab);
+        for (int k = threadIdx.x; k < rows * units; k += blockDim.x) {
+            const int r = k / units, u = k - r * units, q = u - TAB_HEAD / 2;
+            const int g = q < 0 ? u : q < 2 * nb ? TAB_HEAD / 2 + (q >> 1) * (TAB_BODY / 2) + (q & 1)
+                                                 : TAB_HEAD / 2 + nb * (TAB_BODY / 2) + (q - 2 * nb);
+            dst[k] = src[(size_t)r * gunits + g];
+        }
+    }
     __syncthreads();
     const double* steps_tab = stab + (A.reset ? stride : 0);
-    const double hby2 = 0.5 * A.h, hm1 = 1.0 / A.h;
+    const double* steps_gtab = A.tab + gstride;
+    const StepEnv E{A.mu, A.rmu, A.h, 0.5 * A.h, A.rcen, nb};
     const int lane = threadIdx.x & 31;
-    const int npairs = (A.np + 1) >> 1;
-    // Warps claim 32-pair tiles from a launch-wide counter: slots are ordered
+    // Warps claim tiles of 32 slots from a launch-wide counter: slots are ordered
     // slowest-first (Newton-path particles lead), so claiming dynamically
     // balances the SMs (longest-processing-time-first).
-    const int ntiles = (npairs + 31) >> 5;
-    const int S = A.npcap, H = S / 2;
-    const double2* in = reinterpret_cast<const double2*>(A.xin);
-    double2* out = reinterpret_cast<double2*>(A.xout);
+    const int ntiles = (A.np + 31) >> 5;
+    const size_t S = A.npcap;
     int* const tiles = A.tiles ? A.tiles : &A.status->next_tile;
     for (;;) {
         int tile = 0;
         if (lane == 0) tile = atomicAdd(tiles, 1);
         tile = __shfl_sync(FULL, tile, 0);
         if (tile >= ntiles) break;
-        const int pair = tile * 32 + lane;
-        const bool live = pair < npairs;
-        const int j0 = 2 * pair;
-        double3 x, v, acc;
-        if (live) {
-            double2 t[9];
-#pragma unroll
-            for (int c = 0; c < 9; ++c) t[c] = in[c * H + pair];
-            x = make_double3(t[0].x, t[1].x, t[2].x);
-            v = make_double3(t[3].x, t[4].x, t[5].x);
-            acc = make_double3(t[6].x, t[7].x, t[8].x);
-#pragma unroll
-            for (int c = 0; c < 9; ++c) cols.at(Cols::PARK + c) = t[c].y;
-            const double2 rc = reinterpret_cast<const double2*>(A.rce)[pair];
-            const double2 rp = reinterpret_cast<const double2*>(A.rphys)[pair];
-            const double2 ms = reinterpret_cast<const double2*>(A.m)[pair];
-            cols.at(Cols::RCE) = rc.x; cols.at(Cols::RCE + 1) = rc.y;
-            cols.at(Cols::RPHYS) = rp.x; cols.at(Cols::RPHYS + 1) = rp.y;
-            cols.at(Cols::MASS) = ms.x; cols.at(Cols::MASS + 1) = ms.y;
+        const int p = tile * 32 + lane;
+        const bool ok = p < A.np;
+        Particle P{};
+        if (ok) {
+            const double* in = A.xin + p;
+            P.x = make_double3(in[0], in[S], in[2 * S]);
+            P.v = make_double3(in[3 * S], in[4 * S], in[5 * S]);
+            P.acc = make_double3(in[6 * S], in[7 * S], in[8 * S]);
+            const double pad = A.rce[p] * 1.2;
+            cols.at(Cols::PAD) = pad;
+            P.padded = pad != 0.0;
             if (NGF)
-                for (int c = 0; c < 5; ++c) {
-                    const double2 g = reinterpret_cast<const double2*>(A.ngf + (size_t)c * S)[pair];
-                    cols.at(Cols::NGF + c) = g.x;
-                    cols.at(Cols::NGF + 5 + c) = g.y;
-                }
+                for (int c = 0; c < 5; ++c) cols.at(Cols::NGF + c) = A.ngf[c * S + p];
+            if (A.reset)
+                P.acc = small_body_force<NGF, OBL, SROW_BODY>(
+                    P.x, P.v, [&](int c) -> double { return cols.at(Cols::NGF + c); }, stab, nb, A.jcen, A.mu,
+                    A.status);
+            P.derive();
         }
 #pragma unroll 1
-        for (int u = 0; u < 2; ++u) {
-            const bool ok = live && j0 + u < A.np;
-            if (u == 1 && live) {
-                // the first particle's result waits; the second comes in
-                const double3 px = cols.ld3(Cols::PARK), pv = cols.ld3(Cols::PARK + 3),
-                              pa = cols.ld3(Cols::PARK + 6);
-                cols.st3(Cols::PARK, x);
-                cols.st3(Cols::PARK + 3, v);
-                cols.st3(Cols::PARK + 6, acc);
-                x = px;
-                v = pv;
-                acc = pa;
-            }
-            if (A.reset && ok) acc = particle_force<NGF, OBL>(x, v, cols, u, stab, nb, A.jcen, A.mu, A.status);
-            for (int s = 0; s < A.nsteps; ++s)
-                particle_step<NGF, OBL, CENTRAL>(x, v, acc, ok, j0 + u, u, cols, steps_tab + s * stride, s, A, hby2,
-                                                 hm1);
-        }
-        if (live) {
-            const double3 fx = cols.ld3(Cols::PARK), fv = cols.ld3(Cols::PARK + 3), fa = cols.ld3(Cols::PARK + 6);
-            out[0 * H + pair] = make_double2(fx.x, x.x);
-            out[1 * H + pair] = make_double2(fx.y, x.y);
-            out[2 * H + pair] = make_double2(fx.z, x.z);
-            out[3 * H + pair] = make_double2(fv.x, v.x);
-            out[4 * H + pair] = make_double2(fv.y, v.y);
-            out[5 * H + pair] = make_double2(fv.z, v.z);
-            out[6 * H + pair] = make_double2(fa.x, acc.x);
-            out[7 * H + pair] = make_double2(fa.y, acc.y);
-            out[8 * H + pair] = make_double2(fa.z, acc.z);
+        for (int s = 0; s < A.nsteps; ++s)
+            particle_step<NGF, OBL, CENTRAL, SROW_BODY>(
+                P, ok, cols, steps_tab + s * stride, steps_gtab + (size_t)s * gstride, E, A.jcen, A.status,
+                CENTRAL && ok ? A.m[p] : 0.0,
+                [&](bool cand, int b, double3 x0, double3 v0) {
+                    const int slot = claim_slot(cand, A.cand_cap, A.status, &A.status->cands, 2);
+                    if (slot >= 0)
+                        candidate_record(A.cands + slot, make_int4(p, b, A.step0 + s, A.nbig + A.perm[p] + 1),
+                                         A.rce[p], A.rphys[p], x0, v0, P.x, P.v);
+                },
+                [&](bool hit, double temp) {
+                    const int slot = claim_slot(hit, A.event_cap, A.status, &A.status->events, 1);
+                    if (slot >= 0) {
+                        central_record(A.events + slot, A.nbig + A.perm[p] + 1, A.rcen, temp);
+                        A.event_step[slot] = A.step0 + s;
+                    }
+                });
+        if (ok) {
+            double* out = A.xout + p;
+            out[0] = P.x.x;
+            out[S] = P.x.y;
+            out[2 * S] = P.x.z;
+            out[3 * S] = P.v.x;
+            out[4 * S] = P.v.y;
+            out[5 * S] = P.v.z;
+            out[6 * S] = P.acc.x;
+            out[7 * S] = P.acc.y;
+            out[8 * S] = P.acc.z;
             if (A.rows_x) {
                 // rows in particle order for the copy back to the host
-                const int i0 = A.perm[j0];
-                A.rows_x[3 * (size_t)i0] = fx.x;
-                A.rows_x[3 * (size_t)i0 + 1] = fx.y;
-                A.rows_x[3 * (size_t)i0 + 2] = fx.z;
-                A.rows_v[3 * (size_t)i0] = fv.x;
-                A.rows_v[3 * (size_t)i0 + 1] = fv.y;
-                A.rows_v[3 * (size_t)i0 + 2] = fv.z;
-                if (j0 + 1 < A.np) {
-                    const int i1 = A.perm[j0 + 1];
-                    A.rows_x[3 * (size_t)i1] = x.x;
-                    A.rows_x[3 * (size_t)i1 + 1] = x.y;
-                    A.rows_x[3 * (size_t)i1 + 2] = x.z;
-                    A.rows_v[3 * (size_t)i1] = v.x;
-                    A.rows_v[3 * (size_t)i1 + 1] = v.y;
-                    A.rows_v[3 * (size_t)i1 + 2] = v.z;
-                }
+                const size_t i = 3 * (size_t)A.perm[p];
+                A.rows_x[i] = P.x.x;
+                A.rows_x[i + 1] = P.x.y;
+                A.rows_x[i + 2] = P.x.z;
+                A.rows_v[i] = P.v.x;
+                A.rows_v[i + 1] = P.v.y;
+                A.rows_v[i + 2] = P.v.z;
             }
         }
     }
@@ -805,82 +913,17 @@ __global__ void __launch_bounds__(32) mvs_big_batch_kernel(BatchBigArgs B) {
     big_run(A, smem);
 }
 
-// One mdt_mvs step of one test particle of a batched system against its
-// step table T (the same statements as particle_step).
-template <bool CENTRAL>
-__device__ __forceinline__ void batch_particle_step(double3& x, double3& v, double3& acc, bool ok, int p, int sysid,
-                                                    const BatchSys& S, const double* T, int s,
-                                                    const BatchParticleArgs& A, double rce, double rphys, int id) {
-    const int nb = S.nb;
-    const double h = S.h, hby2 = 0.5 * h;
-    double bxlo = 0.0, bxhi = 0.0, bylo = 0.0, byhi = 0.0;
-    double3 x0 = x, v0 = v;
-    CentralStart c0{0.0, 0.0, 0.0, 0.0};
-    if (ok) {
-        if (CENTRAL) c0 = central_start(x, v);
-        v.x = v.x + hby2 * acc.x;
-        v.y = v.y + hby2 * acc.y;
-        v.z = v.z + hby2 * acc.z;
-        x0 = x;
-        v0 = v;
-        drift_one(S.mu, x, v, h);
-        box_extent(x0.x, x.x, v0.x, v.x, h, bxlo, bxhi);
-        box_extent(x0.y, x.y, v0.y, v.y, h, bylo, byhi);
-        const double pad = rce * 1.2;
-        bxlo = bxlo - pad;
-        bxhi = bxhi + pad;
-        bylo = bylo - pad;
-        byhi = byhi + pad;
-    }
-#pragma unroll 1
-    for (int b = 0; b < nb; ++b) {
-        const double* row = T + TAB_HEAD + b * TAB_BODY;
-        const bool cand = ok && row[5] >= bxlo && bxhi >= row[4] && row[7] >= bylo && byhi >= row[6];
-        if (__any_sync(FULL, cand)) {
-            const int slot = claim_slot(cand, A.cand_cap, A.status, &A.status->cands, 2);
-            if (slot >= 0) {
-                EncounterCandidate* c = A.cands + slot;
-                *reinterpret_cast<int4*>(c) = make_int4(sysid, b, A.step0 + s, id);
-                double2* w = reinterpret_cast<double2*>(c);
-                w[1] = make_double2(rce, rphys);
-                w[2] = make_double2(x0.x, x0.y);
-                w[3] = make_double2(x0.z, v0.x);
-                w[4] = make_double2(v0.y, v0.z);
-                w[5] = make_double2(x.x, x.y);
-                w[6] = make_double2(x.z, v.x);
-                w[7] = make_double2(v.y, v.z);
-            }
-        }
-    }
-    if (ok) {
-        acc = small_body_force<false, false>(x, v, [](int) -> double { return 0.0; }, T, nb, nullptr, S.mu,
-                                             A.status);
-        v.x = v.x + hby2 * acc.x;
-        v.y = v.y + hby2 * acc.y;
-        v.z = v.z + hby2 * acc.z;
-    }
-    if (CENTRAL) {
-        double temp = 0.0;
-        bool hit = false;
-        if (ok) hit = central_finish(c0, x, v, S.mu, 0.0, h, A.rcen, temp);
-        const int slot = claim_slot(hit, A.event_cap, A.status, &A.status->events, 1);
-        if (slot >= 0) {
-            MercuryEvent* e = A.events + slot;
-            *reinterpret_cast<int4*>(e) = make_int4(1, id, EV_CENTRAL, 0);
-            reinterpret_cast<double2*>(e)[1] = make_double2(A.rcen, temp);
-            for (int k = 2; k < 8; ++k) reinterpret_cast<double2*>(e)[k] = make_double2(0.0, 0.0);
-            A.event_step[slot] = A.step0 + s;
-            A.event_sys[slot] = sysid;
-        }
-    }
-    (void)p;
-}
-
 // Every test particle of every system: warps claim 32-slot tiles (each of a
 // single system) from a launch-wide counter and run K steps per particle in
-// registers; the step tables are read through the cache.
-template <bool CENTRAL> __global__ void __launch_bounds__(256) mvs_particle_batch_kernel(BatchParticleArgs A) {
-    const int lane = threadIdx.x & 31, S2 = A.npcap;
+// registers (particle_step above); the step tables are read through the cache.
+template <bool CENTRAL, int THREADS>
+__global__ void __launch_bounds__(THREADS, 128 * MB200_PARTICLE_MIN_BLOCKS / THREADS)
+    mvs_particle_batch_kernel(BatchParticleArgs A) {
+    using Cols = ColsOf<THREADS>;
+    __shared__ double col_mem[THREADS * Cols::count(false)];
+    const Cols cols{col_mem + threadIdx.x};
+    const int lane = threadIdx.x & 31;
+    const size_t S2 = A.npcap;
     for (;;) {
         int tile = 0;
         if (lane == 0) tile = atomicAdd(&A.status->next_tile, 1);
@@ -892,21 +935,50 @@ template <bool CENTRAL> __global__ void __launch_bounds__(256) mvs_particle_batc
         const int p = t.first + (ok ? lane : 0);
         const int stride = tab_stride(S.nb);
         const double* tab = A.tab + S.tab_off;
-        double3 x = ld3(A.xin, S2, p), v = ld3(A.xin + 3 * (size_t)S2, S2, p);
-        double3 acc = ld3(A.xin + 6 * (size_t)S2, S2, p);
-        const double rce = A.rce[p], rphys = A.rphys[p];
-        const int id = S.nbig + A.local[p] + 1;
+        const StepEnv E{S.mu, recip_fix(S.mu, recip_near(S.mu)), S.h, 0.5 * S.h, A.rcen, S.nb};
+        const double* in = A.xin + p;
+        Particle P;
+        P.x = make_double3(in[0], in[S2], in[2 * S2]);
+        P.v = make_double3(in[3 * S2], in[4 * S2], in[5 * S2]);
+        P.acc = make_double3(in[6 * S2], in[7 * S2], in[8 * S2]);
+        const double pad = A.rce[p] * 1.2;
+        cols.at(Cols::PAD) = pad;
+        P.padded = pad != 0.0;
+        auto none = [](int) -> double { return 0.0; };
         if (A.reset && ok)
-            acc = small_body_force<false, false>(x, v, [](int) -> double { return 0.0; }, tab, S.nb, nullptr, S.mu,
-                                                 A.status);
+            P.acc = small_body_force<false, false>(P.x, P.v, none, tab, S.nb, nullptr, S.mu, A.status);
+        P.derive();
 #pragma unroll 1
-        for (int s = 0; s < A.nsteps; ++s)
-            batch_particle_step<CENTRAL>(x, v, acc, ok, p, t.sys, S, tab + (size_t)(s + 1) * stride, s, A, rce,
-                                         rphys, id);
+        for (int s = 0; s < A.nsteps; ++s) {
+            const double* T = tab + (size_t)(s + 1) * stride;
+            particle_step<false, false, CENTRAL, TAB_BODY>(
+                P, ok, cols, T, T, E, nullptr, A.status, 0.0,
+                [&](bool cand, int b, double3 x0, double3 v0) {
+                    const int slot = claim_slot(cand, A.cand_cap, A.status, &A.status->cands, 2);
+                    if (slot >= 0)
+                        candidate_record(A.cands + slot, make_int4(t.sys, b, A.step0 + s, S.nbig + A.local[p] + 1),
+                                         A.rce[p], A.rphys[p], x0, v0, P.x, P.v);
+                },
+                [&](bool hit, double temp) {
+                    const int slot = claim_slot(hit, A.event_cap, A.status, &A.status->events, 1);
+                    if (slot >= 0) {
+                        central_record(A.events + slot, S.nbig + A.local[p] + 1, A.rcen, temp);
+                        A.event_step[slot] = A.step0 + s;
+                        A.event_sys[slot] = t.sys;
+                    }
+                });
+        }
         if (ok) {
-            st3(A.xout, S2, p, x);
-            st3(A.xout + 3 * (size_t)S2, S2, p, v);
-            st3(A.xout + 6 * (size_t)S2, S2, p, acc);
+            double* out = A.xout + p;
+            out[0] = P.x.x;
+            out[S2] = P.x.y;
+            out[2 * S2] = P.x.z;
+            out[3 * S2] = P.v.x;
+            out[4 * S2] = P.v.y;
+            out[5 * S2] = P.v.z;
+            out[6 * S2] = P.acc.x;
+            out[7 * S2] = P.acc.y;
+            out[8 * S2] = P.acc.z;
         }
     }
 }
@@ -940,8 +1012,7 @@ void launch_variant(const MvsParticleArgs& a, cudaStream_t s, int threads) {
     auto kern = mvs_particle_kernel<NGF, OBL, CENTRAL>;
     const size_t smem = mvs_particle_smem(a.nb, a.nsteps, a.reset, threads, NGF);
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int npairs = (a.np + 1) / 2;
-    int tiles = (npairs + threads - 1) / threads;
+    int tiles = (a.np + threads - 1) / threads;
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -958,7 +1029,7 @@ void launch_variant(const MvsParticleArgs& a, cudaStream_t s, int threads) {
 }  // namespace
 
 size_t mvs_particle_smem(int nb, int nsteps, int reset, int threads, bool ngf) {
-    return sizeof(double) * ((size_t)tab_stride(nb) * (size_t)(nsteps + (reset ? 1 : 0)) +
+    return sizeof(double) * ((size_t)srow_stride(nb) * (size_t)(nsteps + (reset ? 1 : 0)) +
                              (size_t)Cols::STRIDE * Cols::count(ngf));
 }
 
@@ -999,21 +1070,20 @@ void launch_mvs_big_batch(const BatchBigArgs& a, int nsys, int max_nbig, cudaStr
 
 void launch_mvs_particles_batch(const BatchParticleArgs& a, cudaStream_t s, int threads) {
     if (a.ntiles <= 0) return;
+    using Kernel = void (*)(BatchParticleArgs);
+    const Kernel kern = threads <= 64    ? (a.central ? mvs_particle_batch_kernel<true, 64> : mvs_particle_batch_kernel<false, 64>)
+                        : threads <= 128 ? (a.central ? mvs_particle_batch_kernel<true, 128> : mvs_particle_batch_kernel<false, 128>)
+                                         : (a.central ? mvs_particle_batch_kernel<true, 256> : mvs_particle_batch_kernel<false, 256>);
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (a.central) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mvs_particle_batch_kernel<true>, threads, 0);
-    } else {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mvs_particle_batch_kernel<false>, threads, 0);
-    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0);
     if (per_sm < 1) per_sm = 1;
     const int warps = threads / 32;
     const int want = (a.ntiles + warps - 1) / warps;
     const int slots = sms * per_sm;
     const int grid = want < slots ? want : slots;
-    if (a.central) mvs_particle_batch_kernel<true><<<grid, threads, 0, s>>>(a);
-    else mvs_particle_batch_kernel<false><<<grid, threads, 0, s>>>(a);
+    kern<<<grid, threads, 0, s>>>(a);
 }
 
 void launch_classify_batch(const BatchParticleArgs& a, cudaStream_t s) {
@@ -1032,7 +1102,9 @@ void launch_mvs_big(const MvsBigArgs& a, cudaStream_t s) {
     mvs_big_kernel<<<1, 128, smem, s>>>(a);
 }
 
-void launch_mvs_particles(const MvsParticleArgs& a, cudaStream_t s, int threads) {
+void launch_mvs_particles(const MvsParticleArgs& args, cudaStream_t s, int threads) {
+    MvsParticleArgs a = args;
+    a.rmu = 1.0 / a.mu;
     const bool ngf = a.ngf_on != 0;
     const bool obl = a.jcen[0] != 0.0 || a.jcen[1] != 0.0 || a.jcen[2] != 0.0;
     const bool cen = a.central != 0;

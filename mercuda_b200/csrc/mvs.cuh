@@ -18,8 +18,12 @@ namespace mb200 {
 constexpr int TAB_HEAD = 8;        // a0tp[3], acen[3], pad[2]
 constexpr int TAB_BODY = 8;        // x1, y1, z1, m, xmin, xmax, ymin, ymax
 constexpr int TAB_DETAIL = 16;     // x0[3], v0[3], x1[3], v1[3], rce, rphys, pad[2]
+// After the bodies' rows: each body's padded box again as four integers
+// (order_key of xmin, xmax, ymin, ymax, the lower ones less 1), for the first
+// pass of the particles' box test.
+constexpr int TAB_KEYS = 2;
 
-__host__ __device__ constexpr int tab_stride(int nb) { return TAB_HEAD + TAB_BODY * nb; }
+__host__ __device__ constexpr int tab_stride(int nb) { return TAB_HEAD + (TAB_BODY + TAB_KEYS) * nb; }
 
 // Device-resident Big-body state, Fortran-style C indices 0..nbig-1 (0 is the
 // central body). SoA with stride nbig.
@@ -71,6 +75,7 @@ struct MvsParticleArgs {
     int step0;
     int ngf_on;         // mfo_ngf terms present
     double mu;          // central mass
+    double rmu;         // 1 / mu (set by the launch)
     double h;
     double rcen;
     double jcen[3];

@@ -3,6 +3,7 @@
 // and the event-record writer.
 #pragma once
 #include "common.cuh"
+#include "fp64.cuh"
 #include "mvs.cuh"
 
 namespace mb200 {
@@ -253,16 +254,19 @@ __device__ __forceinline__ void store_event(MercuryEvent* dst, const MercuryEven
     for (int k = 0; k < 8; ++k) d[k] = s[k];
 }
 
-// mfo_mvs for one Small body (mercury6_2.for:5034-5060) plus mfo_ngf, i.e. the
-// total acceleration (angf + 0) + a of the kick; T is a force table and g(c)
-// returns the body's c-th non-gravitational coefficient.
-template <bool NGF, bool OBL, class G>
-__device__ __forceinline__ double3 small_body_force(const double3 x, const double3 v_ngf, G g, const double* T,
-                                                    int nb, const double* jcen, double mu, DeviceStatus* st) {
+// The direct terms of a force on a test particle at x, sum of -m d/|d|^3 in
+// the order of the rows (the first four doubles of each: x, y, z, m), with the
+// statements of mfo_mvs and of mfo_grav, which multiply the same two factors.
+// Four rows at a time: each 1/sqrt is a chain of ten dependent operations
+// without a branch (fp64.cuh), and four of them overlap (in the MVS kernel 2, 4
+// and 1 at a time are within 2 %; where a CTA has few warps it is what counts). s2 outside the range
+// of those (coincident bodies among them) makes the whole sum again with plain
+// statements.
+template <int ROW>
+static __device__ __noinline__ double3 direct_terms_plain(double3 x, const double* rows, int nb) {
     double3 a3 = make_double3(0.0, 0.0, 0.0);
-#pragma unroll 1
     for (int b = 0; b < nb; ++b) {
-        const double* row = T + TAB_HEAD + b * TAB_BODY;
+        const double* row = rows + b * ROW;
         const double dx = x.x - row[0], dy = x.y - row[1], dz = x.z - row[2];
         const double s2 = dx * dx + dy * dy + dz * dz;
         const double s_1 = 1.0 / sqrt(s2);
@@ -272,6 +276,50 @@ __device__ __forceinline__ double3 small_body_force(const double3 x, const doubl
         a3.y = a3.y - faci * dy;
         a3.z = a3.z - faci * dz;
     }
+    return a3;
+}
+constexpr int DIRECT_UNROLL = 4;
+template <int ROW> __device__ __forceinline__ double3 direct_terms(const double3 x, const double* rows, int nb) {
+    double3 a3 = make_double3(0.0, 0.0, 0.0);
+    unsigned bad = 0;   // each high word less 2^-511's, ORed: below 2^30 when every s2 is within 2^-511 .. 2^513
+    auto term = [&](const double* row) {
+        const double2 r01 = *reinterpret_cast<const double2*>(row), r23 = *reinterpret_cast<const double2*>(row + 2);
+        const double dx = x.x - r01.x, dy = x.y - r01.y, dz = x.z - r23.x;
+        const double s2 = dx * dx + dy * dy + dz * dz;
+        double s, s_1;
+        sqrt_recip(s2, s, s_1);
+        bad |= (unsigned)__double2hiint(s2) - 0x20000000u;
+        const double s_3 = s_1 * s_1 * s_1;
+        const double faci = r23.y * s_3;
+        return make_double3(faci * dx, faci * dy, faci * dz);
+    };
+    auto take = [&](const double3 t) {
+        a3.x = a3.x - t.x;
+        a3.y = a3.y - t.y;
+        a3.z = a3.z - t.z;
+    };
+    int b = 0;
+#pragma unroll 1
+    for (; b + DIRECT_UNROLL <= nb; b += DIRECT_UNROLL) {
+        double3 t[DIRECT_UNROLL];
+#pragma unroll
+        for (int q = 0; q < DIRECT_UNROLL; ++q) t[q] = term(rows + (b + q) * ROW);
+#pragma unroll
+        for (int q = 0; q < DIRECT_UNROLL; ++q) take(t[q]);
+    }
+#pragma unroll 1
+    for (; b < nb; ++b) take(term(rows + b * ROW));
+    if (bad >= 0x40000000u) a3 = direct_terms_plain<ROW>(x, rows, nb);
+    return a3;
+}
+
+// mfo_mvs for one Small body (mercury6_2.for:5034-5060) plus mfo_ngf, i.e. the
+// total acceleration (angf + 0) + a of the kick; T is a force table and g(c)
+// returns the body's c-th non-gravitational coefficient; ROW doubles a body.
+template <bool NGF, bool OBL, int ROW = TAB_BODY, class G>
+__device__ __forceinline__ double3 small_body_force(const double3 x, const double3 v_ngf, G g, const double* T,
+                                                    int nb, const double* jcen, double mu, DeviceStatus* st) {
+    const double3 a3 = direct_terms<ROW>(x, T + TAB_HEAD, nb);
     double3 a = make_double3(T[0] + a3.x, T[1] + a3.y, T[2] + a3.z);
     if (OBL) {
         const double3 ao = oblate_accel(x, jcen, mu);

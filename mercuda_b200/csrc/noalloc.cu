@@ -31,7 +31,7 @@ constexpr int NOALLOC_MAX_EVENTS = 8192;
 // Scratch layout in doubles.
 constexpr size_t SCR_STATUS = 0;                                        // DeviceStatus (32 bytes)
 constexpr size_t SCR_TAB = 8;                                           // 2 table rows
-constexpr size_t SCR_DETAIL = SCR_TAB + 2 * (TAB_HEAD + TAB_BODY * NOALLOC_MAX_BIG);
+constexpr size_t SCR_DETAIL = SCR_TAB + 2 * tab_stride(NOALLOC_MAX_BIG);
 constexpr size_t SCR_PERM = SCR_DETAIL + (size_t)TAB_DETAIL * NOALLOC_MAX_BIG;   // int slot map
 constexpr size_t SCR_STEP = SCR_PERM + NOALLOC_MAX_PARTICLES / 2;               // int event step tags
 constexpr size_t SCR_CANDS = SCR_STEP + NOALLOC_MAX_EVENTS / 2;                 // EncounterCandidate

@@ -1,0 +1,103 @@
+"""GPU parity of the particle step's branches against the CPU oracle, one step
+each: the straight-line drift and its limits (orbit classes, operands out of
+its range), the integer box screen (turning points, bodies with a margin, more
+than 32 Big bodies) and the central screen's quick tests, at sizes about a
+warp's 32 slots. Bars as for every step: 1e-12 relative, identical records."""
+import numpy as np
+import pytest
+
+from mercuda_b200.backend import Backend, Batch
+from mercuda_b200.system import elements_to_cartesian, make_system
+
+from test_mvs_gpu import REL_ONE_STEP, assert_events_equal, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def orbits(sys0, kind, seed):
+    """Replace the particles' states by orbits of one class."""
+    rng = np.random.default_rng(seed)
+    n = sys0.n - sys0.nbig
+    ang = [rng.uniform(0, 2 * np.pi, n) for _ in range(3)]
+    inc = rng.uniform(0, 0.5, n)
+    a, e = {"circular": (rng.uniform(0.5, 5, n), np.zeros(n)),
+            "eccentric": (rng.uniform(0.5, 5, n), rng.uniform(0.55, 0.99, n)),
+            "close": (10 ** rng.uniform(-2.2, -0.5, n), rng.uniform(0, 0.5, n)),
+            "far": (10 ** rng.uniform(2, 7, n), rng.uniform(0, 0.5, n)),
+            "mixed": (rng.uniform(0.3, 30, n), rng.uniform(0, 0.9, n)),
+            "hyperbolic": (rng.uniform(0.5, 5, n), np.zeros(n)),
+            "radial": (rng.uniform(0.5, 5, n), np.zeros(n))}[kind]
+    x, v = elements_to_cartesian(np.full(n, sys0.m[0]), a, e, inc, *ang)
+    if kind == "hyperbolic":
+        v *= rng.choice([2.0 ** 0.5, 1.5, 3.0], n)[:, None]      # the first: parabolic to rounding
+    if kind == "radial":
+        v = -x * (np.linalg.norm(v, axis=1) / np.linalg.norm(x, axis=1) * rng.uniform(0.01, 2, n))[:, None]
+    sys0.x[sys0.nbig:], sys0.v[sys0.nbig:] = x, v
+    return sys0
+
+
+def check(oracle, sys0, h, rcen=0.005):
+    b = Backend("MVS")
+    b.configure()
+    try:
+        b.upload(sys0)
+        b.step(0.0, h, dtflag=0)
+        x, v = b.download()
+        ev = b.events(h, h, rcen)
+    finally:
+        b.free()
+    ref = sys0.copy()
+    rev, _ = oracle.mvs_run(ref, 0.0, h, 1, rcen, threads=4)
+    assert rel_err(x, ref.x) <= REL_ONE_STEP
+    assert rel_err(v, ref.v) <= REL_ONE_STEP
+    assert_events_equal(ev, rev)
+
+
+@pytest.mark.parametrize("kind", ["circular", "eccentric", "close", "far", "mixed", "hyperbolic", "radial"])
+@pytest.mark.parametrize("h", [8.0, -0.5])
+def test_orbit_classes(oracle, kind, h):
+    check(oracle, orbits(make_system(seed=3, n_particles=257, nplanets=8), kind, 5), h)
+
+
+@pytest.mark.parametrize("planets", [0, 1, 3, 7, 9, 32, 40])
+@pytest.mark.parametrize("count", [1, 31, 33])
+def test_planet_counts(oracle, planets, count):
+    check(oracle, make_system(seed=planets + count, n_particles=count, nplanets=planets, near_fraction=0.3), 8.0)
+
+
+def test_margins_and_wide_central_body(oracle):
+    """Particles with encounter radii of their own, and a central radius that
+    many pericentres pass."""
+    s = orbits(make_system(seed=8, n_particles=500), "mixed", 9)
+    s.rce[s.nbig::2] = 0.05
+    s.rphys[s.nbig::3] = 1e-4
+    check(oracle, s, 8.0, rcen=0.4)
+
+
+@pytest.mark.parametrize("scale", [1e-36, 1e36])
+def test_operands_out_of_range(oracle, scale):
+    """Masses scaled so far that the general statements have to take over."""
+    s = make_system(seed=21, n_particles=100, near_fraction=0.1)
+    s.m *= scale
+    s.v *= scale ** 0.5
+    check(oracle, s, 8.0 / scale ** 0.5)
+
+
+@pytest.mark.parametrize("threads", [64, 128, 256])
+def test_batch_shapes(oracle, threads):
+    systems = [orbits(make_system(seed=40 + k, n_particles=n, nplanets=k + 1), kind, k)
+               for k, (n, kind) in enumerate([(1, "mixed"), (33, "eccentric"), (64, "hyperbolic"), (300, "close")])]
+    h = np.array([8.0, -4.0, 16.0, 2.0])
+    b = Batch(systems, h)
+    try:
+        b.set(threads=threads, steps_per_launch=1)
+        ev, sy, _ = b.advance(0.0, 1, 0.005)
+        ends = b.download()
+    finally:
+        b.free()
+    for k, s in enumerate(systems):
+        ref = s.copy()
+        rev, _ = oracle.mvs_run(ref, 0.0, float(h[k]), 1, 0.005, threads=4)
+        assert rel_err(ends[k][0], ref.x) <= REL_ONE_STEP
+        assert rel_err(ends[k][1], ref.v) <= REL_ONE_STEP
+        assert_events_equal(ev[sy == k], rev)
