@@ -38,412 +38,603 @@ __device__ __forceinline__ int order_key(double x) {
 }
 
 // ------------------------------------------------------------ Big bodies
-// Shared-memory workspace of the Big-body CTA, all [3][nbig] unless noted.
+// The Big-body step is one CTA's serial chain, and small runs, the per-step
+// calls, batches and the adjoint's forward run all wait for it: what counts is
+// its latency. Sums that the map takes in body order (Jacobi coordinates, the
+// indirect terms, the pair forces) are made by one thread per body and
+// coordinate, each adding its own prefix in that order from terms computed one
+// per thread; everything that depends on the masses alone is computed once per
+// launch; square roots and divisions are those of fp64.cuh; and what the next
+// step does not wait for (boxes, details, encounter and impact screens) is
+// done by warps beside the ones that compute the force. 8 planets: 19 us a
+// step with those loops in one thread and plain divisions, 5.2 us so (half of it
+// the innermost planet's universal-variable drift).
+
+// Shared-memory workspace of the Big-body CTA. Arrays are found by their place
+// in it (a table of pointers would live in local memory): [3][N] vectors, then
+// [N] scalars, the pair terms last.
+constexpr int BIG_PAIR_MAX = 33;   // bodies up to which every pair force has its slot
+constexpr int BIG_THREADS = 256;   // a warp for each of eight planets' drifts
+// (two more than a multiple of eight, so that rows start on different banks)
+__host__ __device__ constexpr int big_row(int N) { return (N + 7) / 8 * 8 + 2; }
 struct BigSmem {
-    double *X, *V, *XJ, *VJ, *ACC, *X0, *V0, *XS, *VS, *A1, *A2, *AOBL, *GM, *misc;
-    __device__ void carve(double* base, int nbig) {
-        double* p = base;
-        double** arrays[] = {&X, &V, &XJ, &VJ, &ACC, &X0, &V0, &XS, &VS, &A1, &A2, &AOBL};
-        for (double** a : arrays) { *a = p; p += 3 * nbig; }
-        GM = p; p += nbig;
-        misc = p;  // a0[3], a0tp[3], acen[3]
-    }
+    double* base;
+    int N;
+    int now;   // parity of the current step: its start state is XS(now), VS(now)
+    __device__ double* vec(int q) const { return base + 3 * N * q; }
+    __device__ double* scal(int q) const { return base + (3 * 17 + q) * N; }
+    __device__ double* X() const { return vec(0); }
+    __device__ double* V() const { return vec(1); }
+    __device__ double* XJ() const { return vec(2); }    // Jacobi
+    __device__ double* VJ() const { return vec(3); }
+    __device__ double* ACC() const { return vec(4); }
+    __device__ double* V0() const { return vec(5); }    // velocity after the first kick
+    __device__ double* XS(int par) const { return vec(6 + par); }
+    __device__ double* VS(int par) const { return vec(8 + par); }
+    __device__ double* X0() const { return XS(now); }   // the kick leaves positions alone
+    __device__ double* A1() const { return vec(10); }   // mfo_mvs's terms, see big_force_terms
+    __device__ double* F0() const { return vec(11); }
+    __device__ double* F2() const { return vec(12); }
+    __device__ double* A3() const { return vec(13); }
+    __device__ double* OT() const { return vec(14); }
+    __device__ double* AO() const { return vec(15); }
+    __device__ double* NG() const { return vec(16); }
+    __device__ double* GM() const { return scal(0); }   // gm_j
+    __device__ double* TH() const { return scal(1); }   // 1 / MI
+    __device__ double* TJ() const { return scal(2); }   // m_j over the mass up to j
+    __device__ double* MI() const { return scal(3); }   // mass inside j
+    __device__ double* MS() const { return scal(4); }   // masses
+    // N <= BIG_PAIR_MAX: for each coordinate c and body k a row of terms by
+    // the other body (its index less 1), padded with zeros to whole chunks of eight:
+    // signed pair forces, then mfo_mvs's second indirect term of the bodies up
+    // to k; and one row a coordinate of the first indirect term
+    __device__ int np() const { return big_row(N); }
+    __device__ double* PT(int c, int k) const { return scal(5) + (c * N + k) * np(); }
+    __device__ double* QT(int c, int k) const { return PT(3 + c, k); }
+    __device__ double* RT(int c) const { return PT(6, 0) + c * np(); }
 };
+__host__ __device__ inline size_t big_smem_doubles(int N) {
+    return (size_t)(17 * 3 + 5) * N + (N <= BIG_PAIR_MAX ? (size_t)(6 * N + 3) * big_row(N) + 1 : 0);
+}
 
 // Bodies held by the Big-body CTA (Big, then massive Small bodies).
 __device__ __forceinline__ int big_count(const MvsBigArgs& A) { return A.nmass > A.nbig ? A.nmass : A.nbig; }
 
-// mco_h2j for the Big bodies (mercury6_2.for:2613-2682), one thread; arrays
-// [3][S].
-__device__ void big_h2j(int nbig, const double* m, const double* X, const double* V, double* XJ, double* VJ, int S) {
-    if (nbig < 2) return;
-    double mtot = m[1];
-    double mx[3], mv[3];
-    for (int c = 0; c < 3; ++c) {
-        XJ[c * S + 1] = X[c * S + 1];
-        VJ[c * S + 1] = V[c * S + 1];
-        mx[c] = m[1] * X[c * S + 1];
-        mv[c] = m[1] * V[c * S + 1];
+__device__ __forceinline__ void big_sync() {
+    if (blockDim.x == 32) __syncwarp();
+    else __syncthreads();
+}
+// The items [0, n) of a job that warp w does while others do theirs (0 and 1
+// the force, 2 to 5 the screens and table rows, which take as long); one-warp
+// CTAs and large systems take the jobs one after another with every thread.
+template <class F> __device__ __forceinline__ void big_job(int w, int N, int n, F f) {
+    const bool all = blockDim.x == 32 || N > BIG_PAIR_MAX;
+    if (!all && (int)(threadIdx.x >> 5) != w) return;
+    const int step = all ? blockDim.x : 32;
+    for (int k = all ? threadIdx.x : threadIdx.x & 31; k < n; k += step) f(k);
+}
+// Every (body k in [k0, k1), coordinate c), each by one thread.
+template <class F> __device__ __forceinline__ void big_each(int k0, int k1, F f) {
+    for (int q = threadIdx.x; q < 3 * (k1 - k0); q += blockDim.x) {
+        const int j = q / 3;
+        f(k0 + j, q - 3 * j);
     }
-    for (int j = 2; j <= nbig - 2; ++j) {
-        const double temp = 1.0 / (mtot + m[0]);
-        mtot = mtot + m[j];
-        for (int c = 0; c < 3; ++c) {
-            XJ[c * S + j] = X[c * S + j] - temp * mx[c];
-            VJ[c * S + j] = V[c * S + j] - temp * mv[c];
-        }
-        for (int c = 0; c < 3; ++c) {
-            mx[c] = mx[c] + m[j] * X[c * S + j];
-            mv[c] = mv[c] + m[j] * V[c * S + j];
+}
+// 1.0 / sqrt(x) and a / b in plain, as calls: the step's code is long, and what
+// does not run should not lie between what does (the instruction cache misses
+// of a lone CTA are not hidden by anything).
+static __device__ __noinline__ double rsqrt_plain(double x) { return 1.0 / sqrt(x); }
+static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
+// 1.0 / sqrt(x): fp64.cuh's where the operand allows, else plain.
+__device__ __forceinline__ double rsqrt_any(double x) {
+    if (!mid_range(x)) return rsqrt_plain(x);
+    double s, r;
+    sqrt_recip(x, s, r);
+    return r;
+}
+
+// What depends on the masses alone. S.MS() is filled; synchronized before.
+__device__ void big_constants(const MvsBigArgs& A, BigSmem& S) {
+    if (threadIdx.x == 0) {
+        double minside = S.MS()[0], mtot = 0.0;   // mtot: Big bodies inside the next one
+        for (int j = 1; j < A.nbig; ++j) {
+            S.GM()[j] = minside;
+            minside = minside + S.MS()[j];
+            S.TH()[j] = minside;
+            S.MI()[j] = mtot + S.MS()[0];
+            mtot = j == 1 ? S.MS()[1] : mtot + S.MS()[j];
+            S.TJ()[j] = mtot;
         }
     }
-    if (nbig > 2) {
-        const double temp = 1.0 / (mtot + m[0]);
-        const int j = nbig - 1;
-        for (int c = 0; c < 3; ++c) {
-            XJ[c * S + j] = X[c * S + j] - temp * mx[c];
-            VJ[c * S + j] = V[c * S + j] - temp * mv[c];
+    big_sync();
+    for (int j = 1 + threadIdx.x; j < A.nbig; j += blockDim.x) {
+        S.GM()[j] = S.MS()[0] * S.TH()[j] / S.GM()[j];
+        S.TJ()[j] = S.MS()[j] / (S.TJ()[j] + S.MS()[0]);
+        S.TH()[j] = 1.0 / S.MI()[j];
+    }
+    big_sync();
+}
+
+// Prefix sums of the products that big_products left in F0 and F2, in body
+// order: A3 and OT receive, for body j, the sum over bodies 1 .. j - 1. Six
+// chains of adds; eight terms are fetched at a time (past the last body's they
+// are not used).
+__device__ __forceinline__ void big_scan(const MvsBigArgs& A, const BigSmem& S) {
+    if (threadIdx.x >= 6) return;
+    const int N = S.N, nbig = A.nbig, c = threadIdx.x % 3;
+    const double* t = (threadIdx.x < 3 ? S.F0() : S.F2()) + c * N;
+    double* out = (threadIdx.x < 3 ? S.A3() : S.OT()) + c * N;
+    if (nbig < 3) return;
+    double p = t[1];
+    out[2] = p;
+    for (int i0 = 2; i0 < nbig - 1; i0 += 8) {
+        double u[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) u[q] = t[i0 + q];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            p = p + u[q];
+            if (i0 + q + 1 < nbig) out[i0 + q + 1] = p;
         }
     }
 }
 
-// mco_j2h for the Big bodies (mercury6_2.for:2700-2770), one thread; arrays
-// [3][S].
-__device__ void big_j2h(int nbig, const double* m, const double* XJ, const double* VJ, double* X, double* V, int S) {
-    if (nbig < 2) return;
-    double mtot = m[1];
-    double temp = m[1] / (mtot + m[0]);
-    double mx[3], mv[3];
-    for (int c = 0; c < 3; ++c) {
-        X[c * S + 1] = XJ[c * S + 1];
-        V[c * S + 1] = VJ[c * S + 1];
-        mx[c] = temp * XJ[c * S + 1];
-        mv[c] = temp * VJ[c * S + 1];
-    }
-    for (int j = 2; j <= nbig - 2; ++j) {
-        for (int c = 0; c < 3; ++c) {
-            X[c * S + j] = XJ[c * S + j] + mx[c];
-            V[c * S + j] = VJ[c * S + j] + mv[c];
+// mco_h2j for the Big bodies (mercury6_2.for:2613-2682) from the products m_j
+// x_j, m_j v_j in F0, F2. All threads; synchronized before and after.
+__device__ __forceinline__ void big_h2j(const MvsBigArgs& A, const BigSmem& S) {
+    const int N = S.N;
+    big_scan(A, S);
+    big_sync();
+    big_each(1, A.nbig, [&](int j, int c) {
+        const int z = c * N + j;
+        const double x = S.X()[z], v = S.V()[z], th = S.TH()[j], px = S.A3()[z], pv = S.OT()[z];
+        S.XJ()[z] = j >= 2 ? x - th * px : x;
+        S.VJ()[z] = j >= 2 ? v - th * pv : v;
+    });
+    big_sync();
+}
+__device__ __forceinline__ void big_products(const MvsBigArgs& A, const BigSmem& S) {
+    const int N = S.N;
+    big_each(1, A.nbig, [&](int j, int c) {
+        const int z = c * N + j;
+        S.F0()[z] = S.MS()[j] * S.X()[z];
+        S.F2()[z] = S.MS()[j] * S.V()[z];
+    });
+    big_sync();
+}
+
+// The drift of mdt_mvs, after h2j: Kepler drift of each Jacobi Big body with
+// gm_j, j2h; each massive Small body drifts heliocentrically about the central
+// mass (mercury6_2.for:4031-4052). All threads.
+__device__ void big_drift(const MvsBigArgs& A, BigSmem& S, double h) {
+    const int nbig = A.nbig, N = big_count(A);
+    // bodies dealt out to the warps: those that need the universal-variable
+    // solve (the innermost planets' steps are long for them) then take no
+    // other body's time
+    const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int k = 1 + w + nw * lane; k < N; k += blockDim.x) {
+        const bool big = k < nbig;
+        double* px = big ? S.XJ() : S.X();
+        double* pv = big ? S.VJ() : S.V();
+        double3 p = ld3(px, N, k), w = ld3(pv, N, k);
+        drift_one(big ? S.GM()[k] : S.MS()[0], p, w, h);
+        st3(px, N, k, p);
+        st3(pv, N, k, w);
+        if (big) {
+            const double tj = S.TJ()[k];
+            st3(S.F0(), N, k, make_double3(tj * p.x, tj * p.y, tj * p.z));
+            st3(S.F2(), N, k, make_double3(tj * w.x, tj * w.y, tj * w.z));
         }
-        mtot = mtot + m[j];
-        temp = m[j] / (mtot + m[0]);
-        for (int c = 0; c < 3; ++c) {
-            mx[c] = mx[c] + temp * XJ[c * S + j];
-            mv[c] = mv[c] + temp * VJ[c * S + j];
-        }
     }
-    if (nbig > 2) {
-        const int j = nbig - 1;
-        for (int c = 0; c < 3; ++c) {
-            X[c * S + j] = XJ[c * S + j] + mx[c];
-            V[c * S + j] = VJ[c * S + j] + mv[c];
-        }
-    }
+    big_sync();
+    // mco_j2h (mercury6_2.for:2700-2770)
+    big_scan(A, S);
+    big_sync();
+    big_each(1, nbig, [&](int j, int c) {
+        const int z = c * N + j;
+        const double x = S.XJ()[z], v = S.VJ()[z], px = S.A3()[z], pv = S.OT()[z];
+        S.X()[z] = j >= 2 ? x + px : x;
+        S.V()[z] = j >= 2 ? v + pv : v;
+    });
+    big_sync();
+}
+
+// The terms of mfo_obl and mfo_ngf (rare, hence a call).
+static __device__ __noinline__ void big_extra_terms(const MvsBigArgs& A, const BigSmem S, const double* V_ngf) {
+    const int nbig = A.nbig, nb = nbig - 1, N = big_count(A);
+    const double* m = S.MS();
+    if (A.obl)
+        big_job(1, N, N - 1, [&](int q) {
+            const int k = 1 + q;
+            const double3 ao = oblate_accel(ld3(S.X(), N, k), A.jcen, m[0]);
+            const double tmp4 = m[k] / m[0];
+            st3(S.AO(), N, k, ao);
+            st3(S.OT(), N, k, make_double3(tmp4 * ao.x, tmp4 * ao.y, tmp4 * ao.z));
+        });
+    if (A.ngflag == 1 || A.ngflag == 3)
+        big_job(0, N, nb, [&](int q) {
+            const int k = 1 + q;
+            double3 g;
+            if (!nongrav_accel(ld3(S.X(), N, k), ld3(V_ngf, N, k), A.ngf + 5 * k, g)) raise_fault(A.status, 2);
+            st3(S.NG(), N, k, g);
+        });
 }
 
 // mfo_mvs for the Big bodies plus the indirect term a0tp that every Small
-// body receives (mercury6_2.for:4946-5070), with mfo_ngf for Big bodies.
-// Writes S.ACC = (angf + 0) + a and S.misc = {a0, a0tp, acen}. All threads.
+// body receives (mercury6_2.for:4946-5070), with mfo_ngf for Big bodies, in two
+// parts with a barrier of the caller's between: the terms, one per thread ...
 // With massive Small bodies held (A.nmass > nbig) their oblateness terms
 // enter acen in body order, as mfo_obl sums over every body
 // (mercury6_2.for:5176-5230); their own accelerations follow from the force
 // row (small_type_force).
-__device__ void big_force(const MvsBigArgs& A, BigSmem& S, const double* V_ngf) {
-    const int nbig = A.nbig, N = big_count(A), tid = threadIdx.x, nt = blockDim.x;
-    const double* m = A.m;
-    double* a0 = S.misc;
-    double* a0tp = S.misc + 3;
-    double* acen = S.misc + 6;
-    if (tid == 0) {
-        a0[0] = a0[1] = a0[2] = 0.0;
-        if (nbig >= 2)
-            for (int c = 0; c < 3; ++c) { S.A1[c * N + 1] = 0.0; S.A2[c * N + 1] = 0.0; }
-        double minside = 0.0;
-        for (int k = 2; k < nbig; ++k) {
-            const int k1 = k - 1;
-            minside = minside + m[k1];
-            const double3 p = ld3(S.X, N, k), pj = ld3(S.XJ, N, k);
-            const double r2 = p.x * p.x + p.y * p.y + p.z * p.z;
-            const double rj2 = pj.x * pj.x + pj.y * pj.y + pj.z * pj.z;
-            const double r = 1.0 / sqrt(r2);
-            const double rj = 1.0 / sqrt(rj2);
-            const double r3 = r * r * r;
-            const double rj3 = rj * rj * rj;
-            const double fac0 = m[k] * r3;
-            const double fac12 = m[0] * rj3;
-            const double fac2 = m[k] * fac12 / (minside + m[0]);
-            const double q = (r2 - rj2) * 0.5 / rj2;
-            const double q2 = q * q, q3 = q * q2, q4 = q2 * q2, q5 = q2 * q3, q6 = q3 * q3, q7 = q3 * q4;
-            const double fac1 = 402.1875 * q7 - 187.6875 * q6 + 86.625 * q5 - 39.375 * q4 + 17.5 * q3 -
-                                7.5 * q2 + 3.0 * q - 1.0;
-            const double pc[3] = {p.x, p.y, p.z}, pjc[3] = {pj.x, pj.y, pj.z};
-            for (int c = 0; c < 3; ++c) {
-                a0[c] = a0[c] - fac0 * pc[c];
-                S.A1[c * N + k] = fac12 * (pjc[c] + fac1 * pc[c]);
-                S.A2[c * N + k] = S.A2[c * N + k1] + fac2 * pjc[c];
+__device__ void big_force_terms(const MvsBigArgs& A, BigSmem& S, const double* V_ngf) {
+    const int nbig = A.nbig, nb = nbig - 1, N = big_count(A);
+    const double* m = S.MS();
+    big_job(0, N, nb, [&](int q) {
+        const int k = 1 + q;
+        const double3 p = ld3(S.X(), N, k), pj = ld3(S.XJ(), N, k);
+        const double r2 = p.x * p.x + p.y * p.y + p.z * p.z;
+        const double rj2 = pj.x * pj.x + pj.y * pj.y + pj.z * pj.z;
+        // both square roots and both quotients in flight together; operands
+        // out of range (k = 1 has no Jacobi terms) take the plain statements
+        double s, r, rj;
+        sqrt_recip(r2, s, r);
+        sqrt_recip(rj2, s, rj);
+        const bool fast = mid_range(r2) && mid_range(rj2);
+        if (!fast) {
+            r = rsqrt_plain(r2);
+            rj = rsqrt_plain(rj2);
+        }
+        const double r3 = r * r * r, rj3 = rj * rj * rj;
+        const double fac0 = m[k] * r3;
+        const double fac12 = m[0] * rj3;
+        const double f2 = m[k] * fac12, dr = (r2 - rj2) * 0.5, mi = S.MI()[k];
+        double fac2 = quotient(f2, mi, S.TH()[k]), u = quotient(dr, rj2, rj * rj);
+        if (!(fast && mid_magnitude(mi) && (mid_magnitude(f2) || f2 == 0.0) && (mid_magnitude(dr) || dr == 0.0))) {
+            fac2 = div_plain(f2, mi);
+            u = div_plain(dr, rj2);
+        }
+        const double q2 = u * u, q3 = u * q2, q4 = q2 * q2, q5 = q2 * q3, q6 = q3 * q3, q7 = q3 * q4;
+        const double fac1 = 402.1875 * q7 - 187.6875 * q6 + 86.625 * q5 - 39.375 * q4 + 17.5 * q3 - 7.5 * q2 +
+                            3.0 * u - 1.0;
+        st3(S.F0(), N, k, make_double3(fac0 * p.x, fac0 * p.y, fac0 * p.z));
+        st3(S.A1(), N, k, k == 1 ? make_double3(0.0, 0.0, 0.0)
+                               : make_double3(fac12 * (pj.x + fac1 * p.x), fac12 * (pj.y + fac1 * p.y),
+                                              fac12 * (pj.z + fac1 * p.z)));
+        const double3 t2 = make_double3(fac2 * pj.x, fac2 * pj.y, fac2 * pj.z);
+        st3(S.F2(), N, k, t2);
+        if (N <= BIG_PAIR_MAX && k >= 2) {
+            S.RT(0)[k - 1] = -(fac0 * p.x);
+            S.RT(1)[k - 1] = -(fac0 * p.y);
+            S.RT(2)[k - 1] = -(fac0 * p.z);
+            for (int j = k; j < nbig; ++j) {
+                S.QT(0, j)[k - 1] = t2.x;
+                S.QT(1, j)[k - 1] = t2.y;
+                S.QT(2, j)[k - 1] = t2.z;
             }
         }
-        a0tp[0] = a0tp[1] = a0tp[2] = 0.0;
-        if (nbig >= 2) {
-            const double3 p = ld3(S.X, N, 1);
-            const double r2 = p.x * p.x + p.y * p.y + p.z * p.z;
-            const double r = 1.0 / sqrt(r2);
-            const double r3 = r * r * r;
-            const double fac0 = m[1] * r3;
-            a0tp[0] = a0[0] - fac0 * p.x;
-            a0tp[1] = a0[1] - fac0 * p.y;
-            a0tp[2] = a0[2] - fac0 * p.z;
-        }
-    }
-    if (A.obl)
-        for (int k = 1 + tid; k < N; k += nt) st3(S.AOBL, N, k, oblate_accel(ld3(S.X, N, k), A.jcen, m[0]));
-    __syncthreads();
-    if (tid == 0) {
-        acen[0] = acen[1] = acen[2] = 0.0;
-        if (A.obl)
-            for (int k = 1; k < N; ++k) {
-                const double tmp4 = m[k] / m[0];
-                const double3 ao = ld3(S.AOBL, N, k);
-                acen[0] = acen[0] - tmp4 * ao.x;
-                acen[1] = acen[1] - tmp4 * ao.y;
-                acen[2] = acen[2] - tmp4 * ao.z;
-            }
-    }
-    __syncthreads();
-    for (int k = 1 + tid; k < nbig; k += nt) {
-        const double3 pk = ld3(S.X, N, k);
-        double3 a3 = make_double3(0.0, 0.0, 0.0);
-        for (int i = 1; i < nbig; ++i) {
-            if (i == k) continue;
-            const double3 pi = ld3(S.X, N, i);
-            // The pair (lower, higher) is differenced higher - lower in mfo_mvs.
-            const bool lower = i < k;
-            const double dx = lower ? pk.x - pi.x : pi.x - pk.x;
-            const double dy = lower ? pk.y - pi.y : pi.y - pk.y;
-            const double dz = lower ? pk.z - pi.z : pi.z - pk.z;
+    });
+    if (N <= BIG_PAIR_MAX) {
+        // a pair (i < k) once: the difference is the later body's less the
+        // earlier one's in both sums
+        big_job(1, N, nb * (nb - 1) / 2, [&](int q) {
+            int i = 1, rem = q;
+            while (rem >= nbig - 1 - i) { rem -= nbig - 1 - i; ++i; }
+            const int k = i + 1 + rem;
+            const double3 pk = ld3(S.X(), N, k), pi = ld3(S.X(), N, i);
+            const double dx = pk.x - pi.x, dy = pk.y - pi.y, dz = pk.z - pi.z;
             const double s2 = dx * dx + dy * dy + dz * dz;
-            const double s_1 = 1.0 / sqrt(s2);
+            const double s_1 = rsqrt_any(s2);
             const double s_3 = s_1 * s_1 * s_1;
-            const double fac = m[i] * s_3;
-            if (lower) { a3.x = a3.x - fac * dx; a3.y = a3.y - fac * dy; a3.z = a3.z - fac * dz; }
-            else { a3.x = a3.x + fac * dx; a3.y = a3.y + fac * dy; a3.z = a3.z + fac * dz; }
-        }
-        double3 a;
-        a.x = a0[0] + S.A1[k] + S.A2[k] + a3.x;
-        a.y = a0[1] + S.A1[N + k] + S.A2[N + k] + a3.y;
-        a.z = a0[2] + S.A1[2 * N + k] + S.A2[2 * N + k] + a3.z;
-        if (A.obl) {
-            const double3 ao = ld3(S.AOBL, N, k);
-            a.x = a.x + (ao.x - acen[0]);
-            a.y = a.y + (ao.y - acen[1]);
-            a.z = a.z + (ao.z - acen[2]);
-        }
-        if (A.ngflag == 1 || A.ngflag == 3) {
-            double3 g;
-            if (!nongrav_accel(pk, ld3(V_ngf, N, k), A.ngf + 5 * k, g)) raise_fault(A.status, 2);
-            a.x = g.x + 0.0 + a.x;
-            a.y = g.y + 0.0 + a.y;
-            a.z = g.z + 0.0 + a.z;
-        }
-        if (!isfinite(a.x) || !isfinite(a.y) || !isfinite(a.z)) raise_fault(A.status, 1);
-        st3(S.ACC, N, k, a);
+            const double fk = m[i] * s_3, fi = m[k] * s_3;
+            S.PT(0, k)[i - 1] = -(fk * dx);
+            S.PT(1, k)[i - 1] = -(fk * dy);
+            S.PT(2, k)[i - 1] = -(fk * dz);
+            S.PT(0, i)[k - 1] = fi * dx;
+            S.PT(1, i)[k - 1] = fi * dy;
+            S.PT(2, i)[k - 1] = fi * dz;
+        });
+    } else {
+        big_job(1, N, nb, [&](int q) {
+            const int k = 1 + q;
+            const double3 pk = ld3(S.X(), N, k);
+            double3 a3 = make_double3(0.0, 0.0, 0.0);
+            for (int i = 1; i < nbig; ++i) {
+                if (i == k) continue;
+                const double3 pi = ld3(S.X(), N, i);
+                const bool lower = i < k;
+                const double dx = lower ? pk.x - pi.x : pi.x - pk.x;
+                const double dy = lower ? pk.y - pi.y : pi.y - pk.y;
+                const double dz = lower ? pk.z - pi.z : pi.z - pk.z;
+                const double s2 = dx * dx + dy * dy + dz * dz;
+                const double s_1 = rsqrt_any(s2);
+                const double s_3 = s_1 * s_1 * s_1;
+                const double fac = m[i] * s_3;
+                if (lower) { a3.x = a3.x - fac * dx; a3.y = a3.y - fac * dy; a3.z = a3.z - fac * dz; }
+                else { a3.x = a3.x + fac * dx; a3.y = a3.y + fac * dy; a3.z = a3.z + fac * dz; }
+            }
+            st3(S.A3(), N, k, a3);
+        });
     }
-    __syncthreads();
+    if (A.obl || A.ngflag == 1 || A.ngflag == 3) big_extra_terms(A, S, V_ngf);
 }
 
-// Force row of a table: head {a0tp, acen} and per-Big-body {x, m}.
-__device__ void write_force_table(const MvsBigArgs& A, const BigSmem& S, double* row) {
+// ... and their sums in mfo_mvs's order: S.ACC() = (angf + 0) + a, and the force
+// row's head {a0tp, acen} (of the step's table row, or null). The caller
+// synchronizes after it.
+__device__ void big_force_sum(const MvsBigArgs& A, BigSmem& S, double* row) {
     const int nbig = A.nbig, N = big_count(A);
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 6; ++c) row[c] = S.misc[3 + c];
-    for (int k = 1 + threadIdx.x; k < nbig; k += blockDim.x) {
-        double* b = row + TAB_HEAD + (k - 1) * TAB_BODY;
-        b[0] = S.X[k];
-        b[1] = S.X[N + k];
-        b[2] = S.X[2 * N + k];
-        b[3] = A.m[k];
-    }
+    big_each(1, nbig, [&](int k, int c) {
+        const double* F0 = S.F0() + c * N;
+        double a0 = 0.0, a2 = 0.0, a3 = 0.0, acen = 0.0;
+        if (N <= BIG_PAIR_MAX) {
+            // every term of a row, the zeros too (x + 0 is x: no sum here is
+            // -0), so that nothing depends on k: three chains of adds
+            const double2 *p3 = reinterpret_cast<const double2*>(S.PT(c, k)),
+                          *p2 = reinterpret_cast<const double2*>(S.QT(c, k)),
+                          *p0 = reinterpret_cast<const double2*>(S.RT(c));
+            for (int i0 = 1; i0 < nbig; i0 += 8, p3 += 4, p2 += 4, p0 += 4) {
+                double2 t3[4], t2[4], t0[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    t3[q] = p3[q];
+                    t2[q] = p2[q];
+                    t0[q] = p0[q];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    a3 = a3 + t3[q].x;
+                    a2 = a2 + t2[q].x;
+                    a0 = a0 + t0[q].x;
+                    a3 = a3 + t3[q].y;
+                    a2 = a2 + t2[q].y;
+                    a0 = a0 + t0[q].y;
+                }
+            }
+        } else {
+            for (int i = 2; i < nbig; ++i) a0 = a0 - F0[i];
+            for (int i = 2; i <= k; ++i) a2 = a2 + S.F2()[c * N + i];
+            a3 = S.A3()[c * N + k];
+        }
+        double a = a0 + S.A1()[c * N + k] + a2 + a3;
+        if (A.obl) {
+            for (int i = 1; i < N; ++i) acen = acen - S.OT()[c * N + i];
+            a = a + (S.AO()[c * N + k] - acen);
+        }
+        if (A.ngflag == 1 || A.ngflag == 3) a = S.NG()[c * N + k] + 0.0 + a;
+        if (!isfinite(a)) raise_fault(A.status, 1);
+        S.ACC()[c * N + k] = a;
+        if (k == 1) {
+            row[c] = a0 - F0[1];
+            row[3 + c] = acen;
+        }
+    });
+    if (nbig < 2)
+        for (int c = threadIdx.x; c < 3; c += blockDim.x) {
+            double acen = 0.0;
+            if (A.obl)
+                for (int i = 1; i < N; ++i) acen = acen - S.OT()[c * N + i];
+            row[c] = 0.0;
+            row[3 + c] = acen;
+        }
+}
+
+// Force rows {x, m} of the Big bodies.
+__device__ void write_force_rows(const MvsBigArgs& A, const BigSmem& S, double* row) {
+    const int N = big_count(A);
+    big_job(5, N, A.nbig - 1, [&](int q) {
+        double* b = row + TAB_HEAD + q * TAB_BODY;
+        b[0] = S.X()[q + 1];
+        b[1] = S.X()[N + q + 1];
+        b[2] = S.X()[2 * N + q + 1];
+        b[3] = S.MS()[q + 1];
+    });
 }
 
 // Accelerations of the massive Small bodies held by the CTA: the particles'
 // mfo_mvs + mfo_ngf statements (small_body_force) against the force row just
-// written. All threads; the row must be visible (after __syncthreads).
-__device__ void small_type_force(const MvsBigArgs& A, BigSmem& S, const double* row, const double* V_ngf) {
+// written. All threads; the row must be visible (after big_sync).
+static __device__ __noinline__ void small_type_force(const MvsBigArgs& A, const BigSmem S, const double* row,
+                                                     const double* V_ngf) {
     const int nbig = A.nbig, N = big_count(A), nb = nbig - 1;
     const bool ngf = A.ngflag == 1 || A.ngflag == 3;
     for (int k = nbig + threadIdx.x; k < N; k += blockDim.x) {
-        const double3 x = ld3(S.X, N, k), v = ld3(V_ngf, N, k);
+        const double3 x = ld3(S.X(), N, k), v = ld3(V_ngf, N, k);
         auto g = [&](int c) -> double { return A.ngf[5 * k + c]; };
         double3 a;
         if (ngf) a = A.obl ? small_body_force<true, true>(x, v, g, row, nb, A.jcen, A.m[0], A.status)
                            : small_body_force<true, false>(x, v, g, row, nb, A.jcen, A.m[0], A.status);
         else a = A.obl ? small_body_force<false, true>(x, v, g, row, nb, A.jcen, A.m[0], A.status)
                        : small_body_force<false, false>(x, v, g, row, nb, A.jcen, A.m[0], A.status);
-        st3(S.ACC, N, k, a);
+        st3(S.ACC(), N, k, a);
     }
-    __syncthreads();
+    big_sync();
 }
 
-// The drift of mdt_mvs: h2j, Kepler drift of each Jacobi Big body with gm_j,
-// j2h; each massive Small body drifts heliocentrically about the central
-// mass (mercury6_2.for:4031-4052). All threads.
-__device__ void big_drift(const MvsBigArgs& A, BigSmem& S, double h) {
-    const int nbig = A.nbig, N = big_count(A), tid = threadIdx.x, nt = blockDim.x;
-    if (tid == 0) big_h2j(nbig, A.m, S.X, S.V, S.XJ, S.VJ, N);
-    __syncthreads();
-    for (int k = 1 + tid; k < N; k += nt) {
-        if (k < nbig) {
-            double3 p = ld3(S.XJ, N, k), w = ld3(S.VJ, N, k);
-            drift_one(S.GM[k], p, w, h);
-            st3(S.XJ, N, k, p);
-            st3(S.VJ, N, k, w);
-        } else {
-            double3 p = ld3(S.X, N, k), w = ld3(S.V, N, k);
-            drift_one(A.m[0], p, w, h);
-            st3(S.X, N, k, p);
-            st3(S.V, N, k, w);
-        }
-    }
-    __syncthreads();
-    if (tid == 0) big_j2h(nbig, A.m, S.XJ, S.VJ, S.X, S.V, N);
-    __syncthreads();
+// The whole force: terms, sums, table row. All threads; synchronized after.
+__device__ void big_force(const MvsBigArgs& A, BigSmem& S, double* row) {
+    big_force_terms(A, S, S.V());
+    write_force_rows(A, S, row);
+    big_sync();
+    big_force_sum(A, S, row);
+    big_sync();
+    if (big_count(A) > A.nbig) small_type_force(A, S, row, S.V());
 }
 
 __device__ void big_load(const MvsBigArgs& A, BigSmem& S, double* smem) {
-    const int nbig = A.nbig, N = big_count(A), tid = threadIdx.x, nt = blockDim.x;
-    S.carve(smem, N);
-    for (int k = tid; k < N; k += nt)
-        for (int c = 0; c < 3; ++c) {
-            S.X[c * N + k] = A.in.x[c * N + k];
-            S.V[c * N + k] = A.in.v[c * N + k];
-            S.ACC[c * N + k] = A.in.a[c * N + k];
-        }
-    if (tid == 0) {
-        double minside = A.m[0];
-        for (int j = 1; j < nbig; ++j) {
-            const double msofar = minside + A.m[j];
-            S.GM[j] = A.m[0] * msofar / minside;
-            minside = msofar;
-        }
+    const int N = big_count(A), tid = threadIdx.x, nt = blockDim.x;
+    S.base = smem;
+    S.N = N;
+    S.now = 0;
+    for (int q = tid; q < 3 * N; q += nt) {
+        S.X()[q] = A.in.x[q];
+        S.V()[q] = A.in.v[q];
+        S.ACC()[q] = A.in.a[q];
     }
-    __syncthreads();
+    for (int k = tid; k < N; k += nt) S.MS()[k] = A.m[k];
+    if (N <= BIG_PAIR_MAX)
+        for (int q = tid; q < (6 * N + 3) * big_row(N); q += nt) S.PT(0, 0)[q] = 0.0;
+    big_sync();
+    big_constants(A, S);
+}
+
+// Boxes, details and mce_stat's pairs of step s (start states X0, V0 after the
+// kick, end states X, V after the drift): jobs for the warps beside the force.
+__device__ void big_screen(const MvsBigArgs& A, BigSmem& S, int s, double* row, double* det) {
+    const int nbig = A.nbig, N = big_count(A), nb = nbig - 1;
+    const double h = A.h, hm1 = 1.0 / h;
+    big_job(2, N, nb, [&](int q) {
+        const int k = 1 + q;
+        double* b = row + TAB_HEAD + q * TAB_BODY;
+        const double pad = A.rce[k] * 1.2;
+        double xlo, xhi, ylo, yhi;
+        box_extent(S.X0()[k], S.X()[k], S.V0()[k], S.V()[k], h, xlo, xhi);
+        box_extent(S.X0()[N + k], S.X()[N + k], S.V0()[N + k], S.V()[N + k], h, ylo, yhi);
+        xlo = xlo - pad; xhi = xhi + pad; ylo = ylo - pad; yhi = yhi + pad;
+        b[4] = xlo; b[5] = xhi; b[6] = ylo; b[7] = yhi;
+        reinterpret_cast<int4*>(row + TAB_HEAD + TAB_BODY * nb)[q] =
+            make_int4(order_key(xlo) - 1, order_key(xhi), order_key(ylo) - 1, order_key(yhi));
+        double* d = det + q * TAB_DETAIL;
+        for (int c = 0; c < 3; ++c) {
+            d[c] = S.X0()[c * N + k];
+            d[3 + c] = S.V0()[c * N + k];
+            d[6 + c] = S.X()[c * N + k];
+            d[9 + c] = S.V()[c * N + k];
+        }
+        d[12] = A.rce[k];
+        d[13] = A.rphys[k];
+    });
+    // mce_stat between Big bodies (pairs 1 <= i < j < nbig), then between
+    // Big bodies and the massive Small bodies held (i < nbig <= j < N).
+    const int npair_big = nb * (nb - 1) / 2;
+    big_job(3, N, npair_big + nb * (N - nbig), [&](int q) {
+        int i = 1, j;
+        if (q < npair_big) {
+            int rem = q;
+            while (rem >= nbig - 1 - i) { rem -= nbig - 1 - i; ++i; }
+            j = i + 1 + rem;
+        } else {
+            const int r = q - npair_big;
+            i = 1 + r / (N - nbig);
+            j = nbig + r % (N - nbig);
+        }
+        double lo_i, hi_i, lo_j, hi_j, ylo_i, yhi_i, ylo_j, yhi_j;
+        const double pi_ = A.rce[i] * 1.2, pj_ = A.rce[j] * 1.2;
+        box_extent(S.X0()[i], S.X()[i], S.V0()[i], S.V()[i], h, lo_i, hi_i);
+        box_extent(S.X0()[N + i], S.X()[N + i], S.V0()[N + i], S.V()[N + i], h, ylo_i, yhi_i);
+        box_extent(S.X0()[j], S.X()[j], S.V0()[j], S.V()[j], h, lo_j, hi_j);
+        box_extent(S.X0()[N + j], S.X()[N + j], S.V0()[N + j], S.V()[N + j], h, ylo_j, yhi_j);
+        lo_i = lo_i - pi_; hi_i = hi_i + pi_; ylo_i = ylo_i - pi_; yhi_i = yhi_i + pi_;
+        lo_j = lo_j - pj_; hi_j = hi_j + pj_; ylo_j = ylo_j - pj_; yhi_j = yhi_j + pj_;
+        if (!(hi_i >= lo_j && hi_j >= lo_i && yhi_i >= ylo_j && yhi_j >= ylo_i)) return;
+        PairEnds I{ld3(S.X0(), N, i), ld3(S.V0(), N, i), ld3(S.X(), N, i), ld3(S.V(), N, i)};
+        PairEnds J{ld3(S.X0(), N, j), ld3(S.V0(), N, j), ld3(S.X(), N, j), ld3(S.V(), N, j)};
+        PairClass pc;
+        if (!pair_classify(I, J, A.rce[i], A.rce[j], A.rphys[i], A.rphys[j], h, pc)) return;
+        const int slot = atomicAdd(&A.status->events, 1);
+        if (slot < A.event_cap) {
+            pair_record(A.events + slot, I, J, pc, hm1, i + 1, j + 1, A.m[j] > A.m[i] && j < nbig);
+            A.event_step[slot] = A.step0 + s;
+            if (A.event_sys) A.event_sys[slot] = A.sys;
+        } else {
+            atomicExch(&A.status->overflow, 1);
+        }
+    });
+}
+
+// mce_cent over step s: its start state is in XS/VS[s & 1], its end state in
+// XS/VS of the next step.
+__device__ void big_central(const MvsBigArgs& A, BigSmem& S, int s) {
+    const int N = big_count(A);
+    const double *x0 = S.XS(s & 1), *v0 = S.VS(s & 1), *x1 = S.XS(~s & 1), *v1 = S.VS(~s & 1);
+    big_job(4, N, N - 1, [&](int q) {
+        const int k = 1 + q;
+        double temp;
+        if (!central_impact(ld3(x0, N, k), ld3(v0, N, k), ld3(x1, N, k), ld3(v1, N, k), A.m[0], A.m[k], A.h, A.rcen,
+                            temp))
+            return;
+        const int slot = atomicAdd(&A.status->events, 1);
+        if (slot < A.event_cap) {
+            MercuryEvent rec = {};
+            rec.i = 1;
+            rec.j = k + 1;
+            rec.kind = EV_CENTRAL;
+            rec.time = temp;
+            rec.distance = A.rcen;
+            store_event(A.events + slot, rec);
+            A.event_step[slot] = A.step0 + s;
+            if (A.event_sys) A.event_sys[slot] = A.sys;
+        } else {
+            atomicExch(&A.status->overflow, 1);
+        }
+    });
 }
 
 // The Big-body integrator of one system (all threads of the CTA), with the
 // massive Small bodies it holds (A.nmass > nbig).
 __device__ void big_run(const MvsBigArgs& A, double* smem) {
-    const int nbig = A.nbig, N = big_count(A), nb = nbig - 1, tid = threadIdx.x, nt = blockDim.x;
+    const int nbig = A.nbig, N = big_count(A), nb = nbig - 1;
     const int stride = tab_stride(nb);
     BigSmem S;
     big_load(A, S, smem);
-    if (A.reset) {
-        if (tid == 0) big_h2j(nbig, A.m, S.X, S.V, S.XJ, S.VJ, N);
-        __syncthreads();
-        big_force(A, S, S.V);
-        write_force_table(A, S, A.tab);
-        __syncthreads();
-        if (N > nbig) small_type_force(A, S, A.tab, S.V);
-    }
-    const double h = A.h, hby2 = 0.5 * h, hm1 = 1.0 / h;
-    for (int s = 0; s < A.nsteps; ++s) {
-        for (int k = 1 + tid; k < N; k += nt)
-            for (int c = 0; c < 3; ++c) {
-                const int z = c * N + k;
-                S.XS[z] = S.X[z];
-                S.VS[z] = S.V[z];
-                S.V[z] = S.V[z] + hby2 * S.ACC[z];
-                S.X0[z] = S.X[z];
-                S.V0[z] = S.V[z];
-            }
-        __syncthreads();
-        big_drift(A, S, h);
+    const double hby2 = 0.5 * A.h;
+    // step -1 is the force alone, for the first kick of a fresh start
+    for (int s = A.reset ? -1 : 0; s < A.nsteps; ++s) {
         double* row = A.tab + (size_t)(s + 1) * stride;
-        double* det = A.detail + (size_t)s * nb * TAB_DETAIL;
-        for (int k = 1 + tid; k < nbig; k += nt) {
-            double* b = row + TAB_HEAD + (k - 1) * TAB_BODY;
-            const double pad = A.rce[k] * 1.2;
-            double lo, hi;
-            box_extent(S.X0[k], S.X[k], S.V0[k], S.V[k], h, lo, hi);
-            b[4] = lo - pad;
-            b[5] = hi + pad;
-            box_extent(S.X0[N + k], S.X[N + k], S.V0[N + k], S.V[N + k], h, lo, hi);
-            b[6] = lo - pad;
-            b[7] = hi + pad;
-            reinterpret_cast<int4*>(row + TAB_HEAD + TAB_BODY * nb)[k - 1] =
-                make_int4(order_key(b[4]) - 1, order_key(b[5]), order_key(b[6]) - 1, order_key(b[7]));
-            double* d = det + (k - 1) * TAB_DETAIL;
-            for (int c = 0; c < 3; ++c) {
-                d[c] = S.X0[c * N + k];
-                d[3 + c] = S.V0[c * N + k];
-                d[6 + c] = S.X[c * N + k];
-                d[9 + c] = S.V[c * N + k];
-            }
-            d[12] = A.rce[k];
-            d[13] = A.rphys[k];
-        }
-        // mce_stat between Big bodies (pairs 1 <= i < j < nbig), then between
-        // Big bodies and the massive Small bodies held (i < nbig <= j < N).
-        const int npair_big = nb * (nb - 1) / 2;
-        const int npair = npair_big + nb * (N - nbig);
-        for (int q = tid; q < npair; q += nt) {
-            int i = 1, j;
-            if (q < npair_big) {
-                int rem = q;
-                while (rem >= nbig - 1 - i) { rem -= nbig - 1 - i; ++i; }
-                j = i + 1 + rem;
-            } else {
-                const int r = q - npair_big;
-                i = 1 + r / (N - nbig);
-                j = nbig + r % (N - nbig);
-            }
-            double lo_i, hi_i, lo_j, hi_j, ylo_i, yhi_i, ylo_j, yhi_j;
-            const double pi_ = A.rce[i] * 1.2, pj_ = A.rce[j] * 1.2;
-            box_extent(S.X0[i], S.X[i], S.V0[i], S.V[i], h, lo_i, hi_i);
-            box_extent(S.X0[N + i], S.X[N + i], S.V0[N + i], S.V[N + i], h, ylo_i, yhi_i);
-            box_extent(S.X0[j], S.X[j], S.V0[j], S.V[j], h, lo_j, hi_j);
-            box_extent(S.X0[N + j], S.X[N + j], S.V0[N + j], S.V[N + j], h, ylo_j, yhi_j);
-            lo_i = lo_i - pi_; hi_i = hi_i + pi_; ylo_i = ylo_i - pi_; yhi_i = yhi_i + pi_;
-            lo_j = lo_j - pj_; hi_j = hi_j + pj_; ylo_j = ylo_j - pj_; yhi_j = yhi_j + pj_;
-            if (!(hi_i >= lo_j && hi_j >= lo_i && yhi_i >= ylo_j && yhi_j >= ylo_i)) continue;
-            PairEnds I{ld3(S.X0, N, i), ld3(S.V0, N, i), ld3(S.X, N, i), ld3(S.V, N, i)};
-            PairEnds J{ld3(S.X0, N, j), ld3(S.V0, N, j), ld3(S.X, N, j), ld3(S.V, N, j)};
-            PairClass pc;
-            if (pair_classify(I, J, A.rce[i], A.rce[j], A.rphys[i], A.rphys[j], h, pc)) {
-                const int slot = atomicAdd(&A.status->events, 1);
-                if (slot < A.event_cap) {
-                    pair_record(A.events + slot, I, J, pc, hm1, i + 1, j + 1, A.m[j] > A.m[i] && j < nbig);
-                    A.event_step[slot] = A.step0 + s;
-                    if (A.event_sys) A.event_sys[slot] = A.sys;
-                } else {
-                    atomicExch(&A.status->overflow, 1);
-                }
-            }
-        }
-        __syncthreads();
-        big_force(A, S, S.V);
-        write_force_table(A, S, row);
-        if (N > nbig) {
-            __syncthreads();
-            small_type_force(A, S, row, S.V);
-        }
-        for (int k = 1 + tid; k < N; k += nt)
-            for (int c = 0; c < 3; ++c) {
+        if (s >= 0) {
+            S.now = s & 1;
+            double *XS = S.XS(S.now), *VS = S.VS(S.now);
+            big_each(1, N, [&](int k, int c) {
                 const int z = c * N + k;
-                S.V[z] = S.V[z] + hby2 * S.ACC[z];
-            }
-        __syncthreads();
-        if (A.central)
-            for (int k = 1 + tid; k < N; k += nt) {
-                double temp;
-                if (central_impact(ld3(S.XS, N, k), ld3(S.VS, N, k), ld3(S.X, N, k), ld3(S.V, N, k), A.m[0],
-                                   A.m[k], h, A.rcen, temp)) {
-                    const int slot = atomicAdd(&A.status->events, 1);
-                    if (slot < A.event_cap) {
-                        MercuryEvent rec = {};
-                        rec.i = 1;
-                        rec.j = k + 1;
-                        rec.kind = EV_CENTRAL;
-                        rec.time = temp;
-                        rec.distance = A.rcen;
-                        store_event(A.events + slot, rec);
-                        A.event_step[slot] = A.step0 + s;
-                        if (A.event_sys) A.event_sys[slot] = A.sys;
-                    } else {
-                        atomicExch(&A.status->overflow, 1);
-                    }
-                }
-            }
-    }
-    __syncthreads();
-    for (int k = tid; k < N; k += nt)
-        for (int c = 0; c < 3; ++c) {
-            A.out.x[c * N + k] = S.X[c * N + k];
-            A.out.v[c * N + k] = S.V[c * N + k];
-            A.out.a[c * N + k] = S.ACC[c * N + k];
+                const double x = S.X()[z], v = S.V()[z], m = S.MS()[k];
+                XS[z] = x;
+                VS[z] = v;
+                const double v0 = v + hby2 * S.ACC()[z];
+                S.V()[z] = v0;
+                S.V0()[z] = v0;
+                S.F0()[z] = m * x;
+                S.F2()[z] = m * v0;
+            });
+            big_sync();
+        } else {
+            big_products(A, S);
         }
+        big_h2j(A, S);
+        if (s >= 0) big_drift(A, S, A.h);
+        big_force_terms(A, S, S.V());
+        write_force_rows(A, S, row);
+        if (s >= 0) big_screen(A, S, s, row, A.detail + (size_t)s * nb * TAB_DETAIL);
+        if (A.central && s > 0) big_central(A, S, s - 1);
+        big_sync();
+        big_force_sum(A, S, row);
+        big_sync();
+        if (N > nbig) small_type_force(A, S, row, S.V());
+        // each thread kicks the entries it takes into the next step itself
+        if (s >= 0)
+            big_each(1, N, [&](int k, int c) {
+                const int z = c * N + k;
+                S.V()[z] = S.V()[z] + hby2 * S.ACC()[z];
+            });
+    }
+    if (A.central && A.nsteps > 0) {
+        double *XS = S.XS(A.nsteps & 1), *VS = S.VS(A.nsteps & 1);
+        big_each(1, N, [&](int k, int c) {
+            const int z = c * N + k;
+            XS[z] = S.X()[z];
+            VS[z] = S.V()[z];
+        });
+        big_sync();
+        big_central(A, S, A.nsteps - 1);
+    }
+    big_sync();
+    for (int q = threadIdx.x; q < 3 * N; q += blockDim.x) {
+        A.out.x[q] = S.X()[q];
+        A.out.v[q] = S.V()[q];
+        A.out.a[q] = S.ACC()[q];
+    }
 }
 
-__global__ void __launch_bounds__(128) mvs_big_kernel(MvsBigArgs A) {
+__global__ void __launch_bounds__(BIG_THREADS, 1) mvs_big_kernel(const __grid_constant__ MvsBigArgs A) {
     extern __shared__ double smem[];
     big_run(A, smem);
 }
@@ -792,43 +983,35 @@ __global__ void __launch_bounds__(128, MB200_PARTICLE_MIN_BLOCKS) mvs_particle_k
 // The Big bodies' part of the corrector (mercury6_2.for:2200-2222 in
 // mco_mvs2h, 2510-2532 in mco_h2mvs) from big.in into big.out, writing the
 // force table of each of the four kicks.
-__global__ void __launch_bounds__(128) mvs_corrector_big_kernel(MvsBigArgs A, CorrectorArgs K) {
+__global__ void __launch_bounds__(BIG_THREADS, 1) mvs_corrector_big_kernel(const __grid_constant__ MvsBigArgs A, const __grid_constant__ CorrectorArgs K) {
     extern __shared__ double smem[];
-    const int nbig = A.nbig, N = big_count(A), nb = nbig - 1, tid = threadIdx.x, nt = blockDim.x;
-    const int stride = tab_stride(nb);
+    const int N = big_count(A);
+    const int stride = tab_stride(A.nbig - 1);
     BigSmem S;
     big_load(A, S, smem);
-    auto force = [&](double* row) {
-        big_force(A, S, S.V);
-        write_force_table(A, S, row);
-        if (N > nbig) {
-            __syncthreads();
-            small_type_force(A, S, row, S.V);
-        }
-    };
     auto kick = [&](double hk, bool subtract) {
-        for (int k = 1 + tid; k < N; k += nt)
-            for (int c = 0; c < 3; ++c) {
-                const int z = c * N + k;
-                const double term = hk * S.ACC[z];
-                S.V[z] = subtract ? S.V[z] - term : S.V[z] + term;
-            }
-        __syncthreads();
+        big_each(1, N, [&](int k, int c) {
+            const int z = c * N + k;
+            const double term = hk * S.ACC()[z];
+            S.V()[z] = subtract ? S.V()[z] - term : S.V()[z] + term;
+        });
+        big_sync();
     };
-    for (int k = 0; k < 2; ++k) {
-        big_drift(A, S, K.ha[k]);
-        force(A.tab + (size_t)(2 * k) * stride);
-        kick(K.hb[k], K.forward != 0);
-        big_drift(A, S, -2.0 * K.ha[k]);
-        force(A.tab + (size_t)(2 * k + 1) * stride);
-        kick(K.hb[k], K.forward == 0);
-        big_drift(A, S, K.ha[k]);
+    // drift ha, kick, drift -2 ha, kick, drift ha, twice
+#pragma unroll 1
+    for (int q = 0; q < 6; ++q) {
+        const int k = q / 3, part = q - 3 * k;
+        big_products(A, S);
+        big_h2j(A, S);
+        big_drift(A, S, part == 1 ? -2.0 * K.ha[k] : K.ha[k]);
+        if (part == 2) continue;
+        big_force(A, S, A.tab + (size_t)(2 * k + part) * stride);
+        kick(K.hb[k], part == 0 ? K.forward != 0 : K.forward == 0);
     }
-    for (int k = tid; k < N; k += nt)
-        for (int c = 0; c < 3; ++c) {
-            A.out.x[c * N + k] = S.X[c * N + k];
-            A.out.v[c * N + k] = S.V[c * N + k];
-        }
+    for (int q = threadIdx.x; q < 3 * N; q += blockDim.x) {
+        A.out.x[q] = S.X()[q];
+        A.out.v[q] = S.V()[q];
+    }
 }
 
 // The Small bodies' part: heliocentric drifts with the central mass and the
@@ -888,28 +1071,33 @@ __global__ void __launch_bounds__(256) classify_kernel(ClassifyArgs A) {
 }
 
 // ------------------------------------------------------------ batched systems
-__global__ void __launch_bounds__(32) mvs_big_batch_kernel(BatchBigArgs B) {
+__global__ void __launch_bounds__(32, 1) mvs_big_batch_kernel(BatchBigArgs B) {
     extern __shared__ double smem[];
     const int q = blockIdx.x;
-    MvsBigArgs A = B.proto[q];
-    if (B.flip) {
-        const BigState t = A.in;
-        A.in = A.out;
-        A.out = t;
+    // in shared memory: registers and local copies of it would be read slower
+    __shared__ MvsBigArgs A;
+    if (threadIdx.x == 0) {
+        A = B.proto[q];
+        if (B.flip) {
+            const BigState t = A.in;
+            A.in = A.out;
+            A.out = t;
+        }
+        A.nsteps = B.nsteps;
+        A.reset = B.reset;
+        A.central = B.central;
+        A.step0 = B.step0;
+        A.rcen = B.rcen;
+        A.tab = B.tab + B.sys[q].tab_off;
+        A.detail = B.detail + B.sys[q].det_off;
+        A.events = B.events;
+        A.event_step = B.event_step;
+        A.event_sys = B.event_sys;
+        A.event_cap = B.event_cap;
+        A.status = B.status;
+        A.sys = q;
     }
-    A.nsteps = B.nsteps;
-    A.reset = B.reset;
-    A.central = B.central;
-    A.step0 = B.step0;
-    A.rcen = B.rcen;
-    A.tab = B.tab + B.sys[q].tab_off;
-    A.detail = B.detail + B.sys[q].det_off;
-    A.events = B.events;
-    A.event_step = B.event_step;
-    A.event_sys = B.event_sys;
-    A.event_cap = B.event_cap;
-    A.status = B.status;
-    A.sys = q;
+    __syncwarp();
     big_run(A, smem);
 }
 
@@ -1046,10 +1234,10 @@ int mvs_max_steps_per_launch(int nb) {
 
 void launch_mvs_corrector(const MvsBigArgs& big, const CorrectorArgs& a, cudaStream_t s) {
     const int N = big.nmass > big.nbig ? big.nmass : big.nbig;
-    const size_t smem = sizeof(double) * ((size_t)12 * 3 * N + N + 16);
+    const size_t smem = sizeof(double) * big_smem_doubles(N);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(mvs_corrector_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    mvs_corrector_big_kernel<<<1, 128, smem, s>>>(big, a);
+    mvs_corrector_big_kernel<<<1, BIG_THREADS, smem, s>>>(big, a);
     if (a.np <= 0) return;
     const int grid = (a.np + 127) / 128;
     if (a.ngf_on) {
@@ -1062,7 +1250,7 @@ void launch_mvs_corrector(const MvsBigArgs& big, const CorrectorArgs& a, cudaStr
 }
 
 void launch_mvs_big_batch(const BatchBigArgs& a, int nsys, int max_nbig, cudaStream_t s) {
-    const size_t smem = sizeof(double) * ((size_t)12 * 3 * max_nbig + max_nbig + 16);
+    const size_t smem = sizeof(double) * big_smem_doubles(max_nbig);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(mvs_big_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (nsys > 0) mvs_big_batch_kernel<<<nsys, 32, smem, s>>>(a);
@@ -1096,10 +1284,10 @@ void launch_classify(const ClassifyArgs& a, cudaStream_t s) {
 
 void launch_mvs_big(const MvsBigArgs& a, cudaStream_t s) {
     const int N = a.nmass > a.nbig ? a.nmass : a.nbig;
-    const size_t smem = sizeof(double) * ((size_t)12 * 3 * N + N + 16);
+    const size_t smem = sizeof(double) * big_smem_doubles(N);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(mvs_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    mvs_big_kernel<<<1, 128, smem, s>>>(a);
+    mvs_big_kernel<<<1, BIG_THREADS, smem, s>>>(a);
 }
 
 void launch_mvs_particles(const MvsParticleArgs& args, cudaStream_t s, int threads) {
