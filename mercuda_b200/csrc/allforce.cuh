@@ -31,23 +31,56 @@ __host__ __device__ constexpr int force_row(int nb) { return FT_HEAD + 4 * nb; }
 // c = 299792458*86400/(AU*0.01) AU/day as mfo_grav/mfo_pr compute it.
 __device__ __forceinline__ double light_c() { return 299792458.0 * 86400.0 / (1.495978707e13 * 0.01); }
 
+// mfo_pr's drag for one body (mercury6_2.for:5300-5343), given r = |x|.
+static __device__ __noinline__ double3 pr_plain(double3 x, double3 v, double beta) {
+    const double c = light_c(), sw = 0.3;
+    const double r = sqrt(x.x * x.x + x.y * x.y + x.z * x.z);
+    const double vr = (x.x * v.x + x.y * v.y + x.z * v.z) / r;
+    const double ff = K2 * beta / (r * r);
+    return make_double3(ff * ((1.0 - (1.0 + sw) * vr / c) * x.x / r - (1.0 + sw) * v.x / c),
+                        ff * ((1.0 - (1.0 + sw) * vr / c) * x.y / r - (1.0 + sw) * v.y / c),
+                        ff * ((1.0 - (1.0 + sw) * vr / c) * x.z / r - (1.0 + sw) * v.z / c));
+}
+
+// |x|, its square and reciprocal for the central terms, rounded as sqrt and
+// 1/sqrt round them; mid: within fp64.cuh's range (else they were made by the
+// plain statements).
+struct Radius {
+    double r2, r, ri;
+    bool mid;
+};
+static __device__ __noinline__ Radius radius_plain(double r2) {
+    const double r = sqrt(r2);
+    return Radius{r2, r, 1.0 / r, false};
+}
+__device__ __forceinline__ Radius radius_of(const double3 x) {
+    Radius R;
+    R.r2 = x.x * x.x + x.y * x.y + x.z * x.z;
+    sqrt_recip(R.r2, R.r, R.ri);
+    R.mid = mid_range(R.r2);
+    return R.mid ? R : radius_plain(R.r2);
+}
+
 // The terms of mfo_all after the direct sums: indirect and central terms of
 // mfo_grav (with the fused 1PN), then mfo_obl, mfo_ngf, mfo_pr.
-// a holds the direct sum; ri = 1/|x|, r3 = ri^3.
-__device__ __forceinline__ double3 finish_force(double3 a, const double3 x, const double3 v, double ri, double r3,
+// a holds the direct sum. The drag's eight divisions and the others are made
+// by fp64.cuh's quotients from 1/r and the reciprocals of constants.
+__device__ __forceinline__ double3 finish_force(double3 a, const double3 x, const double3 v, const Radius R,
                                                const double* T, const ForceCfg& f, double mj, const double* g,
                                                DeviceStatus* st) {
+    const double ri = R.ri;
+    const double r3 = ri * ri * ri;
     const double tmp1 = f.m0 * r3;
+    const double c = light_c();
     if (f.pn == 0) {
         a.x = a.x + T[0] - tmp1 * x.x;
         a.y = a.y + T[1] - tmp1 * x.y;
         a.z = a.z + T[2] - tmp1 * x.z;
     } else {
-        const double c = light_c();
         const double light2 = c * c;
         const double rv = 0.0 + x.x * v.x + x.y * v.y + x.z * v.z;
         const double v2 = 0.0 + v.x * v.x + v.y * v.y + v.z * v.z;
-        const double ff = tmp1 / light2;
+        const double ff = quotient(tmp1, light2, 1.0 / light2);
         const double radial = 4.0 * f.m0 * ri - v2;
         a.x = a.x + T[0] - tmp1 * x.x + ff * (radial * x.x + 4.0 * rv * v.x);
         a.y = a.y + T[1] - tmp1 * x.y + ff * (radial * x.y + 4.0 * rv * v.y);
@@ -61,7 +94,7 @@ __device__ __forceinline__ double3 finish_force(double3 a, const double3 x, cons
     }
     if (f.ngflag == 1 || f.ngflag == 3) {
         double3 ng;
-        if (!nongrav_accel(x, v, g, ng)) raise_fault(st, FAULT_NGF);
+        if (!nongrav_near(x, v, R.r2, g, ng)) raise_fault(st, FAULT_NGF);
         a.x = a.x + ng.x;
         a.y = a.y + ng.y;
         a.z = a.z + ng.z;
@@ -69,13 +102,14 @@ __device__ __forceinline__ double3 finish_force(double3 a, const double3 x, cons
     if (f.ngflag == 2 || f.ngflag == 3) {
         double3 pr = make_double3(0.0, 0.0, 0.0);
         if (!(mj != 0.0 || g[3] == 0.0)) {
-            const double c = light_c(), sw = 0.3;
-            const double r = sqrt(x.x * x.x + x.y * x.y + x.z * x.z);
-            const double vr = (x.x * v.x + x.y * v.y + x.z * v.z) / r;
-            const double ff = K2 * g[3] / (r * r);
-            pr.x = ff * ((1.0 - (1.0 + sw) * vr / c) * x.x / r - (1.0 + sw) * v.x / c);
-            pr.y = ff * ((1.0 - (1.0 + sw) * vr / c) * x.y / r - (1.0 + sw) * v.y / c);
-            pr.z = ff * ((1.0 - (1.0 + sw) * vr / c) * x.z / r - (1.0 + sw) * v.z / c);
+            const double sw = 0.3, yc = 1.0 / c;
+            const double vr = quotient(x.x * v.x + x.y * v.y + x.z * v.z, R.r, ri);
+            const double ff = quotient(K2 * g[3], R.r * R.r, ri * ri);
+            const double rad = 1.0 - quotient((1.0 + sw) * vr, c, yc);
+            pr.x = ff * (quotient(rad * x.x, R.r, ri) - quotient((1.0 + sw) * v.x, c, yc));
+            pr.y = ff * (quotient(rad * x.y, R.r, ri) - quotient((1.0 + sw) * v.y, c, yc));
+            pr.z = ff * (quotient(rad * x.z, R.r, ri) - quotient((1.0 + sw) * v.z, c, yc));
+            if (!R.mid) pr = pr_plain(x, v, g[3]);
         }
         a.x = a.x + pr.x;
         a.y = a.y + pr.y;
@@ -87,28 +121,16 @@ __device__ __forceinline__ double3 finish_force(double3 a, const double3 x, cons
 
 // mfo_all for a massless Small body from a table row T (mfo_grav's direct sum
 // over the Big bodies in index order, then finish_force).
+template <int UNROLL = 4>
 __device__ __forceinline__ double3 particle_allforce(const double3 x, const double3 v, const double* T, int nb,
                                                      const ForceCfg& f, double mj, const double* g,
                                                      DeviceStatus* st) {
-    const double s2c = x.x * x.x + x.y * x.y + x.z * x.z;
-    if (s2c <= 0.0) raise_fault(st, FAULT_COINCIDENT);
-    const double ri = 1.0 / sqrt(s2c);
-    const double r3 = ri * ri * ri;
-    double3 a = make_double3(0.0, 0.0, 0.0);
-#pragma unroll 1
-    for (int b = 0; b < nb; ++b) {
-        const double* row = T + FT_HEAD + 4 * b;
-        const double dx = x.x - row[0], dy = x.y - row[1], dz = x.z - row[2];
-        const double s2 = dx * dx + dy * dy + dz * dz;
-        if (s2 <= 0.0) raise_fault(st, FAULT_COINCIDENT);
-        const double s_1 = 1.0 / sqrt(s2);
-        const double s_3 = s_1 * s_1 * s_1;
-        const double tmp1 = s_3 * row[3];
-        a.x = a.x - tmp1 * dx;
-        a.y = a.y - tmp1 * dy;
-        a.z = a.z - tmp1 * dz;
-    }
-    return finish_force(a, x, v, ri, r3, T, f, mj, g, st);
+    const Radius R = radius_of(x);
+    if (R.r2 <= 0.0) raise_fault(st, FAULT_COINCIDENT);
+    bool coincident = false;
+    const double3 a = direct_terms<4, UNROLL>(x, T + FT_HEAD, nb, &coincident);
+    if (coincident) raise_fault(st, FAULT_COINCIDENT);
+    return finish_force(a, x, v, R, T, f, mj, g, st);
 }
 
 // mfo_all for body k of the massive set, positions X/V [3][ns] in memory,
@@ -119,10 +141,8 @@ __device__ __forceinline__ double3 massive_allforce(int k, const double* X, cons
     const int N = f.nsplit;
     const double3 x = make_double3(X[k], X[N + k], X[2 * N + k]);
     const double3 v = make_double3(V[k], V[N + k], V[2 * N + k]);
-    const double s2c = x.x * x.x + x.y * x.y + x.z * x.z;
-    if (s2c <= 0.0) raise_fault(st, FAULT_COINCIDENT);
-    const double ri = 1.0 / sqrt(s2c);
-    const double r3 = ri * ri * ri;
+    const Radius R = radius_of(x);
+    if (R.r2 <= 0.0) raise_fault(st, FAULT_COINCIDENT);
     double3 a = make_double3(0.0, 0.0, 0.0);
     const int last_i = k < f.nbig ? k : f.nbig;
     for (int i = 1; i < last_i; ++i) {  // earlier Big bodies: k is their "j"
@@ -148,7 +168,7 @@ __device__ __forceinline__ double3 massive_allforce(int k, const double* X, cons
             a.y = a.y + tmp2 * dy;
             a.z = a.z + tmp2 * dz;
         }
-    return finish_force(a, x, v, ri, r3, T, f, m[k], ngfbig + 5 * k, st);
+    return finish_force(a, x, v, R, T, f, m[k], ngfbig + 5 * k, st);
 }
 
 // Row head: sx (mfo_grav's indirect sum over every body, in index order; the
@@ -271,10 +291,8 @@ __device__ __forceinline__ double3 massive_allforce_terms(int k, const double* X
     const int N = f.nsplit;
     const double3 x = make_double3(X[k], X[N + k], X[2 * N + k]);
     const double3 v = make_double3(V[k], V[N + k], V[2 * N + k]);
-    const double s2c = x.x * x.x + x.y * x.y + x.z * x.z;
-    if (s2c <= 0.0) raise_fault(st, FAULT_COINCIDENT);
-    const double ri = 1.0 / sqrt(s2c);
-    const double r3 = ri * ri * ri;
+    const Radius R = radius_of(x);
+    if (R.r2 <= 0.0) raise_fault(st, FAULT_COINCIDENT);
     double3 a = make_double3(0.0, 0.0, 0.0);
     const int ne = massive_earlier(k, f);
     const int nl = k < f.nbig ? N - k - 1 : 0;
@@ -289,7 +307,7 @@ __device__ __forceinline__ double3 massive_allforce_terms(int k, const double* X
         a.y = a.y + t[1];
         a.z = a.z + t[2];
     }
-    return finish_force(a, x, v, ri, r3, T, f, m[k], ngfbig + 5 * k, st);
+    return finish_force(a, x, v, R, T, f, m[k], ngfbig + 5 * k, st);
 }
 
 }  // namespace mb200

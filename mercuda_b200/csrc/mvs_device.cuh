@@ -87,6 +87,38 @@ __device__ __forceinline__ bool nongrav_accel(const double3 p, const double3 u, 
     return true;
 }
 
+// nongrav_accel for a body with a Yarkovsky term alone (the usual case), with
+// fp64.cuh's operations: the same roundings. r2 = |p|^2; anything else, and
+// operands out of range, goes to nongrav_accel by a call.
+static __device__ __noinline__ bool nongrav_plain(double3 p, double3 u, double g0, double g1, double g2, double g4,
+                                                  double3* a) {
+    const double g[5] = {g0, g1, g2, 0.0, g4};
+    double3 q;
+    const bool ok = nongrav_accel(p, u, g, q);
+    *a = q;
+    return ok;
+}
+__device__ __forceinline__ bool nongrav_near(const double3 p, const double3 u, double r2, const double* g, double3& a) {
+    a = make_double3(0.0, 0.0, 0.0);
+    const bool yar_only = g[0] == 0.0 && g[1] == 0.0 && g[2] == 0.0;
+    if (yar_only && g[4] == 0.0) return true;
+    const double y2 = recip_near(r2);
+    const double rv = quotient(0.0 + p.x * u.x + p.y * u.y + p.z * u.z, r2, y2);
+    const double tx = u.x - rv * p.x, ty = u.y - rv * p.y, tz = u.z - rv * p.z;
+    const double t2 = tx * tx + ty * ty + tz * tz;
+    double tn, yt;
+    sqrt_near(t2, tn, yt);
+    const double f = quotient(g[4], r2 * tn, y2 * yt);
+    if (yar_only && mid_range(r2) && mid_range(t2)) {
+        a = make_double3(f * tx, f * ty, f * tz);
+        return true;
+    }
+    double3 q;
+    const bool ok = nongrav_plain(p, u, g[0], g[1], g[2], g[4], &q);
+    a = q;
+    return ok;
+}
+
 // Acceleration of one body from the central body's J2/J4/J6 (mfo_obl,
 // mercury6_2.for:5196-5218); jcen = J2 R^2, J4 R^4, J6 R^6.
 __device__ __forceinline__ double3 oblate_accel(const double3 p, const double* jcen, double m0) {
@@ -261,14 +293,15 @@ __device__ __forceinline__ void store_event(MercuryEvent* dst, const MercuryEven
 // without a branch (fp64.cuh), and four of them overlap (in the MVS kernel 2, 4
 // and 1 at a time are within 2 %; where a CTA has few warps it is what counts). s2 outside the range
 // of those (coincident bodies among them) makes the whole sum again with plain
-// statements.
+// statements, which also report (in *coincident) an s2 <= 0.
 template <int ROW>
-static __device__ __noinline__ double3 direct_terms_plain(double3 x, const double* rows, int nb) {
+static __device__ __noinline__ double3 direct_terms_plain(double3 x, const double* rows, int nb, bool* coincident) {
     double3 a3 = make_double3(0.0, 0.0, 0.0);
     for (int b = 0; b < nb; ++b) {
         const double* row = rows + b * ROW;
         const double dx = x.x - row[0], dy = x.y - row[1], dz = x.z - row[2];
         const double s2 = dx * dx + dy * dy + dz * dz;
+        if (coincident && s2 <= 0.0) *coincident = true;
         const double s_1 = 1.0 / sqrt(s2);
         const double s_3 = s_1 * s_1 * s_1;
         const double faci = row[3] * s_3;
@@ -278,8 +311,9 @@ static __device__ __noinline__ double3 direct_terms_plain(double3 x, const doubl
     }
     return a3;
 }
-constexpr int DIRECT_UNROLL = 4;
-template <int ROW> __device__ __forceinline__ double3 direct_terms(const double3 x, const double* rows, int nb) {
+template <int ROW, int UNROLL = 4>
+__device__ __forceinline__ double3 direct_terms(const double3 x, const double* rows, int nb,
+                                                bool* coincident = nullptr) {
     double3 a3 = make_double3(0.0, 0.0, 0.0);
     unsigned bad = 0;   // each high word less 2^-511's, ORed: below 2^30 when every s2 is within 2^-511 .. 2^513
     auto term = [&](const double* row) {
@@ -300,16 +334,20 @@ template <int ROW> __device__ __forceinline__ double3 direct_terms(const double3
     };
     int b = 0;
 #pragma unroll 1
-    for (; b + DIRECT_UNROLL <= nb; b += DIRECT_UNROLL) {
-        double3 t[DIRECT_UNROLL];
+    for (; b + UNROLL <= nb; b += UNROLL) {
+        double3 t[UNROLL];
 #pragma unroll
-        for (int q = 0; q < DIRECT_UNROLL; ++q) t[q] = term(rows + (b + q) * ROW);
+        for (int q = 0; q < UNROLL; ++q) t[q] = term(rows + (b + q) * ROW);
 #pragma unroll
-        for (int q = 0; q < DIRECT_UNROLL; ++q) take(t[q]);
+        for (int q = 0; q < UNROLL; ++q) take(t[q]);
     }
 #pragma unroll 1
     for (; b < nb; ++b) take(term(rows + b * ROW));
-    if (bad >= 0x40000000u) a3 = direct_terms_plain<ROW>(x, rows, nb);
+    if (bad >= 0x40000000u) {
+        bool zero = false;
+        a3 = direct_terms_plain<ROW>(x, rows, nb, &zero);
+        if (coincident) *coincident = zero;
+    }
     return a3;
 }
 
@@ -331,7 +369,7 @@ __device__ __forceinline__ double3 small_body_force(const double3 x, const doubl
         double gc[5];
         for (int c = 0; c < 5; ++c) gc[c] = g(c);
         double3 ng;
-        if (!nongrav_accel(x, v_ngf, gc, ng)) raise_fault(st, 2);
+        if (!nongrav_near(x, v_ngf, x.x * x.x + x.y * x.y + x.z * x.z, gc, ng)) raise_fault(st, 2);
         a.x = ng.x + 0.0 + a.x;
         a.y = ng.y + 0.0 + a.y;
         a.z = ng.z + 0.0 + a.z;

@@ -378,7 +378,9 @@ template <bool STAGED> __global__ void __launch_bounds__(256) ra15_massive_kerne
 // The particles' sequence: one thread per particle slot, state in registers.
 // Three CTAs of 128 per SM (at most 168 registers, a few spilled words): 12
 // warps per SM hide the FP64 dependency chains better than the 8 the
-// unbounded 194-register build fits (0.361 -> 0.322 ms per step at 100k).
+// unbounded 194-register build fits (0.361 -> 0.322 ms per step at 100k). With
+// the branch-free force the kernel takes 113 us a sequence (149 with division
+// calls); 2 CTAs 114, 4 CTAs 148.
 constexpr int RA15_PARTICLE_THREADS = 128;
 __global__ void __launch_bounds__(RA15_PARTICLE_THREADS, 3) ra15_particle_kernel(Ra15Args A) {
     const ForceCfg& f = A.f;
