@@ -202,13 +202,18 @@ __device__ double3 hkce_particle_force_jvp(const BsArgs& A, int g, const double3
 // ------------------------------------------------------------ massive set
 // One force call of the massive set into `out` and table row T; mb and ngf
 // are the set's masses and non-gravitational constants, head a shared copy of
-// the row's head for the set's own forces, PT shared scratch for the terms
-// computed in parallel (null: the sequential loops).
+// the row's head for the set's own forces, M shared rows for the terms
+// computed in parallel (base null: the sequential loops).
 template <bool HKCE>
 __device__ void massive_call(const BsArgs& A, const double* X, const double* V, double* out, double* T,
-                             DeviceStatus* st, const double* mb, const double* ngf, double* head, double* PT) {
+                             DeviceStatus* st, const double* mb, const double* ngf, double* head,
+                             const MassiveRows M) {
     const ForceCfg& f = A.f;
     const int N = f.nsplit;
+    if (!HKCE && M.base) {
+        massive_rows_call(X, V, out, T, mb, ngf, f, M, head, st);
+        return;
+    }
     __syncthreads();
     if (HKCE) {
         for (int k = 1 + threadIdx.x; k < N; k += blockDim.x) {
@@ -222,13 +227,8 @@ __device__ void massive_call(const BsArgs& A, const double* X, const double* V, 
         __syncthreads();
         return;
     }
-    if (PT) {
-        massive_terms(X, mb, f, PT, st);
-        __syncthreads();
-    }
     if (threadIdx.x == 0) {
-        if (PT) row_head_terms(PT, f, T);
-        else row_head(X, mb, f, T);
+        row_head(X, mb, f, T);
         for (int q = 0; q < FT_HEAD; ++q) head[q] = T[q];
     }
     __syncthreads();
@@ -238,8 +238,7 @@ __device__ void massive_call(const BsArgs& A, const double* X, const double* V, 
             row[0] = X[k]; row[1] = X[N + k]; row[2] = X[2 * N + k]; row[3] = mb[k];
         }
         if (k < 1) continue;
-        const double3 a = PT ? massive_allforce_terms(k, X, V, mb, ngf, head, f, PT, st)
-                             : massive_allforce(k, X, V, mb, ngf, head, f, st);
+        const double3 a = massive_allforce(k, X, V, mb, ngf, head, f, st);
         out[k] = a.x; out[N + k] = a.y; out[2 * N + k] = a.z;
     }
     __syncthreads();
@@ -255,7 +254,7 @@ __device__ void massive_call(const BsArgs& A, const double* X, const double* V, 
 // Neville updates in level order. The start-of-step force is computed by
 // every CTA (the same statements), level 1's writing table row 0 and the
 // others a private row.
-template <int VARIANT, bool HKCE> __global__ void __launch_bounds__(256) bs_massive_level_kernel(BsArgs A) {
+template <int VARIANT, bool HKCE> __global__ void __launch_bounds__(256, 1) bs_massive_level_kernel(BsArgs A) {
     extern __shared__ double sm[];
     double h0 = A.h0;
     if (A.ctl) {
@@ -282,11 +281,18 @@ template <int VARIANT, bool HKCE> __global__ void __launch_bounds__(256) bs_mass
     const double* V0 = p + 3 * N;
     const double* mb = p + 6 * N;
     const double* ngf = p + 7 * N;
-    double* PT = massive_par_scratch(N) ? p + 12 * N : nullptr;
+    // (rounded up to an even place: the rows start on 16 bytes)
+    const MassiveRows M{!HKCE && N <= MASSIVE_PAR_MAX ? sm + (((BS_LEVEL_ROWS + 12) * N + 1) / 2 * 2) : nullptr, N};
+    if (M.base) M.clear();
     __syncthreads();
     __shared__ double head[FT_HEAD];
+    // every entry of the massive set's [3][N] vectors but the central body's
+    auto each = [&](auto g) {
+        for (int z = tid; z < 3 * N; z += nt)
+            if (z != 0 && z != N && z != 2 * N) g(z);
+    };
     auto call = [&](const double* Xc, const double* Vc, double* out, double* T, DeviceStatus* st) {
-        massive_call<HKCE>(A, Xc, Vc, out, T, st, mb, ngf, head, PT);
+        massive_call<HKCE>(A, Xc, Vc, out, T, st, mb, ngf, head, M);
     };
     for (int k = tid; k < N; k += nt)
         for (int c = 0; c < 3; ++c) {
@@ -302,69 +308,53 @@ template <int VARIANT, bool HKCE> __global__ void __launch_bounds__(256) bs_mass
     double* Dn = A.draw + (size_t)(n - 1) * 6 * N;
     if (VARIANT == 1) {
         const double hx2 = h * 2.0;
-        for (int k = 1 + tid; k < N; k += nt)
-            for (int c = 0; c < 3; ++c) {
-                const int z = c * N + k;
-                X[z] = X0[z] + h * V0[z];
-                V[z] = V0[z] + h * A0[z];
-            }
+        each([&](int z) {
+            X[z] = X0[z] + h * V0[z];
+            V[z] = V0[z] + h * A0[z];
+        });
         call(X, V, Acc, A.table + (size_t)(row++) * stride, st);
-        for (int k = 1 + tid; k < N; k += nt)
-            for (int c = 0; c < 3; ++c) {
-                const int z = c * N + k;
-                XE[z] = X0[z] + hx2 * V[z];
-                VE[z] = V0[z] + hx2 * Acc[z];
-            }
+        each([&](int z) {
+            XE[z] = X0[z] + hx2 * V[z];
+            VE[z] = V0[z] + hx2 * Acc[z];
+        });
         for (int j = 2; j <= n; ++j) {
             call(XE, VE, Acc, A.table + (size_t)(row++) * stride, st);
-            for (int k = 1 + tid; k < N; k += nt)
-                for (int c = 0; c < 3; ++c) {
-                    const int z = c * N + k;
-                    X[z] = X[z] + hx2 * VE[z];
-                    V[z] = V[z] + hx2 * Acc[z];
-                }
+            each([&](int z) {
+                X[z] = X[z] + hx2 * VE[z];
+                V[z] = V[z] + hx2 * Acc[z];
+            });
             call(X, V, Acc, A.table + (size_t)(row++) * stride, st);
-            for (int k = 1 + tid; k < N; k += nt)
-                for (int c = 0; c < 3; ++c) {
-                    const int z = c * N + k;
-                    XE[z] = XE[z] + hx2 * V[z];
-                    VE[z] = VE[z] + hx2 * Acc[z];
-                }
+            each([&](int z) {
+                XE[z] = XE[z] + hx2 * V[z];
+                VE[z] = VE[z] + hx2 * Acc[z];
+            });
         }
         call(XE, VE, Acc, A.table + (size_t)(row++) * stride, st);
-        for (int k = 1 + tid; k < N; k += nt)
-            for (int c = 0; c < 3; ++c) {
-                const int z = c * N + k;
-                Dn[z] = 0.5 * (XE[z] + X[z] + h * VE[z]);
-                Dn[3 * N + z] = 0.5 * (VE[z] + V[z] + h * Acc[z]);
-            }
+        each([&](int z) {
+            Dn[z] = 0.5 * (XE[z] + X[z] + h * VE[z]);
+            Dn[3 * N + z] = 0.5 * (VE[z] + V[z] + h * Acc[z]);
+        });
     } else {
         const double hby2 = 0.5 * h, h2by2 = 0.5 * h2n;
-        for (int k = 1 + tid; k < N; k += nt)
-            for (int c = 0; c < 3; ++c) {
-                const int z = c * N + k;
-                B[z] = 0.5 * A0[z];
-                C[z] = 0.0;
-                XE[z] = h2by2 * A0[z] + h * V0[z] + X0[z];
-            }
+        each([&](int z) {
+            B[z] = 0.5 * A0[z];
+            C[z] = 0.0;
+            XE[z] = h2by2 * A0[z] + h * V0[z] + X0[z];
+        });
         for (int j = 2; j <= n; ++j) {
             call(XE, V0, Acc, A.table + (size_t)(row++) * stride, st);
             const double tmp0 = h * double(j);
-            for (int k = 1 + tid; k < N; k += nt)
-                for (int c = 0; c < 3; ++c) {
-                    const int z = c * N + k;
-                    B[z] = B[z] + Acc[z];
-                    C[z] = C[z] + B[z];
-                    XE[z] = h2n * C[z] + h2by2 * A0[z] + tmp0 * V0[z] + X0[z];
-                }
+            each([&](int z) {
+                B[z] = B[z] + Acc[z];
+                C[z] = C[z] + B[z];
+                XE[z] = h2n * C[z] + h2by2 * A0[z] + tmp0 * V0[z] + X0[z];
+            });
         }
         call(XE, V0, Acc, A.table + (size_t)(row++) * stride, st);
-        for (int k = 1 + tid; k < N; k += nt)
-            for (int c = 0; c < 3; ++c) {
-                const int z = c * N + k;
-                Dn[z] = XE[z];
-                Dn[3 * N + z] = h * B[z] + hby2 * Acc[z] + V0[z];
-            }
+        each([&](int z) {
+            Dn[z] = XE[z];
+            Dn[3 * N + z] = h * B[z] + hby2 * Acc[z] + V0[z];
+        });
     }
 }
 
@@ -979,14 +969,14 @@ __global__ void __launch_bounds__(128) enc_post_kernel(EncPostArgs A) {
 // registers nor the code of the general force law.
 template <int VARIANT, bool HKCE> void launch_variant(const BsArgs& a, cudaStream_t s) {
     const int N = a.f.nsplit;
-    const size_t msmem = sizeof(double) * (((size_t)BS_LEVEL_ROWS + 12) * N + massive_par_scratch(N));
+    const size_t msmem = sizeof(double) * (((size_t)BS_LEVEL_ROWS + 12) * N + (HKCE ? 0 : massive_rows_doubles(N)) + 1);
     if (msmem > 48 * 1024)
         cudaFuncSetAttribute(bs_massive_level_kernel<VARIANT, HKCE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)msmem);
-    // one warp per 32 bodies, and with the parallel force terms (mfo_all)
-    // enough for one term each
+    // one warp per 32 bodies; with the parallel force terms (mfo_all) a thread
+    // for most of the pairs
     int mthreads = std::min(256, std::max(32, (N + 31) / 32 * 32));
-    if (massive_par_scratch(N) && !a.hkce) mthreads = std::max(mthreads, std::min(256, (N * N + 31) / 32 * 32));
+    if (!HKCE && N <= MASSIVE_PAR_MAX) mthreads = N <= 16 ? 128 : 256;
     bs_massive_level_kernel<VARIANT, HKCE><<<bs_levels(VARIANT), mthreads, msmem, s>>>(a);
     if (!a.fuse_extrap) bs_massive_extrap_kernel<VARIANT><<<1, mthreads, 0, s>>>(a);
     const int pblocks = (a.np > 0 ? (a.np + 31) / 32 : 0) + (a.fuse_extrap ? 1 : 0);

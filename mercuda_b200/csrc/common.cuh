@@ -32,6 +32,11 @@ constexpr int FAULT_NONFINITE = 1, FAULT_NGF = 2, FAULT_COINCIDENT = 4;
 constexpr int PCONST_ROWS = 9;
 constexpr int PC_M = 0, PC_RCE = 1, PC_RPHYS = 2, PC_NGF = 3, PC_RCRIT = 8;
 
+// Doubles in a row of terms summed in index order by one thread (eight at a
+// time, padded with zeros), one term per other body of a set of N: two more
+// than a multiple of eight, so that rows start on different banks.
+__host__ __device__ constexpr int term_row(int N) { return (N + 7) / 8 * 8 + 2; }
+
 // Device-side status word written by kernels.
 struct DeviceStatus {
     int fault;

@@ -55,8 +55,6 @@ __device__ __forceinline__ int order_key(double x) {
 // [N] scalars, the pair terms last.
 constexpr int BIG_PAIR_MAX = 33;   // bodies up to which every pair force has its slot
 constexpr int BIG_THREADS = 256;   // a warp for each of eight planets' drifts
-// (two more than a multiple of eight, so that rows start on different banks)
-__host__ __device__ constexpr int big_row(int N) { return (N + 7) / 8 * 8 + 2; }
 struct BigSmem {
     double* base;
     int N;
@@ -88,13 +86,13 @@ struct BigSmem {
     // the other body (its index less 1), padded with zeros to whole chunks of eight:
     // signed pair forces, then mfo_mvs's second indirect term of the bodies up
     // to k; and one row a coordinate of the first indirect term
-    __device__ int np() const { return big_row(N); }
+    __device__ int np() const { return term_row(N); }
     __device__ double* PT(int c, int k) const { return scal(5) + (c * N + k) * np(); }
     __device__ double* QT(int c, int k) const { return PT(3 + c, k); }
     __device__ double* RT(int c) const { return PT(6, 0) + c * np(); }
 };
 __host__ __device__ inline size_t big_smem_doubles(int N) {
-    return (size_t)(17 * 3 + 5) * N + (N <= BIG_PAIR_MAX ? (size_t)(6 * N + 3) * big_row(N) + 1 : 0);
+    return (size_t)(17 * 3 + 5) * N + (N <= BIG_PAIR_MAX ? (size_t)(6 * N + 3) * term_row(N) + 1 : 0);
 }
 
 // Bodies held by the Big-body CTA (Big, then massive Small bodies).
@@ -473,7 +471,7 @@ __device__ void big_load(const MvsBigArgs& A, BigSmem& S, double* smem) {
     }
     for (int k = tid; k < N; k += nt) S.MS()[k] = A.m[k];
     if (N <= BIG_PAIR_MAX)
-        for (int q = tid; q < (6 * N + 3) * big_row(N); q += nt) S.PT(0, 0)[q] = 0.0;
+        for (int q = tid; q < (6 * N + 3) * term_row(N); q += nt) S.PT(0, 0)[q] = 0.0;
     big_sync();
     big_constants(A, S);
 }

@@ -210,7 +210,8 @@ __device__ __forceinline__ void atomic_max_abs(unsigned long long* dst, double v
 }
 
 // The massive set's sequence: one CTA. Writes table rows 0 (sequence start)
-// and 1 + (n-1)*7 + (j-2) (iteration n, node j) for the particles. With
+// and 1 + (n-1)*7 + (j-2) (iteration n, node j) for the particles. Sets of more
+// than MASSIVE_PAR_MAX bodies (smaller ones: ra15_massive_rows_kernel). With
 // STAGED the set's positions, velocities, B, G, accelerations, masses and
 // non-gravitational constants live in shared memory for the whole sequence
 // (the set is small and every node reads all of it after a barrier); B, G
@@ -223,7 +224,7 @@ template <bool STAGED> __global__ void __launch_bounds__(256) ra15_massive_kerne
     const bool vpred = (f.ngflag != 0 || f.pn == 1);
     __shared__ double blockmax[8];
     __shared__ double head[FT_HEAD];
-    double *X, *V, *B, *G, *a1, *PT = nullptr;
+    double *X, *V, *B, *G, *a1;
     const double *x1, *v1, *mb, *ngf;
     if (STAGED) {
         X = sm;
@@ -235,7 +236,6 @@ template <bool STAGED> __global__ void __launch_bounds__(256) ra15_massive_kerne
         double* sv1 = sx1 + 3 * N;
         double* smb = sv1 + 3 * N;
         double* sngf = smb + N;
-        PT = massive_par_scratch(N) ? sngf + 5 * N : nullptr;
         for (int q = tid; q < 3 * N; q += nt) {
             sx1[q] = A.bx[q];
             sv1[q] = A.bx[3 * N + q];
@@ -260,24 +260,15 @@ template <bool STAGED> __global__ void __launch_bounds__(256) ra15_massive_kerne
         ngf = A.ngfbig;
     }
     // the head of a table row: written to the table for the particles and
-    // kept in shared memory for the massive set's forces
-    // (with PT the force terms are computed by every thread first; the
-    // caller synchronizes before and after)
+    // kept in shared memory for the massive set's forces (the caller
+    // synchronizes before and after)
     auto write_head = [&](double* T) {
-        if (PT) {
-            massive_terms(X, mb, f, PT, A.status);
-            __syncthreads();
-        }
         if (tid == 0) {
-            if (PT) row_head_terms(PT, f, T);
-            else row_head(X, mb, f, T);
+            row_head(X, mb, f, T);
             for (int q = 0; q < FT_HEAD; ++q) head[q] = T[q];
         }
     };
-    auto force = [&](int k, const double* Vc) {
-        return PT ? massive_allforce_terms(k, X, Vc, mb, ngf, head, f, PT, A.status)
-                  : massive_allforce(k, X, Vc, mb, ngf, head, f, A.status);
-    };
+    auto force = [&](int k, const double* Vc) { return massive_allforce(k, X, Vc, mb, ngf, head, f, A.status); };
     double localmax = 0.0;
     // sequence start: force at (x1, v1), G from B
     for (int k = tid; k < N; k += nt)
@@ -371,6 +362,75 @@ template <bool STAGED> __global__ void __launch_bounds__(256) ra15_massive_kerne
     if (tid == 0) {
         double mx = 0.0;
         for (int w = 0; w < (nt + 31) / 32; ++w) mx = fmax(mx, blockmax[w]);
+        atomic_max_abs(A.maxb7, mx);
+    }
+}
+
+// The same for sets of up to MASSIVE_PAR_MAX bodies: a thread per (body,
+// coordinate) keeps its B, G, a1, x1 and v1 in registers for the whole
+// sequence, and each force call is massive_rows_call. What bounds it is the
+// chain of 15 (43 at a start) force calls; the particles wait for it. Eight
+// planets: 70 us a sequence by the kernel above, 31 us so.
+__global__ void __launch_bounds__(256) ra15_massive_rows_kernel(const __grid_constant__ Ra15Args A) {
+    extern __shared__ double sm[];
+    const ForceCfg& f = A.f;
+    const int N = f.nsplit, tid = threadIdx.x, nt = blockDim.x;
+    const int stride = force_row(f.nbig - 1);
+    const bool vpred = (f.ngflag != 0 || f.pn == 1);
+    __shared__ double head[FT_HEAD];
+    __shared__ double blockmax[8];
+    __shared__ Pred pred[7];
+    const MassiveRows M{sm, N};
+    double* X = sm + (massive_rows_doubles(N) + 1) / 2 * 2;
+    double* V = X + 3 * N;
+    double* ACC = V + 3 * N;
+    double* mb = ACC + 3 * N;
+    double* ngf = mb + N;
+    M.clear();
+    for (int q = tid; q < N; q += nt) mb[q] = A.mbig[q];
+    for (int q = tid; q < 5 * N; q += nt) ngf[q] = A.ngfbig[q];
+    if (tid >= nt - 7) pred[tid - (nt - 7)] = predictor(A.t, tid - (nt - 7) + 2);
+    const bool live = tid < 3 * (N - 1);
+    const int k = live ? 1 + tid / 3 : 1, c = live ? tid - 3 * (k - 1) : 0, z = c * N + k;
+    double x1 = 0.0, v1 = 0.0, a1 = 0.0, b[7], g[7];
+    if (live) {
+        x1 = A.bx[z];
+        v1 = A.bx[3 * N + z];
+        X[z] = x1;
+        V[z] = v1;
+    }
+#pragma unroll
+    for (int m = 0; m < 7; ++m) b[m] = A.reset || !live ? 0.0 : A.bb[(c * 7 + m) * N + k];
+    massive_rows_call(X, V, ACC, A.table, mb, ngf, f, M, head, A.status);
+    if (live) a1 = ACC[z];
+    g_from_b(b, g);
+#pragma unroll 1
+    for (int r = 0; r < 7 * A.niter; ++r) {
+        const int j = 2 + r % 7;
+        if (live) {
+            X[z] = pred_x(pred[j - 2], b, a1, v1, x1);
+            if (vpred) V[z] = pred_v(pred[j - 2], b, a1, v1);
+        }
+        massive_rows_call(X, V, ACC, A.table + (size_t)(1 + r) * stride, mb, ngf, f, M, head, A.status);
+        if (live) update_gb(j, ACC[z], a1, g, b);
+    }
+    double localmax = 0.0;
+    if (live) {
+#pragma unroll
+        for (int m = 0; m < 7; ++m) {
+            A.bb[(c * 7 + m) * N + k] = b[m];
+            A.bg[(c * 7 + m) * N + k] = g[m];
+        }
+        A.bx_a1[z] = a1;
+        if (!isfinite(b[6])) raise_fault(A.status, FAULT_NONFINITE);
+        else localmax = fabs(b[6]);
+    }
+    for (int o = 16; o; o >>= 1) localmax = fmax(localmax, __shfl_xor_sync(FULLMASK, localmax, o));
+    if ((tid & 31) == 0) blockmax[tid >> 5] = localmax;
+    __syncthreads();
+    if (tid == 0) {
+        double mx = 0.0;
+        for (int w = 0; w < nt / 32; ++w) mx = fmax(mx, blockmax[w]);
         atomic_max_abs(A.maxb7, mx);
     }
 }
@@ -655,18 +715,24 @@ int nblocks(int n, int t) { return (n + t - 1) / t; }
 void launch_ra15_sequence(const Ra15Args& a, cudaStream_t s) {
     ensure_constants();
     const int N = a.f.nsplit;
-    // x, v, B, G, a1, x1, v1 (57 N), m, ngf, then the force terms
-    const size_t smem = sizeof(double) * ((size_t)63 * N + massive_par_scratch(N));
-    if (smem <= 200 * 1024) {
+    if (N <= MASSIVE_PAR_MAX) {
+        // four warps hold a thread for each of the largest set's coordinates;
+        // eight give each of its pairs one
+        const size_t smem = sizeof(double) * (size_t)(massive_rows_doubles(N) + 1 + 15 * N);
         if (smem > 48 * 1024)
-            cudaFuncSetAttribute(ra15_massive_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        // one warp per 32 bodies, at most 8, and with the parallel force terms
-        // enough for one term each
-        int threads = std::min(256, std::max(32, (N + 31) / 32 * 32));
-        if (massive_par_scratch(N)) threads = std::max(threads, std::min(256, (N * N + 31) / 32 * 32));
-        ra15_massive_kernel<true><<<1, threads, smem, s>>>(a);
+            cudaFuncSetAttribute(ra15_massive_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        ra15_massive_rows_kernel<<<1, N <= 16 ? 128 : 256, smem, s>>>(a);
     } else {
-        ra15_massive_kernel<false><<<1, 256, 0, s>>>(a);
+        // x, v, B, G, a1, x1, v1 (57 N), m, ngf
+        const size_t smem = sizeof(double) * (size_t)63 * N;
+        if (smem <= 200 * 1024) {
+            if (smem > 48 * 1024)
+                cudaFuncSetAttribute(ra15_massive_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            // one warp per 32 bodies, at most 8
+            ra15_massive_kernel<true><<<1, std::min(256, (N + 31) / 32 * 32), smem, s>>>(a);
+        } else {
+            ra15_massive_kernel<false><<<1, 256, 0, s>>>(a);
+        }
     }
     if (a.np > 0) ra15_particle_kernel<<<nblocks(a.np, RA15_PARTICLE_THREADS), RA15_PARTICLE_THREADS, 0, s>>>(a);
 }
