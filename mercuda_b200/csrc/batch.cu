@@ -14,7 +14,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
 #include <tuple>
 #include <vector>
 
@@ -28,11 +27,12 @@ namespace {
 constexpr int BATCH_MAX_NBIG = 32;
 
 struct Batch {
-    int nsys = 0, nbody = 0, npcap = 0, ntiles = 0, max_nbig = 1, K = 31;
+    int nsys = 0, nbody = 0, npcap = 0, ntiles = 0, nbigs = 0, max_nbig = 1, max_body = 1, K = 31;
     std::vector<int> body_off, nbig, np, first_slot, big_off;
     std::vector<double> h, mu;
     std::vector<BatchSys> sys;
     DBuf<BatchSys> d_sys;
+    DBuf<int> d_body_end;
     DBuf<BatchTile> d_tiles;
     DBuf<MvsBigArgs> d_proto;
     DBuf<double> bigbuf[2];          // per system [9][nbig] at 9 * big_off
@@ -41,6 +41,7 @@ struct Batch {
     DBuf<double> prce, prphys;
     DBuf<int> plocal;
     DBuf<double> tab[2], det[2];
+    DBuf<double> stage;              // the host arrays as they are: x, v (3 a body), m, rce, rphys
     size_t tab_size = 0, det_size = 0;
     DBuf<MercuryEvent> events;
     DBuf<int> event_step, event_sys;
@@ -67,9 +68,10 @@ struct Batch {
 
     void release() {
         DBuf<double>* d[] = {&bigbuf[0], &bigbuf[1], &bm, &brce, &brphys, &pstate[0], &pstate[1],
-                             &prce, &prphys, &tab[0], &tab[1], &det[0], &det[1], &snap};
+                             &prce, &prphys, &tab[0], &tab[1], &det[0], &det[1], &snap, &stage};
         for (auto* b : d) b->release();
         d_sys.release();
+        d_body_end.release();
         d_tiles.release();
         d_proto.release();
         plocal.release();
@@ -115,13 +117,78 @@ Batch& batch() {
     return b;
 }
 
-__global__ void batch_layout_kernel(const double* rows, int n, int comps, const int* dst_index, double* dst,
-                                    int stride) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const int d = dst_index[j];
-    if (d < 0) return;
-    for (int c = 0; c < comps; ++c) dst[(size_t)c * stride + d] = rows[(size_t)j * comps + c];
+// Between the host arrays' rows (staged on the device) and the batch's
+// layout, one block per system and BATCH_CHUNK bodies of it: Big bodies to
+// [9][nbig] at 9 big_off, particles to their slots. GATHER takes positions and
+// velocities back to rows.
+constexpr int BATCH_CHUNK = 1024;
+struct BatchRows {
+    const BatchSys* sys;
+    const int* body_end;      // first row past each system
+    double *x, *v;            // rows, 3 a body
+    const double *m, *rce, *rphys;
+    double* big;
+    double* part;
+    size_t npcap;
+    double *bm, *brce, *brphys, *prce, *prphys;
+    int* local;
+};
+template <bool GATHER> __global__ void __launch_bounds__(128) batch_rows_kernel(BatchRows A) {
+    const BatchSys S = A.sys[blockIdx.x];
+    const int n = A.body_end[blockIdx.x] - S.body;
+    const int j1 = min(n, (int)(blockIdx.y + 1) * BATCH_CHUNK);
+    for (int j = blockIdx.y * BATCH_CHUNK + threadIdx.x; j < j1; j += blockDim.x) {
+        const size_t row = S.body + j;
+        double* x = A.x + 3 * row;
+        double* v = A.v + 3 * row;
+        const bool is_big = j < S.nbig;
+        const int q = j - S.nbig;
+        const size_t slot = S.first_slot + q, st = is_big ? S.nbig : A.npcap;
+        double* d = is_big ? A.big + 9 * (size_t)S.big_off + j : A.part + slot;
+        for (int c = 0; c < 3; ++c) {
+            if (GATHER) {
+                x[c] = d[c * st];
+                v[c] = d[(3 + c) * st];
+            } else {
+                d[c * st] = x[c];
+                d[(3 + c) * st] = v[c];
+                d[(6 + c) * st] = 0.0;
+            }
+        }
+        if (GATHER) continue;
+        if (is_big) {
+            A.bm[S.big_off + j] = A.m[row];
+            A.brce[S.big_off + j] = A.rce[row];
+            A.brphys[S.big_off + j] = A.rphys[row];
+        } else {
+            A.prce[slot] = A.rce[row];
+            A.prphys[slot] = A.rphys[row];
+            A.local[slot] = q;
+        }
+    }
+}
+template <bool GATHER> void launch_batch_rows(Batch& B) {
+    const size_t n = B.nbody;
+    BatchRows a{};
+    a.sys = B.d_sys.p;
+    a.body_end = B.d_body_end.p;
+    a.x = B.stage.p;
+    a.v = a.x + 3 * n;
+    a.m = a.v + 3 * n;
+    a.rce = a.m + n;
+    a.rphys = a.rce + n;
+    a.big = B.bigbuf[B.cur].p;
+    a.part = B.pstate[B.cur].p;
+    a.npcap = B.npcap;
+    a.bm = B.bm.p;
+    a.brce = B.brce.p;
+    a.brphys = B.brphys.p;
+    a.prce = B.prce.p;
+    a.prphys = B.prphys.p;
+    a.local = B.plocal.p;
+    const dim3 grid(B.nsys, (B.max_body + BATCH_CHUNK - 1) / BATCH_CHUNK);
+    batch_rows_kernel<GATHER><<<grid, 128, 0, B.stream>>>(a);
+    check(cudaGetLastError(), "batch rows");
 }
 
 // Table and detail offsets of every system for K steps per chunk, and the
@@ -248,7 +315,7 @@ void tune(Batch& B, double rcen, int nsteps) {
     B.threads = Ts[0];
     B.tuned_K = Ks[0];
     if (B.ntiles == 0 || (Ks.size() == 1 && Ts.size() == 1)) return;
-    const size_t bigs = B.bm.n;
+    const size_t bigs = (size_t)B.nbigs;
     auto copy = [&](void* d, const void* src, size_t bytes) {
         check(cudaMemcpyAsync(d, src, bytes, cudaMemcpyDeviceToDevice, B.stream), "tune");
     };
@@ -281,25 +348,50 @@ void tune(Batch& B, double rcen, int nsteps) {
     check(cudaGetLastError(), "tune");
 }
 
+// The records in (system, step, min id, max id) order; equal keys keep the
+// order in which they came.
 void sort_batch_events(Batch& B) {
-    const size_t n = B.host_events.size();
-    std::vector<size_t> idx(n);
-    for (size_t k = 0; k < n; ++k) idx[k] = k;
-    auto key = [&](size_t k) {
-        const MercuryEvent& e = B.host_events[k];
-        return std::make_tuple(B.host_sys[k], B.host_step[k], std::min(e.i, e.j), std::max(e.i, e.j));
+    struct Key {
+        uint64_t where, pair;
+        uint32_t at;
     };
-    std::stable_sort(idx.begin(), idx.end(), [&](size_t a, size_t b) { return key(a) < key(b); });
+    const size_t n = B.host_events.size();
+    std::vector<Key> keys(n);
+    for (size_t k = 0; k < n; ++k) {
+        const MercuryEvent& e = B.host_events[k];
+        keys[k] = Key{(uint64_t)(uint32_t)B.host_sys[k] << 32 | (uint32_t)B.host_step[k],
+                      (uint64_t)(uint32_t)std::min(e.i, e.j) << 32 | (uint32_t)std::max(e.i, e.j), (uint32_t)k};
+    }
+    std::sort(keys.begin(), keys.end(), [](const Key& a, const Key& b) {
+        return a.where != b.where ? a.where < b.where : a.pair != b.pair ? a.pair < b.pair : a.at < b.at;
+    });
     std::vector<MercuryEvent> e(n);
     std::vector<int> sy(n), st(n);
     for (size_t k = 0; k < n; ++k) {
-        e[k] = B.host_events[idx[k]];
-        sy[k] = B.host_sys[idx[k]];
-        st[k] = B.host_step[idx[k]];
+        e[k] = B.host_events[keys[k].at];
+        sy[k] = B.host_sys[keys[k].at];
+        st[k] = B.host_step[keys[k].at];
     }
     B.host_events.swap(e);
     B.host_sys.swap(sy);
     B.host_step.swap(st);
+}
+
+// Room for a run's records and one chunk's candidates, so that a run need not
+// be made again: the package's workloads give up to 8 records and 400
+// candidates per 10,000 particle-steps (the first is capped at 4M records;
+// an overflow still grows the buffers and redoes the run).
+void size_records(Batch& B, int nsteps, int K) {
+    const long long slots = B.npcap;
+    const size_t records = (size_t)std::min<long long>(4 << 20, slots * nsteps / 1000);
+    const size_t cands = (size_t)std::min<long long>(INT32_MAX / 2, slots * K / 25);
+    if (records > B.events.n || cands > B.cands.n) {
+        B.events.reserve(records);
+        B.event_step.reserve(B.events.n);
+        B.event_sys.reserve(B.events.n);
+        B.cands.reserve(cands);
+        ++B.epoch;
+    }
 }
 
 }  // namespace
@@ -315,10 +407,16 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
     try {
         if (nsys < 1) throw std::runtime_error("batch needs at least one system");
         B.ensure_streams();
-        B.release();
-        B.nsys = nsys;
+        // the buffers of an earlier batch stay (batch_free gives them back);
+        // its graph, records and sizes do not
+        B.drop_graph();
+        B.host_events.clear();
+        B.host_sys.clear();
+        B.host_step.clear();
+        ++B.epoch;
+        B.nsys = 0;
         B.body_off.assign(body_offset, body_offset + nsys + 1);
-        B.nbody = B.body_off[nsys];
+        B.nbody = body_offset[nsys];
         B.nbig.assign(nbig, nbig + nsys);
         B.h.assign(h, h + nsys);
         B.np.resize(nsys);
@@ -327,6 +425,7 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
         B.mu.resize(nsys);
         B.sys.resize(nsys);
         B.max_nbig = 1;
+        B.max_body = 1;
         int slots = 0, bigs = 0;
         std::vector<BatchTile> tiles;
         for (int s = 0; s < nsys; ++s) {
@@ -334,6 +433,7 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
             if (n < 1 || B.nbig[s] < 1 || B.nbig[s] > n) throw std::runtime_error("invalid body counts of a system");
             if (B.nbig[s] > BATCH_MAX_NBIG) throw std::runtime_error("more than 32 Big bodies in a batched system");
             if (!(B.h[s] != 0.0) || !std::isfinite(B.h[s])) throw std::runtime_error("invalid step of a system");
+            B.max_body = std::max(B.max_body, n);
             for (int j = B.body_off[s] + B.nbig[s]; j < B.body_off[s + 1]; ++j)
                 if (m[j] != 0.0) throw std::runtime_error("batched systems take massless Small bodies only");
             B.np[s] = n - B.nbig[s];
@@ -351,9 +451,12 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
             S.nb = B.nbig[s] - 1;
             S.first_slot = B.first_slot[s];
             S.np = B.np[s];
+            S.body = B.body_off[s];
+            S.big_off = B.big_off[s];
         }
         B.npcap = std::max(1, slots);
         B.ntiles = (int)tiles.size();
+        B.nbigs = bigs;
         B.d_sys.reserve(nsys);
         B.d_tiles.reserve(std::max(1, B.ntiles));
         B.d_proto.reserve(nsys);
@@ -373,62 +476,17 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
         B.cands.reserve(std::max(16384, slots / 2));
         B.status.reserve(1);
         B.snap.reserve((size_t)9 * B.npcap + (size_t)9 * bigs);
-        if (B.ntiles)
-            h2d(B.d_tiles.p, tiles.data(), sizeof(BatchTile) * B.ntiles, B.stream);
-        // destination index of every body: Big rows at 9 * big_off + k (stride
-        // nbig within the system) are written per component below; particles
-        // go to their slot
-        std::vector<int> slot_of(B.nbody, -1), local(B.npcap, 0);
-        std::vector<double> hb(9 * (size_t)bigs, 0.0), hm(bigs), hrce(bigs), hrph(bigs);
-        for (int s = 0; s < nsys; ++s) {
-            const int o = B.body_off[s], nb = B.nbig[s];
-            double* base = hb.data() + 9 * (size_t)B.big_off[s];
-            for (int k = 0; k < nb; ++k) {
-                for (int c = 0; c < 3; ++c) {
-                    base[c * nb + k] = xx[3 * (size_t)(o + k) + c];
-                    base[(3 + c) * nb + k] = vv[3 * (size_t)(o + k) + c];
-                }
-                hm[B.big_off[s] + k] = m[o + k];
-                hrce[B.big_off[s] + k] = rce[o + k];
-                hrph[B.big_off[s] + k] = rphys[o + k];
-            }
-            for (int q = 0; q < B.np[s]; ++q) {
-                slot_of[o + nb + q] = B.first_slot[s] + q;
-                local[B.first_slot[s] + q] = q;
-            }
-        }
-        h2d(B.bigbuf[0].p, hb.data(), sizeof(double) * hb.size(), B.stream);
-        check(cudaMemsetAsync(B.bigbuf[1].p, 0, sizeof(double) * hb.size(), B.stream), "upload");
-        h2d(B.bm.p, hm.data(), sizeof(double) * bigs, B.stream);
-        h2d(B.brce.p, hrce.data(), sizeof(double) * bigs, B.stream);
-        h2d(B.brphys.p, hrph.data(), sizeof(double) * bigs, B.stream);
-        h2d(B.plocal.p, local.data(), sizeof(int) * B.npcap, B.stream);
-        // (on the stream of the layout kernels below, so that they run after)
-        check(cudaMemsetAsync(B.pstate[0].p, 0, sizeof(double) * 9 * B.npcap, B.stream), "upload");
-        check(cudaMemsetAsync(B.pstate[1].p, 0, sizeof(double) * 9 * B.npcap, B.stream), "upload");
-        // particle rows through a device staging copy of the host arrays
-        DBuf<double> stage;
-        DBuf<int> dst;
-        stage.reserve((size_t)3 * B.nbody);
-        dst.reserve(B.nbody);
-        h2d(dst.p, slot_of.data(), sizeof(int) * B.nbody, B.stream);
-        const int blocks = (B.nbody + 255) / 256;
-        for (int part = 0; part < 2; ++part) {
-            h2d(stage.p, part ? vv : xx, sizeof(double) * 3 * B.nbody, B.stream);
-            batch_layout_kernel<<<blocks, 256, 0, B.stream>>>(stage.p, B.nbody, 3, dst.p,
-                                                               B.pstate[0].p + (size_t)3 * part * B.npcap, B.npcap);
-            check(cudaStreamSynchronize(B.stream), "upload");
-        }
-        const double* scal[2] = {rce, rphys};
-        double* sdst[2] = {B.prce.p, B.prphys.p};
-        for (int q = 0; q < 2; ++q) {
-            h2d(stage.p, scal[q], sizeof(double) * B.nbody, B.stream);
-            batch_layout_kernel<<<blocks, 256, 0, B.stream>>>(stage.p, B.nbody, 1, dst.p, sdst[q], B.npcap);
-            check(cudaStreamSynchronize(B.stream), "upload");
-        }
-        check(cudaGetLastError(), "upload");
-        stage.release();
-        dst.release();
+        // every host array in one round of copies; layout on the device
+        const size_t n = B.nbody;
+        B.stage.reserve(9 * n);
+        B.d_body_end.reserve(nsys);
+        std::vector<HostSpan> spans = {
+            {B.stage.p, const_cast<double*>(xx), 24 * n},        {B.stage.p + 3 * n, const_cast<double*>(vv), 24 * n},
+            {B.stage.p + 6 * n, const_cast<double*>(m), 8 * n},  {B.stage.p + 7 * n, const_cast<double*>(rce), 8 * n},
+            {B.stage.p + 8 * n, const_cast<double*>(rphys), 8 * n},
+            {B.d_body_end.p, B.body_off.data() + 1, sizeof(int) * nsys}};
+        if (B.ntiles) spans.push_back({B.d_tiles.p, tiles.data(), sizeof(BatchTile) * B.ntiles});
+        copy_in(spans, B.stream);
         // per-system Big-body argument templates (in = set 0, out = set 1)
         std::vector<MvsBigArgs> proto(nsys);
         for (int s = 0; s < nsys; ++s) {
@@ -448,8 +506,13 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
             }
         }
         h2d(B.d_proto.p, proto.data(), sizeof(MvsBigArgs) * nsys, B.stream);
-        layout_tables(B, B.forced_K > 0 ? B.forced_K : 31);
+        B.nsys = nsys;
         B.cur = 0;
+        layout_tables(B, B.forced_K > 0 ? B.forced_K : 31);   // copies the systems' records
+        launch_batch_rows<false>(B);
+        check(cudaMemsetAsync(B.bigbuf[1].p, 0, sizeof(double) * 9 * bigs, B.stream), "upload");
+        check(cudaMemsetAsync(B.pstate[1].p, 0, sizeof(double) * 9 * B.npcap, B.stream), "upload");
+        check(cudaStreamSynchronize(B.stream), "upload");
         B.reset = true;
         B.threads = 0;
         B.tuned_K = 31;
@@ -469,11 +532,12 @@ int mercury_b200_batch_advance(double time, int nsteps, double rcen, int* nevent
         int K = B.forced_K > 0 ? B.forced_K : B.tuned_K;
         K = std::max(1, std::min(K, nsteps));
         if (K != B.K) layout_tables(B, K);
+        size_records(B, nsteps, K);
         const int nchunks = (nsteps + K - 1) / K;
         B.ensure_chunk_events(std::max(2, nchunks));
         const int reset0 = B.reset ? 1 : 0;
         // starting state, for a redo after an event-buffer overflow
-        const size_t bigs = B.bm.n;
+        const size_t bigs = (size_t)B.nbigs;
         auto copy = [&](void* d, const void* s, size_t bytes) {
             check(cudaMemcpyAsync(d, s, bytes, cudaMemcpyDeviceToDevice, B.stream), "snapshot");
         };
@@ -533,21 +597,19 @@ int mercury_b200_batch_advance(double time, int nsteps, double rcen, int* nevent
                   "events");
         }
         // absolute times on each system's own clock (time = time + h per step)
-        std::map<int, std::vector<double>> tend;
+        std::vector<std::vector<double>> tend(B.nsys);
         for (int k = 0; k < nev; ++k) {
             const int s = B.host_sys[k];
-            auto it = tend.find(s);
-            if (it == tend.end()) {
-                std::vector<double> t(nsteps);
+            if (tend[s].empty()) {
+                tend[s].resize(nsteps);
                 double tt = time;
                 for (int q = 0; q < nsteps; ++q) {
                     tt = tt + B.h[s];
-                    t[q] = tt;
+                    tend[s][q] = tt;
                 }
-                it = tend.emplace(s, std::move(t)).first;
             }
             MercuryEvent& e = B.host_events[k];
-            const double te = it->second[B.host_step[k]];
+            const double te = tend[s][B.host_step[k]];
             if (e.kind == EV_CENTRAL) e.time = te - B.h[s] + e.time;
             else e.time = e.time + te;
         }
@@ -575,28 +637,11 @@ int mercury_b200_batch_download(double* xx, double* vv) {
     Batch& B = batch();
     try {
         if (B.nsys < 1) throw std::runtime_error("no batch uploaded");
-        const size_t bigs = B.bm.n;
-        std::vector<double> hb(9 * bigs), hp(6 * (size_t)B.npcap);
-        check(cudaMemcpy(hb.data(), B.bigbuf[B.cur].p, sizeof(double) * hb.size(), cudaMemcpyDeviceToHost),
-              "download");
-        check(cudaMemcpy(hp.data(), B.pstate[B.cur].p, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost),
-              "download");
-        for (int s = 0; s < B.nsys; ++s) {
-            const int o = B.body_off[s], nb = B.nbig[s];
-            const double* base = hb.data() + 9 * (size_t)B.big_off[s];
-            for (int k = 0; k < nb; ++k)
-                for (int c = 0; c < 3; ++c) {
-                    xx[3 * (size_t)(o + k) + c] = base[c * nb + k];
-                    vv[3 * (size_t)(o + k) + c] = base[(3 + c) * nb + k];
-                }
-            for (int q = 0; q < B.np[s]; ++q) {
-                const size_t slot = (size_t)B.first_slot[s] + q;
-                for (int c = 0; c < 3; ++c) {
-                    xx[3 * (size_t)(o + nb + q) + c] = hp[c * (size_t)B.npcap + slot];
-                    vv[3 * (size_t)(o + nb + q) + c] = hp[(3 + c) * (size_t)B.npcap + slot];
-                }
-            }
-        }
+        const size_t n = B.nbody;
+        launch_batch_rows<true>(B);
+        const size_t o = B.body_off[0];   // rows before the first system are not the batch's
+        copy_out({{B.stage.p + 3 * o, xx + 3 * o, 24 * (n - o)}, {B.stage.p + 3 * (n + o), vv + 3 * o, 24 * (n - o)}},
+                 B.stream);
         return 0;
     } catch (const std::exception& e) {
         return report(e);
