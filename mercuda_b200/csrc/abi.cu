@@ -196,14 +196,53 @@ int g_event_cap = 0;
 
 // Adds the device time of one drop-in call (CUDA events on the library
 // stream around it) to the total.
+// With `later`, the call does not wait for its end: the pair of events is
+// read when its time is asked for, or when newer ones need the room.
+struct TimedCall {
+    cudaEvent_t begin, end;
+};
+std::vector<TimedCall> g_timed_free, g_timed;   // g_timed: in order of recording
+void settle_timers(size_t keep) {
+    while (g_timed.size() > keep) {
+        float ms = 0.0f;
+        const TimedCall q = g_timed.front();
+        if (cudaEventSynchronize(q.end) == cudaSuccess && cudaEventElapsedTime(&ms, q.begin, q.end) == cudaSuccess)
+            g_dropin_ms += ms;
+        g_timed.erase(g_timed.begin());
+        g_timed_free.push_back(q);
+    }
+}
 struct DropinTimer {
     Context& c;
-    DropinTimer() : c(ctx()) { check(cudaEventRecord(c.d0, c.stream), "event"); }
+    bool later;
+    TimedCall q;
+    explicit DropinTimer(bool later_ = false) : c(ctx()), later(later_), q{c.d0, c.d1} {
+        if (later) {
+            if (g_timed_free.empty()) {
+                TimedCall fresh{};
+                check(cudaEventCreate(&fresh.begin), "event");
+                check(cudaEventCreate(&fresh.end), "event");
+                g_timed_free.push_back(fresh);
+            }
+            q = g_timed_free.back();
+            g_timed_free.pop_back();
+        }
+        check(cudaEventRecord(q.begin, c.stream), "event");
+    }
     ~DropinTimer() {
         float ms = 0.0f;
-        if (cudaEventRecord(c.d1, c.stream) == cudaSuccess && cudaEventSynchronize(c.d1) == cudaSuccess &&
-            cudaEventElapsedTime(&ms, c.d0, c.d1) == cudaSuccess)
+        const bool recorded = cudaEventRecord(q.end, c.stream) == cudaSuccess;
+        if (later) {
+            if (!recorded) {
+                g_timed_free.push_back(q);
+                return;
+            }
+            g_timed.push_back(q);
+            settle_timers(16);
+        } else if (recorded && cudaEventSynchronize(q.end) == cudaSuccess &&
+                   cudaEventElapsedTime(&ms, q.begin, q.end) == cudaSuccess) {
             g_dropin_ms += ms;
+        }
     }
 };
 
@@ -421,6 +460,7 @@ void spec_drop() {
 void drop_speculation() {
     spec_drop();
     ctx().head_ready = false;
+    ctx().screen_live = false;
 }
 
 // Resizes b to exactly n elements (a swapped-in record buffer keeps the
@@ -635,7 +675,6 @@ void ra15_step_once(double time, double* h, double* hdid, double tol, int64_t* r
         const int niter = reset ? 6 : 2;
         const int in = c.cur, out = 1 - c.cur;
         check(cudaMemsetAsync(c.status.p, 0, sizeof(DeviceStatus), c.stream), "memset");
-        check(cudaMemsetAsync(c.ra_max.p, 0, sizeof(unsigned long long), c.stream), "memset");
         Ra15Args a{};
         a.f = force_cfg();
         a.np = c.np;
@@ -654,17 +693,15 @@ void ra15_step_once(double time, double* h, double* hdid, double tol, int64_t* r
         a.pconst = c.pconst[c.kc].p;
         a.pb = c.ra_pb.p;
         a.table = c.ftab.p;
-        a.maxb7 = c.ra_max.p;
+        a.maxb7 = &c.status.p->max_b7;
         a.status = c.status.p;
         launch_ra15_sequence(a, c.stream);
         c.dropin_launches += 1 + (c.np > 0 ? 1 : 0);
         check(cudaGetLastError(), "launch");
-        unsigned long long bits = 0;
-        check(cudaMemcpyAsync(&bits, c.ra_max.p, sizeof(bits), cudaMemcpyDeviceToHost, c.stream), "status");
         read_status();
         c.nforces += 1 + 7 * niter;
         double err;
-        std::memcpy(&err, &bits, sizeof(err));
+        std::memcpy(&err, &c.status_host->max_b7, sizeof(err));
         if (c.status_host->fault || !std::isfinite(err)) err = INFINITY;
         reduce_step_maxima(&err, 1);
         if (!std::isfinite(err)) throw std::runtime_error("Nonfinite RADAU force or predictor");
@@ -694,7 +731,6 @@ void ra15_step_once(double time, double* h, double* hdid, double tol, int64_t* r
         launch_ra15_commit(k, c.stream);
         c.dropin_launches += 1;
         check(cudaGetLastError(), "launch");
-        check(cudaStreamSynchronize(c.stream), "step");
         *hdid = t;
         *h = next;
         c.reset = false;
@@ -839,11 +875,14 @@ void bs_step_once(double time, double* h, double* hdid, double tol, int64_t* rej
     for (;;) {
         if (time + *h == time) throw std::runtime_error("BS cannot advance time at the requested tolerance");
         const BsArgs a = launch_bs_attempt(*h);
-        unsigned long long errs[13];
-        DeviceStatus lv[13];
+        const unsigned long long* errs = c.bs_host->errs;
+        const DeviceStatus* lv = c.bs_host->lv;
         auto read_levels = [&] {
-            check(cudaMemcpyAsync(errs, c.bs_errs.p, sizeof(errs), cudaMemcpyDeviceToHost, c.stream), "status");
-            check(cudaMemcpyAsync(lv, c.bs_lvst.p, sizeof(lv), cudaMemcpyDeviceToHost, c.stream), "status");
+            check(cudaMemcpyAsync(c.bs_host->errs, c.bs_errs.p, sizeof(c.bs_host->errs), cudaMemcpyDeviceToHost,
+                                  c.stream),
+                  "status");
+            check(cudaMemcpyAsync(c.bs_host->lv, c.bs_lvst.p, sizeof(c.bs_host->lv), cudaMemcpyDeviceToHost, c.stream),
+                  "status");
             check(cudaStreamSynchronize(c.stream), "step");
         };
         read_levels();
@@ -867,7 +906,6 @@ void bs_step_once(double time, double* h, double* hdid, double tol, int64_t* rej
             continue;
         }
         launch_bs_commit_of(a, accepted);
-        check(cudaStreamSynchronize(c.stream), "step");
         *hdid = *h;
         bs_next_trial(a.variant, accepted, h);
         c.nforces += forces;
@@ -933,21 +971,92 @@ void launch_pair_screen(double h, int step) {
     check(cudaGetLastError(), "screen");
 }
 
-// The pair screen of the last step, its records from slot 0 (grown and redone
-// after an overflow).
-void screen_pairs(double h) {
+// mce_cent between the two state buffers; records are appended at the status
+// counter. dh: with heliocentric velocities (hy_off), for HYBRID.
+void launch_central(double h, double rcen, bool dh) {
     Context& c = ctx();
+    const int total = c.nsplit - 1 + c.np, prev = 1 - c.cur;
+    if (!c.stepped || total <= 0) return;
+    CentralArgs a{};
+    a.nbig = c.nsplit;
+    a.np = c.np;
+    a.npcap = c.npcap;
+    a.mu = c.m_host[0];
+    a.h = h;
+    a.rcen = rcen;
+    a.big0 = c.bigstate[prev].p;
+    a.big1 = c.bigstate[c.cur].p;
+    a.part0 = c.pstate[prev].p;
+    a.part1 = c.pstate[c.cur].p;
+    a.pm = c.pm();
+    a.mbig = c.mbig.p;
+    a.voff0 = dh ? c.hy_off.p : nullptr;
+    a.voff1 = dh ? c.hy_off.p + 3 : nullptr;
+    a.perm = c.permp();
+    a.events = c.events.p;
+    a.event_step = c.event_step.p;
+    a.cap = (int)c.events.n;
+    a.status = c.status.p;
+    central_kernel<<<blocks(total), 256, 0, c.stream>>>(a);
+    c.dropin_launches += 1;
+    check(cudaGetLastError(), "central");
+}
+
+// The status and the first records into pinned memory, queued.
+int queue_records(DeviceStatus* status, MercuryEvent* head) {
+    Context& c = ctx();
+    const int n = c.stepped ? std::min(Context::EVENT_HEAD, (int)c.events.n) : 0;
+    check(cudaMemcpyAsync(status, c.status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, c.stream), "status");
+    if (n > 0)
+        check(cudaMemcpyAsync(head, c.events.p, sizeof(MercuryEvent) * n, cudaMemcpyDeviceToHost, c.stream), "events");
+    return n;
+}
+
+// Both screens of an adaptive integrator's last step, with their records
+// queued for the host: one round trip, and none between them.
+int queue_adaptive_screens(double h, double rcen, DeviceStatus* status, MercuryEvent* head) {
+    Context& c = ctx();
+    check(cudaMemsetAsync(c.status.p, 0, sizeof(DeviceStatus), c.stream), "memset");
+    launch_pair_screen(h, 0);
+    launch_central(h, rcen, false);
+    return queue_records(status, head);
+}
+
+// The host screens every adaptive step (mal_hvar): once an events call has
+// named the central radius, a step queues its screens itself, behind its
+// commit, and the events call finds the records on the host. A step of RADAU
+// with its screens (100,000 particles) made six waits for the device and left
+// it idle for 120 of 302 us; with two waits it takes 247.
+void screen_ahead(double h) {
+    Context& c = ctx();
+    if (c.encounter || c.dropin_rcen <= 0.0) return;
+    queue_adaptive_screens(h, c.dropin_rcen, c.spec_status_host, c.spec_head);
+    c.screen_live = true;
+    c.screen_h = h;
+    c.screen_rcen = c.dropin_rcen;
+}
+
+// The records of an adaptive step's screens: those queued with the step when
+// they were made for this call, else made now (grown and redone after an
+// overflow). Returns the number of records in *head.
+int adaptive_records(double h, double rcen, const MercuryEvent** head) {
+    Context& c = ctx();
+    const bool ahead = c.screen_live && h == c.screen_h && rcen == c.screen_rcen;
+    c.screen_live = false;
+    if (ahead) {
+        check(cudaStreamSynchronize(c.stream), "step");
+        *c.status_host = *c.spec_status_host;
+        *head = c.spec_head;
+        if (!c.status_host->overflow) return std::min(Context::EVENT_HEAD, (int)c.events.n);
+        grow_after_overflow();
+    }
     for (int attempt = 0;; ++attempt) {
-        check(cudaMemsetAsync(c.status.p, 0, sizeof(DeviceStatus), c.stream), "memset");
-        launch_pair_screen(h, 0);
-        read_status();
-        if (c.status_host->overflow) {
-            if (attempt > 8) throw std::runtime_error("event buffer growth failed");
-            grow_after_overflow();
-            continue;
-        }
-        c.pair_events = c.status_host->events;
-        return;
+        const int n = queue_adaptive_screens(h, rcen, c.status_host, c.ev_head);
+        check(cudaStreamSynchronize(c.stream), "step");
+        *head = c.ev_head;
+        if (!c.status_host->overflow) return n;
+        if (attempt > 8) throw std::runtime_error("event buffer growth failed");
+        grow_after_overflow();
     }
 }
 
@@ -1867,7 +1976,6 @@ void upload_layout_for(int n, int nbig, int nmass, int pn, int ngflag, const dou
         c.ra_bpx.reserve((size_t)6 * ns);
         c.ra_pb.reserve((size_t)21 * c.npcap);
         c.ra_pe.reserve((size_t)21 * c.npcap);
-        c.ra_max.reserve(1);
     }
     // zero padding and cached accelerations
     check(cudaMemsetAsync(c.pstate[0].p, 0, sizeof(double) * 9 * c.npcap, s), "memset");
@@ -2008,7 +2116,9 @@ int mercury_cuda_step(double time, double* h, double* hdid, double tol, int64_t*
     try {
         inject("step");
         require_system();
-        DropinTimer timer;
+        const bool adaptive = c.algorithm >= 2 && c.algorithm <= 4;
+        DropinTimer timer(adaptive && !c.encounter);
+        c.screen_live = false;
         *rejected = 0;
         const int64_t before = c.nforces;
         if (is_mvs(c.algorithm)) {
@@ -2023,6 +2133,7 @@ int mercury_cuda_step(double time, double* h, double* hdid, double tol, int64_t*
         } else {
             throw std::runtime_error("algorithm not available in this build");
         }
+        if (adaptive) screen_ahead(*hdid);
         *forces = c.nforces - before;
         return 0;
     } catch (const std::exception& e) {
@@ -2051,9 +2162,9 @@ int mercury_cuda_events(double time, double h, double rcen, const MercuryEvent**
     try {
         inject("events");
         require_system();
-        DropinTimer timer;
+        DropinTimer timer(c.algorithm >= 2 && c.algorithm <= 4 && !c.encounter);
         const int prev = 1 - c.cur;
-        if (!is_mvs(c.algorithm) && c.algorithm != 10 && c.stepped) screen_pairs(h);
+        const bool adaptive = !is_mvs(c.algorithm) && c.algorithm != 10 && c.stepped;
         const bool dh = c.algorithm == 10 && c.stepped;
         // an MVS step that screened for central impacts itself (mvs_step_once)
         bool central_done = false;
@@ -2081,6 +2192,8 @@ int mercury_cuda_events(double time, double h, double rcen, const MercuryEvent**
             c.dropin_launches += 2;
         }
         int head = 0;   // records read back with the status
+        const MercuryEvent* first = c.ev_head;
+        if (adaptive) head = adaptive_records(h, rcen, &first);
         // a step taken from the step ahead brought its status and first
         // records to the host already
         const bool fast = central_done && c.head_ready && !dh;
@@ -2089,46 +2202,15 @@ int mercury_cuda_events(double time, double h, double rcen, const MercuryEvent**
             c.status_host->events = c.pair_events;
             head = c.head_count;
         }
-        for (int attempt = 0; !fast; ++attempt) {
+        for (int attempt = 0; !fast && !adaptive; ++attempt) {
             // restart the counter after the step's pair events (from pinned
             // memory: the copy does not block), then screen for central impacts
             *c.status_host = DeviceStatus{0, c.pair_events, 0, 0};
             check(cudaMemcpyAsync(c.status.p, c.status_host, sizeof(DeviceStatus), cudaMemcpyHostToDevice, c.stream),
                   "status");
-            const int total = c.nsplit - 1 + c.np;
-            if (c.stepped && total > 0 && !central_done) {
-                CentralArgs a{};
-                a.nbig = c.nsplit;
-                a.np = c.np;
-                a.npcap = c.npcap;
-                a.mu = c.m_host[0];
-                a.h = h;
-                a.rcen = rcen;
-                a.big0 = c.bigstate[prev].p;
-                a.big1 = c.bigstate[c.cur].p;
-                a.part0 = c.pstate[prev].p;
-                a.part1 = c.pstate[c.cur].p;
-                a.pm = c.pm();
-                a.mbig = c.mbig.p;
-                a.voff0 = dh ? c.hy_off.p : nullptr;
-                a.voff1 = dh ? c.hy_off.p + 3 : nullptr;
-                a.perm = c.permp();
-                a.events = c.events.p;
-                a.event_step = c.event_step.p;
-                a.cap = (int)c.events.n;
-                a.status = c.status.p;
-                central_kernel<<<blocks(total), 256, 0, c.stream>>>(a);
-                c.dropin_launches += 1;
-                check(cudaGetLastError(), "central");
-            }
+            if (!central_done) launch_central(h, rcen, dh);
             // the status and the first records in one round trip
-            head = c.stepped ? std::min(Context::EVENT_HEAD, (int)c.events.n) : 0;
-            check(cudaMemcpyAsync(c.status_host, c.status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, c.stream),
-                  "status");
-            if (head > 0)
-                check(cudaMemcpyAsync(c.ev_head, c.events.p, sizeof(MercuryEvent) * head, cudaMemcpyDeviceToHost,
-                                      c.stream),
-                      "events");
+            head = queue_records(c.status_host, c.ev_head);
             check(cudaStreamSynchronize(c.stream), "step");
             if (!c.status_host->overflow) break;
             if (attempt > 8) throw std::runtime_error("event buffer growth failed");
@@ -2151,7 +2233,7 @@ int mercury_cuda_events(double time, double h, double rcen, const MercuryEvent**
         size_records(c.host_events, nev);
         if (nev) {
             const int got = std::min(nev, head);
-            std::memcpy(c.host_events.data(), c.ev_head, sizeof(MercuryEvent) * got);
+            std::memcpy(c.host_events.data(), first, sizeof(MercuryEvent) * got);
             if (nev > got)
                 check(cudaMemcpy(c.host_events.data() + got, c.events.p + got, sizeof(MercuryEvent) * (nev - got),
                                  cudaMemcpyDeviceToHost),
@@ -2976,6 +3058,7 @@ int mercury_b200_advance_launches(int* steps, double* kernel_ms, int cap) {
 }
 
 int mercury_b200_dropin_time(double* ms, int64_t* launches, int reset) {
+    settle_timers(0);
     if (ms) *ms = g_dropin_ms;
     if (launches) *launches = g_contexts[0].dropin_launches + g_contexts[1].dropin_launches;
     if (reset) {

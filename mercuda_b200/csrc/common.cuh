@@ -44,7 +44,8 @@ struct DeviceStatus {
     int overflow;      // bit 0: an event slot was beyond capacity; bit 1: a candidate slot
     int cands;         // encounter candidates claimed in the current launch
     int next_tile;     // dynamic work counter of the current particle launch
-    int pad[3];
+    int pad;
+    unsigned long long max_b7;   // RADAU: bits of the sequence's max |b7|
 };
 
 // A Small body whose padded x-y box overlapped a Big body's box during one

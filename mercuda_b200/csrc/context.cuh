@@ -84,10 +84,9 @@ struct Context {
     DBuf<double> tab, detail;
     // RA15: B, E, G and predictor scratch of the massive set ([21][nsplit],
     // [6][nsplit]), B and E of the particle slots ([21][npcap]), the per-node
-    // force table, max |b7| and the force entry's output ([3][nsplit] then
+    // force table and the force entry's output ([3][nsplit] then
     // [3][npcap]); screen boxes of the adaptive integrators ([nbig-1][4])
     DBuf<double> ra_bb, ra_be, ra_bg, ra_bpx, ra_pb, ra_pe, ftab, force_out, boxes;
-    DBuf<unsigned long long> ra_max;
     // output corrector scratch: Big [9][nbig], particles [6][npcap]
     DBuf<double> corr_big, corr_part;
     DBuf<double> energy_scr;         // mxx_en: per-body pair sums, then e and l2
@@ -197,6 +196,16 @@ struct Context {
     cudaEvent_t ah_done = nullptr, spec_merged = nullptr;
     bool ah_live = false;
     double ah_h = 0.0, ah_rcen = 0.0;
+    // an adaptive step's screens for (h, central radius), made with the step:
+    // their status and first records go to spec_status_host / spec_head
+    bool screen_live = false;
+    double screen_h = 0.0, screen_rcen = 0.0;
+    // each BS level's error maximum and force faults, read back at once
+    struct BsLevels {
+        unsigned long long errs[13];
+        DeviceStatus lv[13];
+    };
+    BsLevels* bs_host = nullptr;
     // the last step's status and first records are in status_host / ev_head
     // already (head_count records)
     bool head_ready = false;
@@ -244,6 +253,7 @@ struct Context {
             check(cudaEventCreate(&d1), "event");
             check(cudaMallocHost(reinterpret_cast<void**>(&status_host), sizeof(DeviceStatus)), "pinned");
             check(cudaMallocHost(reinterpret_cast<void**>(&enc_host), sizeof(EncCtl)), "pinned");
+            check(cudaMallocHost(reinterpret_cast<void**>(&bs_host), sizeof(BsLevels)), "pinned");
             check(cudaMallocHost(reinterpret_cast<void**>(&ev_head), sizeof(MercuryEvent) * EVENT_HEAD), "pinned");
             check(cudaMallocHost(reinterpret_cast<void**>(&spec_head), sizeof(MercuryEvent) * EVENT_HEAD), "pinned");
             check(cudaMallocHost(reinterpret_cast<void**>(&spec_status_host), sizeof(DeviceStatus)), "pinned");
@@ -262,7 +272,6 @@ struct Context {
         pinned_n = 0;
         DBuf<int>* ibufs[] = {&perm[0], &perm[1], &inv, &order_bucket, &order_hist, &snap_perm, &ej_ids, &run_tiles};
         for (auto* b : ibufs) b->release();
-        ra_max.release();
         bs_errs.release();
         bs_lvst.release();
         enc_ctl.release();
@@ -283,6 +292,7 @@ struct Context {
         ah_status.release();
         ah_live = false;
         spec_live = false;
+        screen_live = false;
         head_ready = false;
         dropin_rcen = 0.0;
         step_central = false;
