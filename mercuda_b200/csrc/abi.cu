@@ -3203,10 +3203,10 @@ void add_dropin_span(cudaEvent_t a, cudaEvent_t b) {
 // alternate between two control blocks and two sets of level maxima
 // (attempt parity p reads set p and prepares set 1 - p), so that no launch
 // reads what it writes. After the subsystem reached h every launch returns at
-// once. The host enqueues attempts in blocks, as replays of a CUDA graph of
-// GRAPH_ATTEMPTS attempts, and reads the control block back once per block;
-// the block size follows the attempts still needed, estimated from the
-// progress. Records stay on the device, tagged with their substep, until the
+// once. The host queues attempts a few ahead of the count that the decision
+// kernel leaves in page-locked memory, and reads the control block back at the
+// end; the launches overlap (chain_begin in bs.cu).
+// Records stay on the device, tagged with their substep, until the
 // subsystem reaches h. The states do not depend on the records, so after an
 // event-buffer or substep-table overflow the buffers grow and the run is
 // redone from its starting state.
@@ -3214,7 +3214,6 @@ void encounter_run_device(double time, double h, double tol, double* hrec, int64
                           std::vector<MercuryEvent>& keep) {
     Context& c = ctx();
     if (c.algorithm != 3) throw std::runtime_error("the encounter subsystem steps by algorithm 3 (mdt_bs2)");
-    constexpr int GRAPH_ATTEMPTS = 8;   // even: a replay leaves the parity where it found it
     mercury_cuda_reset(1);
     const int in = c.cur;
     const double hrec0 = *hrec;
@@ -3230,14 +3229,6 @@ void encounter_run_device(double time, double h, double tol, double* hrec, int64
     c.enc_bpre.reserve((size_t)6 * c.nsplit);
     c.bs_errs.reserve(26);
     c.bs_lvst.reserve(26);
-    struct Graph {
-        cudaGraph_t g = nullptr;
-        cudaGraphExec_t e = nullptr;
-        ~Graph() {
-            if (e) cudaGraphExecDestroy(e);
-            if (g) cudaGraphDestroy(g);
-        }
-    };
     for (int redo = 0;; ++redo) {
         // the first substep's trial step: hrec, clipped to the subsystem's end
         EncCtl k{};
@@ -3256,13 +3247,16 @@ void encounter_run_device(double time, double h, double tol, double* hrec, int64
         BsArgs base = bs_attempt_args(0.0);
         base.bx_pre = c.enc_bpre.p;
         base.fuse_extrap = 1;
-        auto attempt = [&](int p) {
+        auto attempt = [&](int number) {
+            const int p = number & 1;   // two control blocks alternate
             BsArgs a = base;
             a.ctl = c.enc_ctl.p + p;
             a.errs = c.bs_errs.p + 13 * p;
             a.lvst = c.bs_lvst.p + 13 * p;
             launch_bs_sequence(a, c.stream);
             EncPostArgs e{};
+            e.progress = c.enc_progress;
+            e.attempt = number;
             e.ctl_in = c.enc_ctl.p + p;
             e.ctl_out = c.enc_ctl.p + (1 - p);
             e.errs = a.errs;
@@ -3295,35 +3289,35 @@ void encounter_run_device(double time, double h, double tol, double* hrec, int64
         check(cudaMemsetAsync(c.status.p, 0, sizeof(DeviceStatus), c.stream), "memset");
         check(cudaMemsetAsync(c.bs_errs.p, 0, sizeof(unsigned long long) * 26, c.stream), "memset");
         check(cudaMemsetAsync(c.bs_lvst.p, 0, sizeof(DeviceStatus) * 26, c.stream), "memset");
-        // attempt 0 eagerly (kernel attributes set), then the graph of attempts
-        // 1.. GRAPH_ATTEMPTS (parities 1, 0, 1, ...); after every block the
-        // newest control block is copy 1
+        // Attempts are queued AHEAD of the last one the device has decided, by
+        // the count its decision kernel leaves in page-locked memory: enough to
+        // keep it busy (three launches take the host ~8 us, an attempt ~25), and
+        // little to run out when it stops. A graph of eight attempts, replayed
+        // with a readback between, cost its capture in every HYBRID step and 9
+        // us more an attempt.
+        constexpr int AHEAD = 3;
+        volatile int* progress = &c.enc_progress->x;
+        progress[0] = progress[1] = 0;
         check(cudaEventRecord(c.d0, c.stream), "event");
-        attempt(0);
-        Graph graph;
-        check(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed), "graph");
-        for (int q = 0; q < GRAPH_ATTEMPTS; ++q) attempt((1 + q) % 2);
-        check(cudaStreamEndCapture(c.stream, &graph.g), "graph");
-        check(cudaGraphInstantiate(&graph.e, graph.g, 0), "graph");
-        c.dropin_launches += 3;
-        int blocks = 2;   // graph replays in the first block
-        for (;;) {
-            for (int b = 0; b < blocks; ++b) check(cudaGraphLaunch(graph.e, c.stream), "graph");
-            c.dropin_launches += (int64_t)blocks * GRAPH_ATTEMPTS * 3;
-            check(cudaMemcpyAsync(c.enc_host, c.enc_ctl.p + 1, sizeof(EncCtl), cudaMemcpyDeviceToHost, c.stream),
-                  "status");
-            check(cudaEventRecord(c.d1, c.stream), "event");
-            check(cudaEventSynchronize(c.d1), "step");
-            add_dropin_span(c.d0, c.d1);
-            const EncCtl& now = *c.enc_host;
-            if (now.stop) break;
-            // the attempts still needed at the rate so far, and a little more
-            const double done = std::fabs(now.tlocal) / std::fabs(h);
-            const double rate = now.attempts / std::max(done, 1e-3);
-            const double need = rate * (1.0 - done) * 1.1 + 1.0;
-            blocks = (int)std::min(64.0, std::max(1.0, std::ceil(need / GRAPH_ATTEMPTS)));
-            check(cudaEventRecord(c.d0, c.stream), "event");
+        int queued = 0;
+        for (int spin = 0; !progress[1];) {
+            if (queued - progress[0] < AHEAD) {
+                attempt(queued++);
+                c.dropin_launches += 3;
+                spin = 0;
+            } else if (++spin % 4096 == 0) {
+                // not for ever: a failed launch or an idle stream ends the wait
+                const cudaError_t q = cudaStreamQuery(c.stream);
+                if (q != cudaSuccess && q != cudaErrorNotReady) check(q, "encounter attempt");
+                if (q == cudaSuccess && progress[0] < queued && !progress[1])
+                    throw std::runtime_error("encounter attempts ended without a decision");
+            }
         }
+        check(cudaMemcpyAsync(c.enc_host, c.enc_ctl.p + (queued & 1), sizeof(EncCtl), cudaMemcpyDeviceToHost, c.stream),
+              "status");
+        check(cudaEventRecord(c.d1, c.stream), "event");
+        check(cudaEventSynchronize(c.d1), "step");
+        add_dropin_span(c.d0, c.d1);
         const EncCtl done = *c.enc_host;
         if (done.error == ENC_ERR_FORCE) throw std::runtime_error("BS force failed");
         if (done.error == ENC_ERR_NONFINITE) throw std::runtime_error("Nonfinite BS2 force or extrapolation");

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include "allforce.cuh"
 #include "bs.cuh"
+#include "hybrid_device.cuh"
 #include "mvs.cuh"
 
 namespace mb200 {
@@ -42,6 +43,31 @@ template <int VARIANT> __device__ __forceinline__ void neville_coefficients(doub
     }
 }
 
+// The kernels of the encounter subsystem's attempts follow one another in a
+// chain (massive levels, members, decision): each is launched while the one
+// ahead still runs and begins here, which lets the next one start its launch,
+// waits until everything ahead has ended and its writes are visible, and
+// before which it may only read what no attempt writes. Without the launch
+// attribute both instructions do nothing.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... Params, class Args>
+void launch_chained(void (*kern)(Params...), int blocks, int threads, size_t smem, cudaStream_t s, const Args& args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, args);
+}
+
 __device__ __forceinline__ void level_error(double err, bool finite, unsigned long long* dst) {
     atomicMax(dst, finite ? (unsigned long long)__double_as_longlong(err) : ERR_NONFINITE);
 }
@@ -61,13 +87,13 @@ __device__ __forceinline__ bool body_error(const double* q, double xscal, double
 __device__ __forceinline__ bool hkce_pair(double s2, double rc, double& tmp2) {
     const double rc2 = rc * rc;
     if (!(s2 < rc2)) return false;
-    const double s_1 = 1.0 / sqrt(s2);
+    double s0, s_1;
+    sqrt_recip_any(s2, s0, s_1);
     const double s_3 = s_1 * s_1 * s_1;
     if (s2 <= 0.01 * rc2) {
         tmp2 = s_3;
     } else {
-        const double s = 1.0 / s_1;
-        const double q = (s - 0.1 * rc) / (0.9 * rc);
+        const double q = changeover_q(s0, s_1, rc);
         const double q2 = q * q, q3 = q * q2, q4 = q2 * q2, q5 = q2 * q3;
         tmp2 = (1.0 - 10.0 * q3 + 15.0 * q4 - 6.0 * q5) * s_3;
     }
@@ -77,7 +103,8 @@ __device__ __forceinline__ bool hkce_pair(double s2, double rc, double& tmp2) {
 // mfo_hkce's central term (mercury6_2.for:4898-4905).
 __device__ __forceinline__ double3 hkce_central(double3 a, const double3 x, double m0) {
     const double s2 = x.x * x.x + x.y * x.y + x.z * x.z;
-    const double s_1 = 1.0 / sqrt(s2);
+    double s0, s_1;
+    sqrt_recip_any(s2, s0, s_1);
     const double tmp2 = m0 * s_1 * s_1 * s_1;
     a.x = a.x - tmp2 * x.x;
     a.y = a.y - tmp2 * x.y;
@@ -128,6 +155,30 @@ __device__ __forceinline__ double3 hkce_member_force(const BsArgs& A, int g, int
                                                      const double* crc, const double3 x, double rcrit_p,
                                                      const double* B) {
     double3 a = make_double3(0.0, 0.0, 0.0);
+    // The usual member has one pair: its square root, the changeover's
+    // divisions and the central term's square root are three chains of dependent
+    // operations, made side by side before anything is decided.
+    const double sc = x.x * x.x + x.y * x.y + x.z * x.z;
+    double c0, c_1;
+    sqrt_recip(sc, c0, c_1);
+    int q0 = 0;
+    if (npair > 0) {
+        const double* row = B + 4 * (ci[0] - 1);
+        const double rc = crc[0], rc2 = rc * rc, d = 0.9 * rc;
+        const double dx = x.x - row[0], dy = x.y - row[1], dz = x.z - row[2];
+        const double s2 = dx * dx + dy * dy + dz * dz;
+        double s0, s_1;
+        sqrt_recip(s2, s0, s_1);
+        const double s_3 = s_1 * s_1 * s_1;
+        const double q = quotient(recip_fix(s_1, s0) - 0.1 * rc, d, recip_near(d));
+        const double q2 = q * q, q3 = q * q2, q4 = q2 * q2, q5 = q2 * q3;
+        const double K = (1.0 - 10.0 * q3 + 15.0 * q4 - 6.0 * q5) * s_3;
+        const double faci = (s2 <= 0.01 * rc2 ? s_3 : K) * row[3];
+        if (mid_range(s2) && mid_range(d)) {
+            if (s2 < rc2) a = make_double3(a.x - faci * dx, a.y - faci * dy, a.z - faci * dz);
+            q0 = 1;
+        }
+    }
     auto term = [&](int i, double rc) {
         const double* row = B + 4 * (i - 1);
         const double dx = x.x - row[0], dy = x.y - row[1], dz = x.z - row[2];
@@ -139,13 +190,15 @@ __device__ __forceinline__ double3 hkce_member_force(const BsArgs& A, int g, int
         a.z = a.z - faci * dz;
     };
     const int nc = npair < PAIR_CACHE ? npair : PAIR_CACHE;
-    for (int q = 0; q < nc; ++q) term(ci[32 * q], crc[32 * q]);
+    for (int q = q0; q < nc; ++q) term(ci[32 * q], crc[32 * q]);
     if (npair > PAIR_CACHE)
         for (int e = A.adj_off[g] + PAIR_CACHE; e < A.adj_off[g + 1]; ++e) {
             const int i = A.adj[e].x;
             term(i, fmax(A.rcrit[i], rcrit_p));
         }
-    return hkce_central(a, x, A.f.m0);
+    if (!mid_range(sc)) return hkce_central(a, x, A.f.m0);
+    const double tmp2 = A.f.m0 * c_1 * c_1 * c_1;
+    return make_double3(a.x - tmp2 * x.x, a.y - tmp2 * x.y, a.z - tmp2 * x.z);
 }
 
 // hkce_particle_force and its derivative along dx (J dx with J = da/dx; the
@@ -258,6 +311,7 @@ template <int VARIANT, bool HKCE> __global__ void __launch_bounds__(256, 1) bs_m
     extern __shared__ double sm[];
     double h0 = A.h0;
     if (A.ctl) {
+        chain_begin();
         if (A.ctl->stop) return;
         h0 = A.ctl->h0;
     }
@@ -459,8 +513,35 @@ __global__ void __launch_bounds__((HI - LO + 1) * 16, HKCE ? 3 : 384 / ((HI - LO
     __shared__ double pair_rc[PAIR_CACHE * 32];
     extern __shared__ double staged[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + lane;
+    const bool ok = p < A.np && A.perm[p] < A.active_np;
+    const int nb = A.f.nbig - 1, stride = force_row(nb), S = A.npcap;
+    double3 x0 = make_double3(0.0, 0.0, 0.0), v0 = x0;
+    double mj = 0.0, g5[5] = {0, 0, 0, 0, 0};
+    // the encounter subsystem (BS2 only): mfo_hkce from the member's pairs,
+    // which do not change while it runs and are read before the kernels ahead
+    // of this one have ended
+    constexpr bool hkce = VARIANT == 2 && HKCE;
+    const bool stage = hkce && A.stage_bodies;
+    const int bw = 4 * nb;   // body block of a table row
+    int g = 0;
+    double rcrit_p = 0.0;
+    if (hkce && ok) {
+        g = A.f.nsplit + A.perm[p];
+        rcrit_p = A.pconst[(size_t)PC_RCRIT * S + p];
+    }
+    if (hkce && w == 0) {
+        const int e0 = ok ? A.adj_off[g] : 0, e1 = ok ? A.adj_off[g + 1] : 0;
+        pair_n[lane] = e1 - e0;
+        for (int q = 0; q < PAIR_CACHE && e0 + q < e1; ++q) {
+            const int i = A.adj[e0 + q].x;
+            pair_i[32 * q + lane] = i;
+            pair_rc[32 * q + lane] = fmax(A.rcrit[i], rcrit_p);
+        }
+    }
     double h0 = A.h0;
     if (A.ctl) {
+        chain_begin();
         if (A.ctl->stop) return;
         h0 = A.ctl->h0;
     }
@@ -471,31 +552,7 @@ __global__ void __launch_bounds__((HI - LO + 1) * 16, HKCE ? 3 : 384 / ((HI - LO
         massive_extrap_block<VARIANT>(A, co);
         return;
     }
-    const int p = blockIdx.x * 32 + lane;
-    const bool ok = p < A.np && A.perm[p] < A.active_np;
-    const int nb = A.f.nbig - 1, stride = force_row(nb), S = A.npcap;
-    double3 x0 = make_double3(0.0, 0.0, 0.0), v0 = x0;
-    double mj = 0.0, g5[5] = {0, 0, 0, 0, 0};
-    // the encounter subsystem (BS2 only): mfo_hkce from the member's pairs
-    constexpr bool hkce = VARIANT == 2 && HKCE;
-    const bool stage = hkce && A.stage_bodies;
-    const int bw = 4 * nb;   // body block of a table row
-    int g = 0;
-    double rcrit_p = 0.0;
     if (hkce) {
-        if (ok) {
-            g = A.f.nsplit + A.perm[p];
-            rcrit_p = A.pconst[(size_t)PC_RCRIT * S + p];
-        }
-        if (w == 0) {
-            const int e0 = ok ? A.adj_off[g] : 0, e1 = ok ? A.adj_off[g + 1] : 0;
-            pair_n[lane] = e1 - e0;
-            for (int q = 0; q < PAIR_CACHE && e0 + q < e1; ++q) {
-                const int i = A.adj[e0 + q].x;
-                pair_i[32 * q + lane] = i;
-                pair_rc[32 * q + lane] = fmax(A.rcrit[i], rcrit_p);
-            }
-        }
         if (stage)
             for (int q = threadIdx.x; q < bs_rows(VARIANT) * bw; q += blockDim.x) {
                 const int r = q / bw;
@@ -847,11 +904,14 @@ __device__ __forceinline__ int enc_decide(EncCtl& c, const unsigned long long* e
 // test and classification inline. Records carry the substep index.
 __global__ void __launch_bounds__(128) enc_post_kernel(EncPostArgs A) {
     extern __shared__ double sh[];
+    chain_begin();
     EncCtl c = *A.ctl_in;
     const int acc = enc_decide(c, A.errs, A.lvst);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (acc) c.tstep[c.substeps - 1] = c.time + c.tlocal;
         *A.ctl_out = c;
+        // for the host, which queues attempts a few ahead of this count
+        *A.progress = make_int2(A.attempt + 1, c.stop);
         for (int n = 0; n < 13; ++n) {
             A.errs_next[n] = 0ull;
             A.lvst_next[n] = DeviceStatus{};
@@ -977,7 +1037,8 @@ template <int VARIANT, bool HKCE> void launch_variant(const BsArgs& a, cudaStrea
     // for most of the pairs
     int mthreads = std::min(256, std::max(32, (N + 31) / 32 * 32));
     if (!HKCE && N <= MASSIVE_PAR_MAX) mthreads = N <= 16 ? 128 : 256;
-    bs_massive_level_kernel<VARIANT, HKCE><<<bs_levels(VARIANT), mthreads, msmem, s>>>(a);
+    if (a.ctl) launch_chained(bs_massive_level_kernel<VARIANT, HKCE>, bs_levels(VARIANT), mthreads, msmem, s, a);
+    else bs_massive_level_kernel<VARIANT, HKCE><<<bs_levels(VARIANT), mthreads, msmem, s>>>(a);
     if (!a.fuse_extrap) bs_massive_extrap_kernel<VARIANT><<<1, mthreads, 0, s>>>(a);
     const int pblocks = (a.np > 0 ? (a.np + 31) / 32 : 0) + (a.fuse_extrap ? 1 : 0);
     if (pblocks <= 0) return;
@@ -1000,7 +1061,9 @@ template <int VARIANT, bool HKCE> void launch_variant(const BsArgs& a, cudaStrea
         bs_particle_kernel<2, false, 1, 8><<<pblocks, 8 * 16, 0, s>>>(b);
         return;
     }
-    bs_particle_kernel<VARIANT, HKCE><<<pblocks, bs_levels(VARIANT) * 16, psmem, s>>>(b);
+    const auto kern = bs_particle_kernel<VARIANT, HKCE>;
+    if (a.ctl) launch_chained(kern, pblocks, bs_levels(VARIANT) * 16, psmem, s, b);
+    else kern<<<pblocks, bs_levels(VARIANT) * 16, psmem, s>>>(b);
 }
 
 }  // namespace
@@ -1029,7 +1092,7 @@ void launch_enc_post(const EncPostArgs& a, cudaStream_t s) {
     const size_t smem = sizeof(double) * (size_t)(nb > 0 ? nb : 1) * (4 + TAB_DETAIL);
     if (smem > 48 * 1024) cudaFuncSetAttribute(enc_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int blocks = std::max(1, (a.np + 127) / 128);
-    enc_post_kernel<<<blocks, 128, smem, s>>>(a);
+    launch_chained(enc_post_kernel, blocks, 128, smem, s, a);
 }
 
 void launch_bs_commit(const BsCommitArgs& a, cudaStream_t s) {

@@ -93,6 +93,8 @@ struct BsCommitArgs {
 // block of the next attempt with its level maxima cleared, and after an
 // acceptance the commit in place and the pair screen of the substep.
 struct EncPostArgs {
+    int2* progress;        // page-locked: {attempts decided, stop}
+    int attempt;           // this attempt's number
     const EncCtl* ctl_in;              // the control block this attempt ran with
     EncCtl* ctl_out;                   // the next attempt's
     const unsigned long long* errs;    // [13] this attempt's level maxima

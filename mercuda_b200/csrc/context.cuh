@@ -213,6 +213,7 @@ struct Context {
     // the encounter subsystem's step control, read back once per block of
     // attempts
     EncCtl* enc_host = nullptr;
+    int2* enc_progress = nullptr;   // written by the device, read by the host
     // the encounter subsystem's step control on the device (two copies that
     // alternate between attempts), the end time of each accepted substep, and
     // the massive set's state at the start of the current attempt
@@ -253,6 +254,7 @@ struct Context {
             check(cudaEventCreate(&d1), "event");
             check(cudaMallocHost(reinterpret_cast<void**>(&status_host), sizeof(DeviceStatus)), "pinned");
             check(cudaMallocHost(reinterpret_cast<void**>(&enc_host), sizeof(EncCtl)), "pinned");
+            check(cudaMallocHost(reinterpret_cast<void**>(&enc_progress), sizeof(int2)), "pinned");
             check(cudaMallocHost(reinterpret_cast<void**>(&bs_host), sizeof(BsLevels)), "pinned");
             check(cudaMallocHost(reinterpret_cast<void**>(&ev_head), sizeof(MercuryEvent) * EVENT_HEAD), "pinned");
             check(cudaMallocHost(reinterpret_cast<void**>(&spec_head), sizeof(MercuryEvent) * EVENT_HEAD), "pinned");

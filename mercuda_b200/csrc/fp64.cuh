@@ -81,4 +81,19 @@ __device__ __forceinline__ void sqrt_recip(double x, double& s, double& r) {
     r = recip_fix(s, y);
 }
 
+// The same for any operands: what is out of range takes the plain statements,
+// by a call (their code then stays out of the way of the code around).
+static __device__ __noinline__ double sqrt_plain(double x) { return sqrt(x); }
+static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
+__device__ __forceinline__ void sqrt_recip_any(double x, double& s, double& r) {
+    sqrt_recip(x, s, r);
+    if (!mid_range(x)) {
+        s = sqrt_plain(x);
+        r = div_plain(1.0, s);
+    }
+}
+__device__ __forceinline__ bool mid_magnitude(double x) {   // mid_range of |x|
+    return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((1023u - 200u) << 20) < (400u << 20);
+}
+
 }  // namespace mb200

@@ -315,9 +315,6 @@ __device__ __forceinline__ bool drift_near(double mu, double rmu, double3& p, do
 // first, still ends a launch of 16 to 31 steps last: what counts here is the
 // length of the chain. False where drift_kepmd applies, an operand is out of
 // range or Laguerre's iteration fails: drift_dan then decides.
-__device__ __forceinline__ bool mid_magnitude(double x) {   // mid_range of |x|
-    return ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((1023u - 200u) << 20) < (400u << 20);
-}
 // stumpff with the number of quarterings taken from the exponent (|x| 4^-n is
 // exact either way), for |x| below 2^200.
 __device__ __forceinline__ void stumpff_near(double x, double& c0, double& c1, double& c2, double& c3) {

@@ -118,16 +118,9 @@ template <class F> __device__ __forceinline__ void big_each(int k0, int k1, F f)
         f(k0 + j, q - 3 * j);
     }
 }
-// 1.0 / sqrt(x) and a / b in plain, as calls: the step's code is long, and what
-// does not run should not lie between what does (the instruction cache misses
-// of a lone CTA are not hidden by anything).
-static __device__ __noinline__ double rsqrt_plain(double x) { return 1.0 / sqrt(x); }
-static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
-// 1.0 / sqrt(x): fp64.cuh's where the operand allows, else plain.
 __device__ __forceinline__ double rsqrt_any(double x) {
-    if (!mid_range(x)) return rsqrt_plain(x);
     double s, r;
-    sqrt_recip(x, s, r);
+    sqrt_recip_any(x, s, r);
     return r;
 }
 
@@ -280,8 +273,8 @@ __device__ void big_force_terms(const MvsBigArgs& A, BigSmem& S, const double* V
         sqrt_recip(rj2, s, rj);
         const bool fast = mid_range(r2) && mid_range(rj2);
         if (!fast) {
-            r = rsqrt_plain(r2);
-            rj = rsqrt_plain(rj2);
+            r = div_plain(1.0, sqrt_plain(r2));
+            rj = div_plain(1.0, sqrt_plain(rj2));
         }
         const double r3 = r * r * r, rj3 = rj * rj * rj;
         const double fac0 = m[k] * r3;
