@@ -15,8 +15,8 @@
 //             checkpoint keeping each step's drift input and output, then
 //             walk it backwards: kick, force (gravity from the table, yar) and
 //             the Kepler drift's state-transition matrix, transposed. The
-//             recomputation of segment k-1 (second stream, second record
-//             buffer) overlaps the walk through segment k.
+//             recomputations of the segments before it (streams and record
+//             buffers of their own) overlap the walk through segment k.
 #include <cmath>
 #include <cstdio>
 
@@ -31,6 +31,7 @@
 namespace mb200 {
 namespace {
 
+constexpr int ADJ_CTAS = 6;  // of 128 threads an SM (80 registers): 100,000 particles in one wave
 constexpr int REC = 12;  // per step of a segment: x, v after the kick (drift input), x, v after the drift
 
 struct AdjArgs {
@@ -40,11 +41,13 @@ struct AdjArgs {
     const double* x0;        // (np, 3) rows
     const double* v0;
     const double* yar;       // [np] or null
+    int* perm;               // [nseg][np]: each segment's slot -> particle
+    int* nslow;              // [nseg][2]: slots filled from the front, from the back
     double* xf;              // (np, 3)
     double* vf;
-    double* ckpt;            // [nseg][9][np]
-    double* rec;             // [K][REC][np] records of one segment
-    double* lam;             // [10][np] adjoint state between segments
+    double* ckpt;            // [nseg][9][np], by particle
+    double* rec;             // [K][REC][np] records of one segment, by slot
+    double* lam;             // [10][np] adjoint state between segments, by particle
     const double* gx;        // (np, 3) adjoint of the final positions
     const double* gv;        // (np, 3) or null
     double* dx0;             // (np, 3)
@@ -76,19 +79,22 @@ __device__ __forceinline__ double3 accel(const double3 x, const double3 v, doubl
 template <bool YAR>
 __device__ __forceinline__ void accel_vjp(const double3 x, const double3 v, double yar, const double* T, int nb,
                                           const double3 la, double3& gx, double3& gv, double& gyar) {
-#pragma unroll 1
+    // (not bound to the reference's roundings: 1/|d| to half an ulp, fused
+    // multiply-adds, two bodies at a time)
+#pragma unroll 2
     for (int b = 0; b < nb; ++b) {
         const double* row = T + TAB_HEAD + b * TAB_BODY;
-        const double dx = x.x - row[0], dy = x.y - row[1], dz = x.z - row[2];
-        const double s2 = dx * dx + dy * dy + dz * dz;
-        const double s_1 = 1.0 / sqrt(s2);
-        const double s_3 = s_1 * s_1 * s_1;
-        const double s_5 = s_3 * s_1 * s_1;
-        const double dl = dx * la.x + dy * la.y + dz * la.z;
-        const double m = row[3];
-        gx.x -= m * (s_3 * la.x - 3.0 * s_5 * dl * dx);
-        gx.y -= m * (s_3 * la.y - 3.0 * s_5 * dl * dy);
-        gx.z -= m * (s_3 * la.z - 3.0 * s_5 * dl * dz);
+        const double2 r01 = *reinterpret_cast<const double2*>(row), r23 = *reinterpret_cast<const double2*>(row + 2);
+        const double dx = x.x - r01.x, dy = x.y - r01.y, dz = x.z - r23.x;
+        const double s2 = fma(dx, dx, fma(dy, dy, dz * dz));
+        double s, s_1;
+        sqrt_near(s2, s, s_1);
+        if (!mid_range(s2)) s_1 = div_plain(1.0, sqrt_plain(s2));
+        const double k3 = r23.y * s_1 * s_1 * s_1;
+        const double k5 = 3.0 * k3 * (s_1 * s_1) * fma(dx, la.x, fma(dy, la.y, dz * la.z));
+        gx.x += fma(k5, dx, -k3 * la.x);
+        gx.y += fma(k5, dy, -k3 * la.y);
+        gx.z += fma(k5, dz, -k3 * la.z);
     }
     if (YAR) yar_vjp(x, v, yar, la, gx, gv, gyar);
 }
@@ -98,19 +104,83 @@ __device__ __forceinline__ void st_ckpt(double* c, int np, int p, double3 x, dou
     for (int k = 0; k < 9; ++k) c[(size_t)k * np + p] = q[k];
 }
 
+// Particle slots of a segment: those whose drifts take the universal-variable
+// solve at its start from the front, the others from the back. A warp with
+// one such particle takes several times an ordinary warp's time, and in the
+// caller's order half of the warps had one. Which slot a particle gets changes
+// nothing else (atomics order them within a class as they come).
+__global__ void __launch_bounds__(256) adj_partition_kernel(AdjArgs A, int seg) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const bool ok = p < A.np;
+    bool slow = false;
+    if (ok) {
+        const double* c = A.ckpt + (size_t)seg * 9 * A.np + p;
+        const size_t S = A.np;
+        const double3 x = seg ? make_double3(c[0], c[S], c[2 * S]) : ld_row(A.x0, p);
+        const double3 v = seg ? make_double3(c[3 * S], c[4 * S], c[5 * S]) : ld_row(A.v0, p);
+        const double r0 = sqrt(x.x * x.x + x.y * x.y + x.z * x.z);
+        const double alpha = 2.0 * A.mu / r0 - (v.x * v.x + v.y * v.y + v.z * v.z);
+        const double a = A.mu / alpha, en = sqrt(A.mu / (a * a * a));
+        const double ec = 1.0 - r0 / a, es = (x.x * v.x + x.y * v.y + x.z * v.z) / (en * a * a);
+        const double esq = ec * ec + es * es, dm2 = A.h * en * (A.h * en);
+        // drift_dan's conditions for drift_kepmd (NaN counts as slow)
+        slow = !(alpha > 0.0 && dm2 <= 0.16 && esq <= 0.36 && esq * dm2 < 0.0016);
+    }
+    const unsigned live = __ballot_sync(0xffffffffu, ok), front = __ballot_sync(0xffffffffu, slow);
+    const unsigned back = live & ~front;
+    int* n = A.nslow + 2 * seg;
+    int f0 = 0, b0 = 0;
+    if (lane == 0) {
+        if (front) f0 = atomicAdd(n, __popc(front));
+        if (back) b0 = atomicAdd(n + 1, __popc(back));
+    }
+    f0 = __shfl_sync(0xffffffffu, f0, 0);
+    b0 = __shfl_sync(0xffffffffu, b0, 0);
+    if (!ok) return;
+    const unsigned before = (1u << lane) - 1u;
+    A.perm[(size_t)seg * A.np +
+           (slow ? f0 + __popc(front & before) : A.np - 1 - (b0 + __popc(back & before)))] = p;
+}
+
+// The slot of this thread in the forward and recompute launches, or -1. The
+// slow slots go eight to a warp where the launch has the warps for it (it has
+// half as many again as full warps would need): the segment ends with its
+// slowest warp, and a warp's drift takes as many passes of the solver as its
+// worst lane's. 100,000 particles, a forward segment of 50 steps: 0.68 ms with
+// full warps in the order of the initial states, 0.66 so; the rest is the
+// serial steps of the few particles whose Newton iteration never converges.
+constexpr int SLOW_LANES = 8;
+int adj_grid(int np) { return ((np + 31) / 32 + (np + 63) / 64 + 3) / 4; }
+__device__ __forceinline__ int adj_slot(const AdjArgs& A, int seg) {
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5, nslow = A.nslow[2 * seg];
+    const int few = (nslow + SLOW_LANES - 1) / SLOW_LANES;
+    int slot;
+    if (few + (A.np - nslow + 31) / 32 > warps) {
+        slot = w * 32 + lane;
+    } else if (w < few) {
+        slot = w * SLOW_LANES + lane;
+        if (lane >= SLOW_LANES || slot >= nslow) return -1;
+    } else {
+        slot = nslow + (w - few) * 32 + lane;
+    }
+    return slot < A.np ? slot : -1;
+}
+
 // One K-step segment of the forward run: from the initial state (segment 0)
 // or the segment's checkpoint, to the next checkpoint or the final state.
-template <bool YAR> __global__ void __launch_bounds__(128) adj_forward_kernel(AdjArgs A, int seg) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= A.np) return;
+template <bool YAR> __global__ void __launch_bounds__(128, ADJ_CTAS) adj_forward_kernel(AdjArgs A, int seg) {
+    const int slot = adj_slot(A, seg);
+    if (slot < 0) return;
+    const int row = A.perm[(size_t)seg * A.np + slot], p = row;
     const int stride = tab_stride(A.nb), np = A.np;
     const double hby2 = 0.5 * A.h;
-    const double yar = YAR ? A.yar[p] : 0.0;
+    const double yar = YAR ? A.yar[row] : 0.0;
     const int s0 = seg * A.K, s1 = min(A.nsteps, s0 + A.K);
     double3 x, v, acc;
     if (seg == 0) {
-        x = ld_row(A.x0, p);
-        v = ld_row(A.v0, p);
+        x = ld_row(A.x0, row);
+        v = ld_row(A.v0, row);
         acc = accel<YAR>(x, v, yar, A.tab, A.nb, A.mu, A.status);
         st_ckpt(A.ckpt, np, p, x, v, acc);
     } else {
@@ -133,20 +203,21 @@ template <bool YAR> __global__ void __launch_bounds__(128) adj_forward_kernel(Ad
     if (s1 < A.nsteps) {
         st_ckpt(A.ckpt + (size_t)(seg + 1) * 9 * np, np, p, x, v, acc);
     } else {
-        st_row(A.xf, p, x);
-        st_row(A.vf, p, v);
+        st_row(A.xf, row, x);
+        st_row(A.vf, row, v);
     }
 }
 
 // Reverse sweep, per segment (last first): recompute the segment from its
 // checkpoint keeping each step's drift input and output ...
-template <bool YAR> __global__ void __launch_bounds__(128) adj_recompute_kernel(AdjArgs A, int seg) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= A.np) return;
+template <bool YAR> __global__ void __launch_bounds__(128, ADJ_CTAS) adj_recompute_kernel(AdjArgs A, int seg) {
+    const int slot = adj_slot(A, seg);
+    if (slot < 0) return;
+    const int row = A.perm[(size_t)seg * A.np + slot], p = row;
     const int stride = tab_stride(A.nb), np = A.np;
     const double hby2 = 0.5 * A.h;
-    const double yar = YAR ? A.yar[p] : 0.0;
-    auto R = [&](int sl, int c) -> double& { return A.rec[((size_t)sl * REC + c) * np + p]; };
+    const double yar = YAR ? A.yar[row] : 0.0;
+    auto R = [&](int sl, int c) -> double& { return A.rec[((size_t)sl * REC + c) * np + slot]; };
     const int s0 = seg * A.K, s1 = min(A.nsteps, s0 + A.K);
     const double* c = A.ckpt + (size_t)seg * 9 * np;
     double3 x = make_double3(c[p], c[np + p], c[2 * (size_t)np + p]);
@@ -175,18 +246,19 @@ template <bool YAR> __global__ void __launch_bounds__(128) adj_recompute_kernel(
 // segments; the first segment also differentiates the initial acceleration
 // and writes the gradients.
 template <bool YAR> __global__ void __launch_bounds__(128) adj_vjp_kernel(AdjArgs A, int seg, int last) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= A.np) return;
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= A.np) return;
+    const int row = A.perm[(size_t)seg * A.np + slot], p = row;
     const int stride = tab_stride(A.nb), np = A.np;
     const double hby2 = 0.5 * A.h;
-    const double yar = YAR ? A.yar[p] : 0.0;
-    auto R = [&](int sl, int c) -> double { return A.rec[((size_t)sl * REC + c) * np + p]; };
+    const double yar = YAR ? A.yar[row] : 0.0;
+    auto R = [&](int sl, int c) -> double { return A.rec[((size_t)sl * REC + c) * np + slot]; };
     auto L = [&](int c) -> double& { return A.lam[(size_t)c * np + p]; };
     double3 lx, lv, la;
     double lyar;
     if (last) {
-        lx = ld_row(A.gx, p);
-        lv = A.gv ? ld_row(A.gv, p) : make_double3(0.0, 0.0, 0.0);
+        lx = ld_row(A.gx, row);
+        lv = A.gv ? ld_row(A.gv, row) : make_double3(0.0, 0.0, 0.0);
         la = make_double3(0.0, 0.0, 0.0);
         lyar = 0.0;
     } else {
@@ -225,12 +297,12 @@ template <bool YAR> __global__ void __launch_bounds__(128) adj_vjp_kernel(AdjArg
         return;
     }
     // the acceleration of the initial state (computed before the first kick)
-    const double3 x0 = ld_row(A.x0, p), v0 = ld_row(A.v0, p);
+    const double3 x0 = ld_row(A.x0, row), v0 = ld_row(A.v0, row);
     double3 gx = make_double3(0.0, 0.0, 0.0), gv = make_double3(0.0, 0.0, 0.0);
     accel_vjp<YAR>(x0, v0, yar, A.tab, A.nb, la, gx, gv, lyar);
-    st_row(A.dx0, p, make_double3(lx.x + gx.x, lx.y + gx.y, lx.z + gx.z));
-    st_row(A.dv0, p, make_double3(lv.x + gv.x, lv.y + gv.y, lv.z + gv.z));
-    if (A.dyar) A.dyar[p] = lyar;
+    st_row(A.dx0, row, make_double3(lx.x + gx.x, lx.y + gx.y, lx.z + gx.z));
+    st_row(A.dv0, row, make_double3(lv.x + gv.x, lv.y + gv.y, lv.z + gv.z));
+    if (A.dyar) A.dyar[row] = lyar;
     if (!isfinite(lx.x) || !isfinite(lv.x) || !isfinite(lyar)) raise_fault(A.status, FAULT_NONFINITE);
 }
 
@@ -238,11 +310,20 @@ struct Adjoint {
     int nbig = 0, np = 0, nsteps = 0, K = 0, has_yar = 0;
     double h = 0.0, mu = 0.0;
     const double *x0 = nullptr, *v0 = nullptr, *yar = nullptr;
-    DBuf<double> bigstate[2], mbig, zeros, tab, detail, ckpt, rec[2], lam;
+    // Record buffers: a recomputation ends with its slowest particle's serial
+    // steps, but segments can be recomputed side by side from their
+    // checkpoints: up to three run ahead of the walk (one, where a buffer takes
+    // more than REC_BYTES). 100,000 particles, 20 segments of 50 steps:
+    // backward 17.7 ms with one ahead, 12.2 with three.
+    static constexpr int MAX_REC = 4;
+    static constexpr size_t REC_BYTES = (size_t)1 << 30;
+    int nrec = 2;
+    DBuf<double> bigstate[2], mbig, zeros, tab, detail, ckpt, rec[MAX_REC], lam;
     DBuf<MercuryEvent> events;
     DBuf<int> event_step;
     DBuf<DeviceStatus> status;
-    cudaStream_t stream = nullptr, stream2 = nullptr;
+    DBuf<int> perm, nslow;
+    cudaStream_t stream = nullptr, stream2 = nullptr, ahead[MAX_REC - 1] = {};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     std::vector<cudaEvent_t> done2, done1;   // per segment: second-stream and main-stream work finished
     float fwd_ms = 0.0f, bwd_ms = 0.0f;
@@ -251,6 +332,7 @@ struct Adjoint {
         if (stream) return;
         check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "stream");
         check(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking), "stream");
+        for (cudaStream_t& s : ahead) check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
         check(cudaEventCreate(&e0), "event");
         check(cudaEventCreate(&e1), "event");
     }
@@ -264,11 +346,14 @@ struct Adjoint {
         }
     }
     void release() {
-        DBuf<double>* b[] = {&bigstate[0], &bigstate[1], &mbig, &zeros, &tab, &detail, &ckpt, &rec[0], &rec[1], &lam};
+        DBuf<double>* b[] = {&bigstate[0], &bigstate[1], &mbig, &zeros, &tab, &detail, &ckpt, &lam};
         for (auto* d : b) d->release();
+        for (auto& r : rec) r.release();
         events.release();
         event_step.release();
         status.release();
+        perm.release();
+        nslow.release();
         ready = false;
     }
 };
@@ -291,6 +376,8 @@ AdjArgs adj_args(Adjoint& J) {
     a.x0 = J.x0;
     a.v0 = J.v0;
     a.yar = J.yar;
+    a.perm = J.perm.p;
+    a.nslow = J.nslow.p;
     a.ckpt = J.ckpt.p;
     a.rec = J.rec[0].p;
     a.lam = J.lam.p;
@@ -331,13 +418,16 @@ int mercury_b200_adjoint_forward(int nbig, const double* mbig, const double* xbi
         J.tab.reserve((size_t)(nsteps + 1) * tab_stride(nb));
         J.detail.reserve((size_t)nsteps * std::max(1, nb) * TAB_DETAIL);
         J.ckpt.reserve((size_t)nseg * 9 * np);
-        J.rec[0].reserve((size_t)J.K * REC * np);
-        J.rec[1].reserve(nseg > 1 ? (size_t)J.K * REC * np : 1);
+        const size_t rec_el = (size_t)J.K * REC * np;
+        J.nrec = std::min(nseg, sizeof(double) * rec_el > Adjoint::REC_BYTES ? 2 : Adjoint::MAX_REC);
+        for (int k = 0; k < J.nrec; ++k) J.rec[k].reserve(rec_el);
         J.ensure_events(nseg);
         J.lam.reserve((size_t)10 * np);
         J.events.reserve(4096);
         J.event_step.reserve(4096);
         J.status.reserve(1);
+        J.perm.reserve((size_t)nseg * np);
+        J.nslow.reserve((size_t)2 * nseg);
         // Big bodies: SoA [9][nbig] from the host rows, a(3) zero (reset)
         std::vector<double> b(9 * (size_t)nbig, 0.0);
         for (int k = 0; k < nbig; ++k)
@@ -354,7 +444,8 @@ int mercury_b200_adjoint_forward(int nbig, const double* mbig, const double* xbi
         AdjArgs f = adj_args(J);
         f.xf = x_final;
         f.vf = v_final;
-        const int grid = (np + 127) / 128, stride = tab_stride(nb);
+        const int grid = adj_grid(np), stride = tab_stride(nb);
+        check(cudaMemsetAsync(J.nslow.p, 0, 2 * sizeof(int) * nseg, J.stream), "memset");
         for (int seg = 0; seg < nseg; ++seg) {
             const int s0 = seg * J.K, ks = std::min(J.K, nsteps - s0);
             // the Big bodies' steps of this segment and their force tables
@@ -385,6 +476,7 @@ int mercury_b200_adjoint_forward(int nbig, const double* mbig, const double* xbi
             launch_mvs_big(a, J.stream2);
             check(cudaEventRecord(J.done2[seg], J.stream2), "event");
             check(cudaStreamWaitEvent(J.stream, J.done2[seg], 0), "wait");
+            adj_partition_kernel<<<(np + 255) / 256, 256, 0, J.stream>>>(f, seg);
             if (J.has_yar) adj_forward_kernel<true><<<grid, 128, 0, J.stream>>>(f, seg);
             else adj_forward_kernel<false><<<grid, 128, 0, J.stream>>>(f, seg);
         }
@@ -415,27 +507,28 @@ int mercury_b200_adjoint_backward(const double* gx, const double* gv, double* dx
         a.dv0 = dv0;
         a.dyar = dyar;
         check(cudaEventRecord(J.e0, J.stream), "event");
-        check(cudaStreamWaitEvent(J.stream2, J.e0, 0), "wait");
-        const int grid = (J.np + 127) / 128;
+        const int grid = (J.np + 127) / 128, grid_slow = adj_grid(J.np);
         const int nseg = (J.nsteps + J.K - 1) / J.K;
-        // segment seg's records live in rec[seg & 1]: recomputing seg - 1 on
-        // the second stream waits only for the walk through seg + 1, the last
-        // reader of that buffer
+        const int streams = std::max(1, J.nrec - 1);
+        for (int k = 0; k < streams; ++k) check(cudaStreamWaitEvent(J.ahead[k], J.e0, 0), "wait");
+        // segment seg's records live in rec[seg % nrec]: recomputing it waits
+        // only for the walk through seg + nrec, the last reader of that buffer
         auto recompute = [&](int seg) {
             AdjArgs r = a;
-            r.rec = J.rec[seg & 1].p;
-            if (seg + 2 < nseg) check(cudaStreamWaitEvent(J.stream2, J.done1[seg + 2], 0), "wait");
-            if (J.has_yar) adj_recompute_kernel<true><<<grid, 128, 0, J.stream2>>>(r, seg);
-            else adj_recompute_kernel<false><<<grid, 128, 0, J.stream2>>>(r, seg);
-            check(cudaEventRecord(J.done2[seg], J.stream2), "event");
+            cudaStream_t s = J.ahead[seg % streams];
+            r.rec = J.rec[seg % J.nrec].p;
+            if (seg + J.nrec < nseg) check(cudaStreamWaitEvent(s, J.done1[seg + J.nrec], 0), "wait");
+            if (J.has_yar) adj_recompute_kernel<true><<<grid_slow, 128, 0, s>>>(r, seg);
+            else adj_recompute_kernel<false><<<grid_slow, 128, 0, s>>>(r, seg);
+            check(cudaEventRecord(J.done2[seg], s), "event");
         };
-        recompute(nseg - 1);
+        for (int seg = nseg - 1; seg > nseg - 1 - streams && seg >= 0; --seg) recompute(seg);
         for (int seg = nseg - 1; seg >= 0; --seg) {
             const int last = seg == nseg - 1 ? 1 : 0;
-            if (seg > 0) recompute(seg - 1);
+            if (seg - streams >= 0) recompute(seg - streams);
             check(cudaStreamWaitEvent(J.stream, J.done2[seg], 0), "wait");
             AdjArgs w = a;
-            w.rec = J.rec[seg & 1].p;
+            w.rec = J.rec[seg % J.nrec].p;
             if (J.has_yar) adj_vjp_kernel<true><<<grid, 128, 0, J.stream>>>(w, seg, last);
             else adj_vjp_kernel<false><<<grid, 128, 0, J.stream>>>(w, seg, last);
             check(cudaEventRecord(J.done1[seg], J.stream), "event");

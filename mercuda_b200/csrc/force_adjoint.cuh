@@ -5,32 +5,41 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fp64.cuh"
+
 namespace mb200 {
 
 // Yarkovsky (mfo_ngf, mercury6_2.for:5106-5153): a = yar t / (r^2 |t|) with
 // t = v - (x.v / r^2) x, differentiated in yar even where yar is zero.
 __device__ __forceinline__ void yar_vjp(const double3 x, const double3 v, double yar, const double3 la, double3& gx,
                                         double3& gv, double& gyar) {
-    const double r2 = x.x * x.x + x.y * x.y + x.z * x.z;
-    const double p = x.x * v.x + x.y * v.y + x.z * v.z;
-    const double q = p / r2;
-    const double3 t = make_double3(v.x - q * x.x, v.y - q * x.y, v.z - q * x.z);
-    const double tn = sqrt(t.x * t.x + t.y * t.y + t.z * t.z);
-    const double A = la.x * t.x + la.y * t.y + la.z * t.z;
-    const double k = yar / (r2 * tn);
-    const double kt = A * yar / (r2 * tn * tn * tn);
-    const double3 lt = make_double3(k * la.x - kt * t.x, k * la.y - kt * t.y, k * la.z - kt * t.z);
-    double lr2 = -A * yar / (r2 * r2 * tn);
-    gyar += A / (r2 * tn);
+    // 1/r^2 and 1/|t| to half an ulp, shared (the gradient is not bound to the
+    // reference's roundings)
+    const double r2 = fma(x.x, x.x, fma(x.y, x.y, x.z * x.z));
+    const double p = fma(x.x, v.x, fma(x.y, v.y, x.z * v.z));
+    const double ir2 = recip_near(r2);
+    const double q = p * ir2;
+    const double3 t = make_double3(fma(-q, x.x, v.x), fma(-q, x.y, v.y), fma(-q, x.z, v.z));
+    const double t2 = fma(t.x, t.x, fma(t.y, t.y, t.z * t.z));
+    double tn, itn;
+    sqrt_near(t2, tn, itn);
+    if (!mid_range(t2)) itn = div_plain(1.0, sqrt_plain(t2));
+    const double A = fma(la.x, t.x, fma(la.y, t.y, la.z * t.z));
+    const double w = ir2 * itn;
+    const double k = yar * w;
+    const double kt = A * k * itn * itn;
+    const double3 lt = make_double3(fma(k, la.x, -kt * t.x), fma(k, la.y, -kt * t.y), fma(k, la.z, -kt * t.z));
+    double lr2 = -A * k * ir2;
+    gyar += A * w;
     gv.x += lt.x;
     gv.y += lt.y;
     gv.z += lt.z;
-    const double lq = -(lt.x * x.x + lt.y * x.y + lt.z * x.z);
+    const double lq = -fma(lt.x, x.x, fma(lt.y, x.y, lt.z * x.z));
     gx.x -= q * lt.x;
     gx.y -= q * lt.y;
     gx.z -= q * lt.z;
-    const double lp = lq / r2;
-    lr2 -= lq * p / (r2 * r2);
+    const double lp = lq * ir2;
+    lr2 -= lp * q;
     gx.x += lp * v.x + 2.0 * lr2 * x.x;
     gx.y += lp * v.y + 2.0 * lr2 * x.y;
     gx.z += lp * v.z + 2.0 * lr2 * x.z;

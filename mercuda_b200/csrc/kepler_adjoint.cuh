@@ -16,12 +16,30 @@
 #include <math.h>
 
 #ifdef __CUDACC__
+#include "fp64.cuh"
+#endif
+
+#ifdef __CUDACC__
 #define MB200_HD __host__ __device__
 #else
 #define MB200_HD
 #endif
 
 namespace mb200 {
+
+// The gradient is not bound to the reference's roundings: fused multiply-adds
+// where they fit, and reciprocals to half an ulp shared by the divisions.
+MB200_HD inline double adj_recip(double b) {
+#ifdef __CUDA_ARCH__
+    return recip_near(b);
+#else
+    return 1.0 / b;
+#endif
+}
+MB200_HD inline double dot3(const double a[3], const double b[3]) {
+    return fma(a[0], b[0], fma(a[1], b[1], a[2] * b[2]));
+}
+MB200_HD inline double det2(double a, double b, double c, double d) { return fma(a, b, -(c * d)); }
 
 // Stumpff functions c0..c5 of z. For |z| < 1, c4 and c5 by their series and
 // the rest by c_k = 1/k! - z c_{k+2}; beyond, the closed forms.
@@ -82,30 +100,26 @@ MB200_HD inline void gfuncs(double s, double alpha, double G[6]) {
 
 // A starting value of the universal anomaly from the drift's end position x1:
 // g and f follow from x x x1 = g (x x v) and x1 x v = f (x x v), then
-// G2 = (1 - f) r0 / mu, G1 = (g - sigma0 G2) / r0, G0 = 1 - alpha G2, and s is
-// the angle (or hyperbolic angle) with cosine G0 and sine sqrt(alpha) G1.
-MB200_HD inline double anomaly_guess(const double x[3], const double v[3], const double x1[3], double r0,
-                                     double sig0, double alpha, double mu, double dt) {
-    const double h[3] = {x[1] * v[2] - x[2] * v[1], x[2] * v[0] - x[0] * v[2], x[0] * v[1] - x[1] * v[0]};
-    const double hh = h[0] * h[0] + h[1] * h[1] + h[2] * h[2];
-    const double fallback = dt / r0;
+// G2 = (1 - f) r0 / mu, G1 = (g - sigma0 G2) / r0, and by Kepler's equation
+// G3 = (dt - r0 G1 - sigma0 G2) / mu; c1 = 1 - z c3 makes that s = G1 + alpha
+// G3, for any alpha and without a trigonometric function, to a few roundings
+// (the cancellations in G2 and G3 enter multiplied by sigma0 and alpha).
+MB200_HD inline double anomaly_guess(const double x[3], const double v[3], const double x1[3], double r0, double ir0,
+                                     double sig0, double alpha, double mu, double imu, double dt) {
+    const double h[3] = {det2(x[1], v[2], x[2], v[1]), det2(x[2], v[0], x[0], v[2]), det2(x[0], v[1], x[1], v[0])};
+    const double hh = dot3(h, h);
+    const double fallback = dt * ir0;
     if (!(hh > 0.0)) return fallback;
-    const double a[3] = {x[1] * x1[2] - x[2] * x1[1], x[2] * x1[0] - x[0] * x1[2], x[0] * x1[1] - x[1] * x1[0]};
-    const double b[3] = {x1[1] * v[2] - x1[2] * v[1], x1[2] * v[0] - x1[0] * v[2], x1[0] * v[1] - x1[1] * v[0]};
-    const double g = (a[0] * h[0] + a[1] * h[1] + a[2] * h[2]) / hh;
-    const double f = (b[0] * h[0] + b[1] * h[1] + b[2] * h[2]) / hh;
-    const double G2 = (1.0 - f) * r0 / mu;
-    const double G1 = (g - sig0 * G2) / r0;
-    double s;
-    if (alpha > 0.0) {
-        const double w = sqrt(alpha);
-        s = atan2(w * G1, 1.0 - alpha * G2) / w;
-    } else if (alpha < 0.0) {
-        const double w = sqrt(-alpha);
-        s = asinh(w * G1) / w;
-    } else {
-        s = G1;
-    }
+    const double a[3] = {det2(x[1], x1[2], x[2], x1[1]), det2(x[2], x1[0], x[0], x1[2]),
+                         det2(x[0], x1[1], x[1], x1[0])};
+    const double b[3] = {det2(x1[1], v[2], x1[2], v[1]), det2(x1[2], v[0], x1[0], v[2]),
+                         det2(x1[0], v[1], x1[1], v[0])};
+    const double ih = adj_recip(hh);
+    const double g = dot3(a, h) * ih;
+    const double f = dot3(b, h) * ih;
+    const double G2 = (1.0 - f) * r0 * imu;
+    const double G1 = fma(-sig0, G2, g) * ir0;
+    const double s = fma(alpha * imu, fma(-sig0, G2, fma(-r0, G1, dt)), G1);
     return isfinite(s) ? s : fallback;
 }
 
@@ -140,50 +154,69 @@ MB200_HD inline bool universal_anomaly(double r0, double sig0, double alpha, dou
 // converge.
 MB200_HD inline bool drift_vjp(double mu, const double x[3], const double v[3], double dt, const double x1[3],
                               const double lx1[3], const double lv1[3], double lx[3], double lv[3]) {
-    const double r0 = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-    const double sig0 = x[0] * v[0] + x[1] * v[1] + x[2] * v[2];
-    const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-    const double alpha = 2.0 * mu / r0 - vv;
-    double s = anomaly_guess(x, v, x1, r0, sig0, alpha, mu, dt);
-    if (!universal_anomaly(r0, sig0, alpha, mu, dt, s)) return false;
+    const double r02 = dot3(x, x);
+    const double sig0 = dot3(x, v);
+#ifdef __CUDA_ARCH__
+    double r0, ir0;
+    sqrt_near(r02, r0, ir0);
+#else
+    const double r0 = sqrt(r02), ir0 = 1.0 / r0;
+#endif
+    const double imu = adj_recip(mu);
+    const double alpha = fma(2.0 * mu, ir0, -dot3(v, v));
+    double s = anomaly_guess(x, v, x1, r0, ir0, sig0, alpha, mu, imu, dt);
     double G[6];
     gfuncs(s, alpha, G);
-    const double r = r0 * G[0] + sig0 * G[1] + mu * G[2];
-    const double f = 1.0 - mu * G[2] / r0;
-    const double g = r0 * G[1] + sig0 * G[2];
-    const double fd = -mu * G[1] / (r * r0);
-    const double gd = 1.0 - mu * G[2] / r;
+    // one Newton step, and the G functions moved along it by dG_k/ds = G_{k-1}
+    // to second order: with the usual guess the third is far below a rounding;
+    // a poor one goes through the iteration
+    const double F = fma(r0, G[1], fma(sig0, G[2], fma(mu, G[3], -dt)));
+    const double ds = -F * adj_recip(fma(r0, G[0], fma(sig0, G[1], mu * G[2])));
+    if (fabs(ds) <= 1e-7 * fabs(s)) {
+        const double d2 = 0.5 * ds * ds, Gm1 = -alpha * G[1], Gm2 = -alpha * G[0];
+        G[5] += fma(ds, G[4], d2 * G[3]);
+        G[4] += fma(ds, G[3], d2 * G[2]);
+        G[3] += fma(ds, G[2], d2 * G[1]);
+        G[2] += fma(ds, G[1], d2 * G[0]);
+        G[1] += fma(ds, G[0], d2 * Gm1);
+        G[0] += fma(ds, Gm1, d2 * Gm2);
+        s += ds;
+    } else {
+        if (!universal_anomaly(r0, sig0, alpha, mu, dt, s)) return false;
+        gfuncs(s, alpha, G);
+    }
+    const double r = fma(r0, G[0], fma(sig0, G[1], mu * G[2]));
+    const double ir = adj_recip(r), irr = ir * ir0;
+    const double f = fma(-mu * G[2], ir0, 1.0);
+    const double g = fma(r0, G[1], sig0 * G[2]);
+    const double fd = -mu * G[1] * irr;
+    const double gd = fma(-mu * G[2], ir, 1.0);
     // derivatives of G0..G3 with respect to alpha (fixed s) and s
     double Ga[4], Gs[4];
-    for (int k = 0; k < 4; ++k) Ga[k] = 0.5 * (k * G[k + 2] - s * G[k + 1]);
+    for (int k = 0; k < 4; ++k) Ga[k] = 0.5 * fma((double)k, G[k + 2], -s * G[k + 1]);
     Gs[0] = -alpha * G[1];
     for (int k = 1; k < 4; ++k) Gs[k] = G[k - 1];
     // ds/dtheta for theta = r0, sigma0, alpha
-    const double Fa = r0 * Ga[1] + sig0 * Ga[2] + mu * Ga[3];
-    const double dsd[3] = {-G[1] / r, -G[2] / r, -Fa / r};
-    const double ra = r0 * Ga[0] + sig0 * Ga[1] + mu * Ga[2];
-    const double rs = r0 * Gs[0] + sig0 * Gs[1] + mu * Gs[2];
-    const double c1 = lx1[0] * x[0] + lx1[1] * x[1] + lx1[2] * x[2];
-    const double c2 = lx1[0] * v[0] + lx1[1] * v[1] + lx1[2] * v[2];
-    const double c3 = lv1[0] * x[0] + lv1[1] * x[1] + lv1[2] * x[2];
-    const double c4 = lv1[0] * v[0] + lv1[1] * v[1] + lv1[2] * v[2];
+    const double Fa = fma(r0, Ga[1], fma(sig0, Ga[2], mu * Ga[3]));
+    const double dsd[3] = {-G[1] * ir, -G[2] * ir, -Fa * ir};
+    const double ra = fma(r0, Ga[0], fma(sig0, Ga[1], mu * Ga[2]));
+    const double rs = fma(r0, Gs[0], fma(sig0, Gs[1], mu * Gs[2]));
+    const double c1 = dot3(lx1, x), c2 = dot3(lx1, v), c3 = dot3(lv1, x), c4 = dot3(lv1, v);
     double DS[3];
     for (int t = 0; t < 3; ++t) {
         const double is_r0 = t == 0 ? 1.0 : 0.0, is_sig = t == 1 ? 1.0 : 0.0, is_a = t == 2 ? 1.0 : 0.0;
-        double DG[4];
-        for (int k = 0; k < 4; ++k) DG[k] = is_a * Ga[k] + Gs[k] * dsd[t];
-        const double DR = is_r0 * G[0] + is_sig * G[1] + is_a * ra + rs * dsd[t];
-        const double Df = -mu * DG[2] / r0 + is_r0 * mu * G[2] / (r0 * r0);
-        const double Dg = is_r0 * G[1] + is_sig * G[2] + r0 * DG[1] + sig0 * DG[2];
-        const double rr0 = r * r0;
-        const double Dfd = -mu * (DG[1] / rr0 - G[1] * (DR * r0 + r * is_r0) / (rr0 * rr0));
-        const double Dgd = -mu * (DG[2] / r - G[2] * DR / (r * r));
-        DS[t] = c1 * Df + c2 * Dg + c3 * Dfd + c4 * Dgd;
+        const double DG1 = fma(Gs[1], dsd[t], is_a * Ga[1]), DG2 = fma(Gs[2], dsd[t], is_a * Ga[2]);
+        const double DR = fma(rs, dsd[t], is_r0 * G[0] + is_sig * G[1] + is_a * ra);
+        const double Df = -mu * (DG2 - is_r0 * G[2] * ir0) * ir0;
+        const double Dg = fma(r0, DG1, fma(sig0, DG2, is_r0 * G[1] + is_sig * G[2]));
+        const double Dfd = -mu * fma(-G[1], fma(DR, ir, is_r0 * ir0), DG1) * irr;
+        const double Dgd = -mu * fma(-G[2] * DR, ir, DG2) * ir;
+        DS[t] = fma(c1, Df, fma(c2, Dg, fma(c3, Dfd, c4 * Dgd)));
     }
-    const double kx = DS[0] / r0 - DS[2] * 2.0 * mu / (r0 * r0 * r0);
+    const double kx = fma(-2.0 * mu * DS[2], ir0 * ir0, DS[0]) * ir0;
     for (int c = 0; c < 3; ++c) {
-        lx[c] = f * lx1[c] + fd * lv1[c] + kx * x[c] + DS[1] * v[c];
-        lv[c] = g * lx1[c] + gd * lv1[c] + DS[1] * x[c] - 2.0 * DS[2] * v[c];
+        lx[c] = fma(f, lx1[c], fma(fd, lv1[c], fma(kx, x[c], DS[1] * v[c])));
+        lv[c] = fma(g, lx1[c], fma(gd, lv1[c], fma(DS[1], x[c], -2.0 * DS[2] * v[c])));
     }
     return true;
 }
