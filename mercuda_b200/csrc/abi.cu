@@ -1,6 +1,7 @@
 // The drop-in C ABI (include/mercury_cuda.h) and the MVS extension entry
 // points (include/mercury_b200.h): host orchestration of the device context.
 #include <algorithm>
+#include <optional>
 #include <array>
 #include <cmath>
 #include <cstdlib>
@@ -351,9 +352,10 @@ MvsParticleArgs particle_args(int in, int out, int nsteps, int reset, int centra
 // encounter candidates into event records (same stream, the records, status
 // and candidates pa names). detail is the base of the run's pair details: a
 // candidate carries its step within the run.
-void particles_and_events(const MvsParticleArgs& pa, const double* detail, cudaStream_t s) {
+// `fresh`: the status was cleared for this launch alone.
+void particles_and_events(const MvsParticleArgs& pa, const double* detail, cudaStream_t s, bool fresh = false) {
     Context& c = ctx();
-    check(cudaMemsetAsync(pa.tiles ? pa.tiles : &pa.status->next_tile, 0, sizeof(int), s), "memset");
+    if (!fresh) check(cudaMemsetAsync(pa.tiles ? pa.tiles : &pa.status->next_tile, 0, sizeof(int), s), "memset");
     launch_mvs_particles(pa, s, c.particle_threads);
     ClassifyArgs ca{};
     ca.nb = c.nbig - 1;
@@ -368,7 +370,7 @@ void particles_and_events(const MvsParticleArgs& pa, const double* detail, cudaS
     ca.status = pa.status;
     ca.step_base = 0;
     if (ca.nb > 0) launch_classify(ca, s);
-    check(cudaMemsetAsync(&pa.status->cands, 0, sizeof(int), s), "memset");
+    if (!fresh) check(cudaMemsetAsync(&pa.status->cands, 0, sizeof(int), s), "memset");
 }
 
 // Candidate room for a launch of `steps` steps: box overlaps run at 2-4 % of
@@ -427,15 +429,29 @@ __global__ void spec_merge_kernel(const DeviceStatus* ss, const MercuryEvent* se
                                   DeviceStatus* st, MercuryEvent* ev, int* ev_step, int cap) {
     const int n = ss->events;
     if (threadIdx.x == 0 && blockIdx.x == 0) {
-        st->events = n;
-        st->fault |= ss->fault;
-        if (n > scap || n > cap || ss->overflow) st->overflow |= 1;
+        DeviceStatus fresh{};
+        fresh.events = n;
+        fresh.fault = ss->fault;
+        fresh.overflow = n > scap || n > cap || ss->overflow ? 1 : 0;
+        *st = fresh;
     }
     const int m = min(n, min(scap, cap));
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
         store_event(ev + k, sev[k]);
         ev_step[k] = sstep[k];
     }
+}
+
+// A step's status and first records straight into page-locked memory, only as
+// many as there are: one launch of a few us instead of two copies, one of
+// them of the whole first 128 KB.
+__global__ void __launch_bounds__(256) publish_kernel(const DeviceStatus* st, const MercuryEvent* ev, int cap,
+                                                      DeviceStatus* host_st, MercuryEvent* host_ev, int head) {
+    const int n = min(min(st->events, cap), head);
+    const int4* src = reinterpret_cast<const int4*>(ev);
+    int4* dst = reinterpret_cast<int4*>(host_ev);
+    for (int k = threadIdx.x; k < 8 * n; k += blockDim.x) dst[k] = src[k];
+    if (threadIdx.x == 0) *host_st = *st;
 }
 
 // Waits for the speculative step (host-side: later calls may copy into its
@@ -505,10 +521,10 @@ void spec_launch(double h, double rcen) {
     check(cudaEventRecord(c.spec_ready, c.stream), "event");
     check(cudaStreamWaitEvent(s, c.spec_ready, 0), "wait");
     const int cap = (int)c.spec_events.n;
-    check(cudaMemsetAsync(c.spec_status.p, 0, sizeof(DeviceStatus), s), "memset");
     if (c.ah_live && c.ah_h == h && c.ah_rcen == rcen) {
         // this step's Big bodies ran ahead: their state, table rows and
-        // details become the step's, their records its first records
+        // details become the step's, their records its first records (and its
+        // status a fresh one with them)
         check(cudaStreamWaitEvent(s, c.ah_done, 0), "wait");
         std::swap(c.spec_big, c.ah_state);
         std::swap(c.spec_tab, c.ah_tab);
@@ -517,6 +533,7 @@ void spec_launch(double h, double rcen) {
                                             c.spec_status.p, c.spec_events.p, c.spec_event_step.p, cap);
     } else {
         spec_drop();
+        check(cudaMemsetAsync(c.spec_status.p, 0, sizeof(DeviceStatus), s), "memset");
         MvsBigArgs a = big_args(c.cur, 1 - c.cur, 1, 0, cen, 0, h, rcen, c.spec_tab.p, c.spec_detail.p);
         a.out = big_state_at(c.spec_big.p, c.nsplit);
         a.events = c.spec_events.p;
@@ -531,7 +548,6 @@ void spec_launch(double h, double rcen) {
     // writes are read
     check(cudaEventRecord(c.spec_merged, s), "event");
     check(cudaStreamWaitEvent(sa, c.spec_merged, 0), "wait");
-    check(cudaMemsetAsync(c.ah_status.p, 0, sizeof(DeviceStatus), sa), "memset");
     MvsBigArgs b = big_args(c.cur, 1 - c.cur, 1, 0, cen, 0, h, rcen, c.ah_tab.p, c.ah_detail.p);
     b.in = big_state_at(c.spec_big.p, c.nsplit);
     b.out = big_state_at(c.ah_state.p, c.nsplit);
@@ -539,6 +555,7 @@ void spec_launch(double h, double rcen) {
     b.event_step = c.ah_event_step.p;
     b.event_cap = AHEAD_RECORDS;
     b.status = c.ah_status.p;
+    b.fresh_status = 1;
     launch_mvs_big(b, sa);
     check(cudaEventRecord(c.ah_done, sa), "event");
     c.dropin_launches += 1;
@@ -552,15 +569,12 @@ void spec_launch(double h, double rcen) {
         pa.event_step = c.spec_event_step.p;
         pa.event_cap = cap;
         pa.status = c.spec_status.p;
-        particles_and_events(pa, c.spec_detail.p, s);
+        particles_and_events(pa, c.spec_detail.p, s, true);
         c.dropin_launches += 1 + (nb > 0 ? 1 : 0);
     }
-    check(cudaMemcpyAsync(c.spec_status_host, c.spec_status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, s),
-          "status");
-    const int head = std::min(Context::EVENT_HEAD, cap);
-    if (head > 0)
-        check(cudaMemcpyAsync(c.spec_head, c.spec_events.p, sizeof(MercuryEvent) * head, cudaMemcpyDeviceToHost, s),
-              "events");
+    publish_kernel<<<1, 256, 0, s>>>(c.spec_status.p, c.spec_events.p, cap, c.spec_status_host, c.spec_head,
+                                     Context::EVENT_HEAD);
+    c.dropin_launches += 1;
     check(cudaGetLastError(), "launch");
     check(cudaEventRecord(c.spec_done, s), "event");
     c.spec_live = true;
@@ -588,8 +602,7 @@ bool spec_take(double h, double rcen) {
     std::swap(c.event_step, c.spec_event_step);
     std::swap(c.ev_head, c.spec_head);
     *c.status_host = st;
-    check(cudaMemcpyAsync(c.status.p, c.spec_status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToDevice, c.stream),
-          "status");
+    std::swap(c.status, c.spec_status);
     c.head_ready = true;
     c.head_count = std::min(Context::EVENT_HEAD, (int)c.events.n);
     return true;
@@ -628,7 +641,7 @@ void mvs_step_once(double h) {
         c.dropin_launches += 1 + (c.np > 0 ? 1 + (c.nbig > 1 ? 1 : 0) : 0);
         if (c.np > 0)
             particles_and_events(particle_args(in, out, 1, reset, cen, 0, h, rc, c.tab.p, c.detail.p), c.detail.p,
-                                 c.stream);
+                                 c.stream, true);
         check(cudaGetLastError(), "launch");
         read_status();
         if (c.status_host->fault) throw std::runtime_error("MVS force failed");
@@ -2117,7 +2130,7 @@ int mercury_cuda_step(double time, double* h, double* hdid, double tol, int64_t*
         inject("step");
         require_system();
         const bool adaptive = c.algorithm >= 2 && c.algorithm <= 4;
-        DropinTimer timer(adaptive && !c.encounter);
+        DropinTimer timer((adaptive || is_mvs(c.algorithm)) && !c.encounter);
         c.screen_live = false;
         *rejected = 0;
         const int64_t before = c.nforces;
@@ -2162,7 +2175,11 @@ int mercury_cuda_events(double time, double h, double rcen, const MercuryEvent**
     try {
         inject("events");
         require_system();
-        DropinTimer timer(c.algorithm >= 2 && c.algorithm <= 4 && !c.encounter);
+        // (nothing to time where the records are on the host already)
+        const bool on_host = is_mvs(c.algorithm) && c.stepped && c.step_central && c.head_ready && rcen == c.step_rcen &&
+                             h == c.step_h;
+        std::optional<DropinTimer> timer;
+        if (!on_host) timer.emplace((is_mvs(c.algorithm) || (c.algorithm >= 2 && c.algorithm <= 4)) && !c.encounter);
         const int prev = 1 - c.cur;
         const bool adaptive = !is_mvs(c.algorithm) && c.algorithm != 10 && c.stepped;
         const bool dh = c.algorithm == 10 && c.stepped;

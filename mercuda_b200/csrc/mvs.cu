@@ -454,6 +454,7 @@ __device__ void big_force(const MvsBigArgs& A, BigSmem& S, double* row) {
 
 __device__ void big_load(const MvsBigArgs& A, BigSmem& S, double* smem) {
     const int N = big_count(A), tid = threadIdx.x, nt = blockDim.x;
+    if (A.fresh_status && tid == 0) *A.status = DeviceStatus{};   // big_constants synchronizes
     S.base = smem;
     S.N = N;
     S.now = 0;
@@ -1192,14 +1193,26 @@ void launch_variant(const MvsParticleArgs& a, cudaStream_t s, int threads) {
     const size_t smem = mvs_particle_smem(a.nb, a.nsteps, a.reset, threads, NGF);
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int tiles = (a.np + threads - 1) / threads;
-    int dev = 0, sms = 148, per_sm = 1;
+    // the device's room for this launch shape, asked for when it changes (a
+    // per-step host launches the same shape every time)
+    static thread_local struct {
+        int dev = -1, threads = 0, slots = 1;
+        size_t smem = 0;
+    } room;
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-    if (per_sm < 1) per_sm = 1;
+    if (room.dev != dev || room.threads != threads || room.smem != smem) {
+        int sms = 148, per_sm = 1;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+        room.dev = dev;
+        room.threads = threads;
+        room.smem = smem;
+        room.slots = sms * (per_sm < 1 ? 1 : per_sm);
+    }
     // One CTA slot fewer than the device holds, so that the Big-body CTA of
     // the next chunk (another stream) can start beside this persistent grid.
-    int slots = sms * per_sm - 1;
+    int slots = room.slots - 1;
     if (slots < 1) slots = 1;
     const int grid = tiles < slots ? tiles : slots;
     if (grid > 0) kern<<<grid, threads, smem, s>>>(a);

@@ -46,6 +46,7 @@ struct MvsBigArgs {
     int nsteps;
     int central;        // screen Big bodies against the central body (fused runs)
     int step0;          // global index of the first step (for event step tags)
+    int fresh_status;   // clear *status first (no other launch uses it meanwhile)
     double jcen[3];
     double h;
     double rcen;
