@@ -1015,13 +1015,13 @@ void launch_central(double h, double rcen, bool dh) {
     check(cudaGetLastError(), "central");
 }
 
-// The status and the first records into pinned memory, queued.
+// The status and the first records into page-locked memory, queued.
 int queue_records(DeviceStatus* status, MercuryEvent* head) {
     Context& c = ctx();
     const int n = c.stepped ? std::min(Context::EVENT_HEAD, (int)c.events.n) : 0;
-    check(cudaMemcpyAsync(status, c.status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, c.stream), "status");
-    if (n > 0)
-        check(cudaMemcpyAsync(head, c.events.p, sizeof(MercuryEvent) * n, cudaMemcpyDeviceToHost, c.stream), "events");
+    publish_kernel<<<1, 256, 0, c.stream>>>(c.status.p, c.events.p, (int)c.events.n, status, head, n);
+    c.dropin_launches += 1;
+    check(cudaGetLastError(), "publish");
     return n;
 }
 

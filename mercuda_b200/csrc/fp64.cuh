@@ -12,8 +12,9 @@
 // third-order step to half an ulp, then one correction by the exact residual.
 // The value before the last rounding is within 2^-103 of the true one, so the
 // result is the IEEE one unless the true value lies that close to the middle
-// of two doubles (an exact quotient or root always comes out exact); 2^36
-// random operands and the nearest ones to a middle gave no difference.
+// of two doubles (an exact quotient or root always comes out exact). 2^36
+// random operands and 400,000 quotients and roots made to lie next to a middle
+// gave no difference; of 14,218 operands made so for 1/sqrt one did, by an ulp.
 // A denominator that several quotients share pays for its reciprocal once,
 // and sqrt and 1/sqrt share one seed.
 //
