@@ -162,21 +162,7 @@ __global__ void central_kernel(CentralArgs A) {
         }
         hit = central_impact(p0, u0, p1, u1, A.mu, mj, A.h, A.rcen, temp);
     }
-    if (hit) {
-        const int slot = atomicAdd(&A.status->events, 1);
-        if (slot < A.cap) {
-            MercuryEvent rec = {};
-            rec.i = 1;
-            rec.j = id;
-            rec.kind = EV_CENTRAL;
-            rec.time = temp;
-            rec.distance = A.rcen;
-            store_event(A.events + slot, rec);
-            A.event_step[slot] = 0;
-        } else {
-            atomicExch(&A.status->overflow, 1);
-        }
-    }
+    if (hit) central_record(A.events, A.event_step, A.cap, A.status, id, temp, A.rcen, 0);
 }
 
 int blocks(int n, int t = 256) { return (n + t - 1) / t; }
@@ -440,6 +426,23 @@ __global__ void spec_merge_kernel(const DeviceStatus* ss, const MercuryEvent* se
         store_event(ev + k, sev[k]);
         ev_step[k] = sstep[k];
     }
+}
+
+// What an adaptive attempt's decision needs, into page-locked memory, and the
+// status cleared for the screens behind the decision: the level maxima and
+// faults of BS (errs not null) or the status itself. One launch instead of two
+// copies and a memset, each of which holds the stream for some microseconds.
+__global__ void __launch_bounds__(64) take_status_kernel(DeviceStatus* st, DeviceStatus* host_st,
+                                                         const unsigned long long* errs, const DeviceStatus* lv,
+                                                         Context::BsLevels* host_lv) {
+    const int k = threadIdx.x;
+    if (errs && k < 13) {
+        host_lv->errs[k] = errs[k];
+        host_lv->lv[k] = lv[k];
+    }
+    if (k != 32) return;
+    if (!errs) *host_st = *st;
+    *st = DeviceStatus{};
 }
 
 // A step's status and first records straight into page-locked memory, only as
@@ -711,7 +714,10 @@ void ra15_step_once(double time, double* h, double* hdid, double tol, int64_t* r
         launch_ra15_sequence(a, c.stream);
         c.dropin_launches += 1 + (c.np > 0 ? 1 : 0);
         check(cudaGetLastError(), "launch");
-        read_status();
+        take_status_kernel<<<1, 64, 0, c.stream>>>(c.status.p, c.status_host, nullptr, nullptr, nullptr);
+        c.dropin_launches += 1;
+        check(cudaGetLastError(), "launch");
+        check(cudaStreamSynchronize(c.stream), "step");
         c.nforces += 1 + 7 * niter;
         double err;
         std::memcpy(&err, &c.status_host->max_b7, sizeof(err));
@@ -756,7 +762,7 @@ void ra15_step_once(double time, double* h, double* hdid, double tol, int64_t* r
 
 // Every level of one mdt_bs1 (algorithm 2) or mdt_bs2 (algorithm 3) attempt
 // at trial step h from the current state buffer: per-level error maxima in
-// bs_errs, per-level force faults in bs_lvst, candidates for the commit.
+// bs_levels, candidates for the commit.
 // The arguments of one BS/BS2 attempt from the current buffer with trial
 // step h (the workspace reserved).
 BsArgs bs_attempt_args(double h) {
@@ -767,8 +773,7 @@ BsArgs bs_attempt_args(double h) {
     c.bs_scr.reserve(bs_massive_scratch(V, N, nb));
     c.bs_bcand.reserve((size_t)bs_candidates(V) * 6 * N);
     c.bs_pcand.reserve((size_t)bs_candidates(V) * 6 * c.npcap);
-    c.bs_errs.reserve(13);
-    c.bs_lvst.reserve(13);
+    c.bs_levels.reserve(1);
     const int in = c.cur;
     BsArgs a{};
     a.f = force_cfg();
@@ -786,8 +791,8 @@ BsArgs bs_attempt_args(double h) {
     a.table = c.ftab.p;
     a.bcand = c.bs_bcand.p;
     a.pcand = c.bs_pcand.p;
-    a.errs = c.bs_errs.p;
-    a.lvst = c.bs_lvst.p;
+    a.errs = c.bs_levels.p->errs;
+    a.lvst = c.bs_levels.p->lv;
     a.hkce = c.encounter ? 1 : 0;
     a.rcrit = c.rcritbig.p;
     a.adj_off = c.adj_off.p;
@@ -805,8 +810,7 @@ BsArgs bs_attempt_args(double h) {
 BsArgs launch_bs_attempt(double h) {
     Context& c = ctx();
     const BsArgs a = bs_attempt_args(h);
-    check(cudaMemsetAsync(c.bs_errs.p, 0, sizeof(unsigned long long) * 13, c.stream), "memset");
-    check(cudaMemsetAsync(c.bs_lvst.p, 0, sizeof(DeviceStatus) * 13, c.stream), "memset");
+    check(cudaMemsetAsync(c.bs_levels.p, 0, sizeof(Context::BsLevels), c.stream), "memset");
     launch_bs_sequence(a, c.stream);
     c.dropin_launches += 2 + (c.np > 0 ? 1 : 0);  // level CTAs, extrapolation, particles
     check(cudaGetLastError(), "launch");
@@ -891,11 +895,9 @@ void bs_step_once(double time, double* h, double* hdid, double tol, int64_t* rej
         const unsigned long long* errs = c.bs_host->errs;
         const DeviceStatus* lv = c.bs_host->lv;
         auto read_levels = [&] {
-            check(cudaMemcpyAsync(c.bs_host->errs, c.bs_errs.p, sizeof(c.bs_host->errs), cudaMemcpyDeviceToHost,
-                                  c.stream),
-                  "status");
-            check(cudaMemcpyAsync(c.bs_host->lv, c.bs_lvst.p, sizeof(c.bs_host->lv), cudaMemcpyDeviceToHost, c.stream),
-                  "status");
+            take_status_kernel<<<1, 64, 0, c.stream>>>(c.status.p, nullptr, a.errs, a.lvst, c.bs_host);
+            c.dropin_launches += 1;
+            check(cudaGetLastError(), "launch");
             check(cudaStreamSynchronize(c.stream), "step");
         };
         read_levels();
@@ -929,16 +931,10 @@ void bs_step_once(double time, double* h, double* hdid, double tol, int64_t* rej
     }
 }
 
-// mce_stat between the buffers before and after the last step of an adaptive
-// integrator (mercury6_2.for:1765-1918): Big/massive pairs by one CTA, the
-// particles' box overlaps as candidates, classified like the MVS path's.
-// Records are appended at the status counter and tagged `step`; the caller
-// clears the candidate counter first.
-void launch_pair_screen(double h, int step) {
+// mce_stat and mce_cent between the buffers before and after the last step of
+// an adaptive integrator (mercury6_2.for:1765-1918, 1059-1167), one launch.
+void launch_step_screens(double h, double rcen) {
     Context& c = ctx();
-    const int nb = c.nbig - 1;
-    c.boxes.reserve((size_t)4 * std::max(1, nb));
-    c.detail.reserve((size_t)std::max(1, nb) * TAB_DETAIL);
     const int cur = c.cur, prev = 1 - cur;
     ScreenArgs a{};
     a.nbig = c.nbig;
@@ -946,6 +942,8 @@ void launch_pair_screen(double h, int step) {
     a.np = c.np;
     a.npcap = c.npcap;
     a.h = h;
+    a.m0 = c.m_host[0];
+    a.rcen = rcen;
     a.b0 = c.bigstate[prev].p;
     a.b1 = c.bigstate[cur].p;
     a.mbig = c.mbig.p;
@@ -955,32 +953,12 @@ void launch_pair_screen(double h, int step) {
     a.p1 = c.pstate[cur].p;
     a.pconst = c.pconst[c.kc].p;
     a.perm = c.permp();
-    a.boxes = c.boxes.p;
-    a.detail = c.detail.p;
     a.events = c.events.p;
     a.event_step = c.event_step.p;
     a.event_cap = (int)c.events.n;
-    a.cands = c.cands.p;
-    a.cand_cap = (int)c.cands.n;
     a.status = c.status.p;
-    a.step = step;
     launch_screen(a, c.stream);
-    c.dropin_launches += 1 + (c.np > 0 && nb > 0 ? 2 : 0);
-    if (nb > 0 && c.np > 0) {
-        ClassifyArgs ca{};
-        ca.nb = nb;
-        ca.nbig = c.nbig;
-        ca.h = h;
-        ca.detail = c.detail.p;
-        ca.cands = c.cands.p;
-        ca.cand_cap = (int)c.cands.n;
-        ca.events = c.events.p;
-        ca.event_step = c.event_step.p;
-        ca.event_cap = (int)c.events.n;
-        ca.status = c.status.p;
-        ca.step_base = step;
-        launch_classify(ca, c.stream);
-    }
+    c.dropin_launches += 1;
     check(cudaGetLastError(), "screen");
 }
 
@@ -1026,12 +1004,10 @@ int queue_records(DeviceStatus* status, MercuryEvent* head) {
 }
 
 // Both screens of an adaptive integrator's last step, with their records
-// queued for the host: one round trip, and none between them.
+// queued for the host: one round trip, and none between them. The status is
+// clear: the step's own wait left it so.
 int queue_adaptive_screens(double h, double rcen, DeviceStatus* status, MercuryEvent* head) {
-    Context& c = ctx();
-    check(cudaMemsetAsync(c.status.p, 0, sizeof(DeviceStatus), c.stream), "memset");
-    launch_pair_screen(h, 0);
-    launch_central(h, rcen, false);
+    launch_step_screens(h, rcen);
     return queue_records(status, head);
 }
 
@@ -1039,7 +1015,8 @@ int queue_adaptive_screens(double h, double rcen, DeviceStatus* status, MercuryE
 // named the central radius, a step queues its screens itself, behind its
 // commit, and the events call finds the records on the host. A step of RADAU
 // with its screens (100,000 particles) made six waits for the device and left
-// it idle for 120 of 302 us; with two waits it takes 247.
+// it idle for 120 of 302 us; with two waits it took 247, with the screens in one
+// launch and no copies or clears between them (take_status_kernel) 200.
 void screen_ahead(double h) {
     Context& c = ctx();
     if (c.encounter || c.dropin_rcen <= 0.0) return;
@@ -1064,6 +1041,7 @@ int adaptive_records(double h, double rcen, const MercuryEvent** head) {
         grow_after_overflow();
     }
     for (int attempt = 0;; ++attempt) {
+        check(cudaMemsetAsync(c.status.p, 0, sizeof(DeviceStatus), c.stream), "memset");
         const int n = queue_adaptive_screens(h, rcen, c.status_host, c.ev_head);
         check(cudaStreamSynchronize(c.stream), "step");
         *head = c.ev_head;
@@ -3244,8 +3222,7 @@ void encounter_run_device(double time, double h, double tol, double* hrec, int64
     c.enc_ctl.reserve(2);
     c.enc_tstep.reserve(1024);
     c.enc_bpre.reserve((size_t)6 * c.nsplit);
-    c.bs_errs.reserve(26);
-    c.bs_lvst.reserve(26);
+    c.bs_levels.reserve(2);
     for (int redo = 0;; ++redo) {
         // the first substep's trial step: hrec, clipped to the subsystem's end
         EncCtl k{};
@@ -3268,8 +3245,8 @@ void encounter_run_device(double time, double h, double tol, double* hrec, int64
             const int p = number & 1;   // two control blocks alternate
             BsArgs a = base;
             a.ctl = c.enc_ctl.p + p;
-            a.errs = c.bs_errs.p + 13 * p;
-            a.lvst = c.bs_lvst.p + 13 * p;
+            a.errs = c.bs_levels.p[p].errs;
+            a.lvst = c.bs_levels.p[p].lv;
             launch_bs_sequence(a, c.stream);
             EncPostArgs e{};
             e.progress = c.enc_progress;
@@ -3278,8 +3255,8 @@ void encounter_run_device(double time, double h, double tol, double* hrec, int64
             e.ctl_out = c.enc_ctl.p + (1 - p);
             e.errs = a.errs;
             e.lvst = a.lvst;
-            e.errs_next = c.bs_errs.p + 13 * (1 - p);
-            e.lvst_next = c.bs_lvst.p + 13 * (1 - p);
+            e.errs_next = c.bs_levels.p[1 - p].errs;
+            e.lvst_next = c.bs_levels.p[1 - p].lv;
             e.nbig = c.nbig;
             e.nsplit = c.nsplit;
             e.np = c.np;
@@ -3304,8 +3281,7 @@ void encounter_run_device(double time, double h, double tol, double* hrec, int64
         };
         check(cudaMemcpyAsync(c.enc_ctl.p, c.enc_host, sizeof(EncCtl), cudaMemcpyHostToDevice, c.stream), "upload");
         check(cudaMemsetAsync(c.status.p, 0, sizeof(DeviceStatus), c.stream), "memset");
-        check(cudaMemsetAsync(c.bs_errs.p, 0, sizeof(unsigned long long) * 26, c.stream), "memset");
-        check(cudaMemsetAsync(c.bs_lvst.p, 0, sizeof(DeviceStatus) * 26, c.stream), "memset");
+        check(cudaMemsetAsync(c.bs_levels.p, 0, 2 * sizeof(Context::BsLevels), c.stream), "memset");
         // Attempts are queued AHEAD of the last one the device has decided, by
         // the count its decision kernel leaves in page-locked memory: enough to
         // keep it busy (three launches take the host ~8 us, an attempt ~25), and

@@ -85,8 +85,8 @@ struct Context {
     // RA15: B, E, G and predictor scratch of the massive set ([21][nsplit],
     // [6][nsplit]), B and E of the particle slots ([21][npcap]), the per-node
     // force table and the force entry's output ([3][nsplit] then
-    // [3][npcap]); screen boxes of the adaptive integrators ([nbig-1][4])
-    DBuf<double> ra_bb, ra_be, ra_bg, ra_bpx, ra_pb, ra_pe, ftab, force_out, boxes;
+    // [3][npcap])
+    DBuf<double> ra_bb, ra_be, ra_bg, ra_bpx, ra_pb, ra_pe, ftab, force_out;
     // output corrector scratch: Big [9][nbig], particles [6][npcap]
     DBuf<double> corr_big, corr_part;
     DBuf<double> energy_scr;         // mxx_en: per-body pair sums, then e and l2
@@ -94,8 +94,11 @@ struct Context {
     // Bulirsch-Stoer: massive-set scratch, per-level candidate states, per-level
     // error maxima and force-fault words
     DBuf<double> bs_scr, bs_bcand, bs_pcand, bs_ptab;
-    DBuf<unsigned long long> bs_errs;
-    DBuf<DeviceStatus> bs_lvst;
+    struct BsLevels {
+        unsigned long long errs[13];
+        DeviceStatus lv[13];
+    };
+    DBuf<BsLevels> bs_levels;   // two: the encounter attempts alternate
     // HYBRID: rcrit of the massive set, the massive set after the first solar
     // drift, the three force/begin rows, dh2h velocity shifts of the previous
     // and current states, members' packed rows, encounter pairs and member ids
@@ -201,10 +204,6 @@ struct Context {
     bool screen_live = false;
     double screen_h = 0.0, screen_rcen = 0.0;
     // each BS level's error maximum and force faults, read back at once
-    struct BsLevels {
-        unsigned long long errs[13];
-        DeviceStatus lv[13];
-    };
     BsLevels* bs_host = nullptr;
     // the last step's status and first records are in status_host / ev_head
     // already (head_count records)
@@ -264,7 +263,7 @@ struct Context {
     void release_all() {
         DBuf<double>* bufs[] = {&mbig, &rcebig, &rphysbig, &ngfbig, &bigstate[0], &bigstate[1], &pstate[0],
                                 &pstate[1], &pconst[0], &pconst[1], &tab, &detail, &transfer, &snapshot, &snap_const,
-                                &ra_bb, &ra_be, &ra_bg, &ra_bpx, &ra_pb, &ra_pe, &ftab, &force_out, &boxes, &corr_big, &corr_part, &energy_scr,
+                                &ra_bb, &ra_be, &ra_bg, &ra_bpx, &ra_pb, &ra_pe, &ftab, &force_out, &corr_big, &corr_part, &energy_scr,
                                 &bs_scr, &bs_bcand, &bs_pcand, &bs_ptab, &rcritbig, &hy_scr, &hy_tab, &hy_off,
                                 &hy_packed, &tg, &stage};
         for (auto* b : bufs) b->release();
@@ -274,8 +273,7 @@ struct Context {
         pinned_n = 0;
         DBuf<int>* ibufs[] = {&perm[0], &perm[1], &inv, &order_bucket, &order_hist, &snap_perm, &ej_ids, &run_tiles};
         for (auto* b : ibufs) b->release();
-        bs_errs.release();
-        bs_lvst.release();
+        bs_levels.release();
         enc_ctl.release();
         enc_tstep.release();
         enc_bpre.release();

@@ -286,6 +286,24 @@ __device__ __forceinline__ void store_event(MercuryEvent* dst, const MercuryEven
     for (int k = 0; k < 8; ++k) d[k] = s[k];
 }
 
+// Appends the record of an impact on the central body (entry time offset `temp`).
+__device__ __forceinline__ void central_record(MercuryEvent* events, int* event_step, int cap, DeviceStatus* st,
+                                               int id, double temp, double rcen, int step) {
+    const int slot = atomicAdd(&st->events, 1);
+    if (slot >= cap) {
+        atomicOr(&st->overflow, 1);
+        return;
+    }
+    MercuryEvent rec = {};
+    rec.i = 1;
+    rec.j = id;
+    rec.kind = EV_CENTRAL;
+    rec.time = temp;
+    rec.distance = rcen;
+    store_event(events + slot, rec);
+    event_step[slot] = step;
+}
+
 // The direct terms of a force on a test particle at x, sum of -m d/|d|^3 in
 // the order of the rows (the first four doubles of each: x, y, z, m), with the
 // statements of mfo_mvs and of mfo_grav, which multiply the same two factors.

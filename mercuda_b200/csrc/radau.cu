@@ -610,18 +610,30 @@ __global__ void __launch_bounds__(128) force_particle_kernel(ForceAllArgs A) {
 }
 
 // ---------------------------------------------------------------- screen
-__global__ void __launch_bounds__(256) screen_massive_kernel(ScreenArgs A) {
-    const int N = A.nsplit, nb = A.nbig - 1;
+// One launch: every block keeps the Big bodies' boxes and end states in shared
+// memory (SCREEN_BODIES at a time), a thread takes one particle through its
+// boxes, the exact test of the pairs whose boxes overlap (a few of a hundred
+// thousand) and the central body; the pairs within the massive set and its
+// bodies' own impacts are spread over the grid. The kernel moves 12 MB of L2
+// per 100,000 particles and is bounded by its launch and two dependent loads;
+// as four launches (boxes and massive pairs by one CTA, candidates, their exact
+// tests, impacts) it took 22 us of a step's serial chain, as one 8.
+constexpr int SCREEN_BODIES = 64;
+__global__ void __launch_bounds__(128) screen_kernel(ScreenArgs A) {
+    __shared__ double sbox[SCREEN_BODIES][4];
+    __shared__ double sdet[SCREEN_BODIES][14];   // x0, v0, x1, v1, rce, rphys
+    const int N = A.nsplit, nb = A.nbig - 1, S = A.npcap;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const double h = A.h, hm1 = 1.0 / h;
-    auto ends = [&](int k) {
-        return PairEnds{make_double3(A.b0[k], A.b0[N + k], A.b0[2 * N + k]),
-                        make_double3(A.b0[3 * N + k], A.b0[4 * N + k], A.b0[5 * N + k]),
-                        make_double3(A.b1[k], A.b1[N + k], A.b1[2 * N + k]),
-                        make_double3(A.b1[3 * N + k], A.b1[4 * N + k], A.b1[5 * N + k])};
+    auto ends_of = [](const double* r0, const double* r1, size_t L, size_t k) {
+        return PairEnds{make_double3(r0[k], r0[L + k], r0[2 * L + k]),
+                        make_double3(r0[3 * L + k], r0[4 * L + k], r0[5 * L + k]),
+                        make_double3(r1[k], r1[L + k], r1[2 * L + k]),
+                        make_double3(r1[3 * L + k], r1[4 * L + k], r1[5 * L + k])};
     };
-    auto box = [&](int k, double* bx) {
-        const PairEnds E = ends(k);
-        const double pad = A.rcebig[k] * 1.2;
+    // {lo x, hi x, lo y, hi y}, padded
+    auto box = [&](const PairEnds& E, double rce, double* bx) {
+        const double pad = rce * 1.2;
         double lo, hi;
         box_extent(E.x0.x, E.x1.x, E.v0.x, E.v1.x, h, lo, hi);
         bx[0] = lo - pad;
@@ -630,81 +642,81 @@ __global__ void __launch_bounds__(256) screen_massive_kernel(ScreenArgs A) {
         bx[2] = lo - pad;
         bx[3] = hi + pad;
     };
-    for (int k = 1 + threadIdx.x; k < A.nbig; k += blockDim.x) {
-        box(k, A.boxes + 4 * (k - 1));
-        const PairEnds E = ends(k);
-        double* d = A.detail + (size_t)(k - 1) * TAB_DETAIL;
-        const double3 q[4] = {E.x0, E.v0, E.x1, E.v1};
-        for (int w = 0; w < 4; ++w) {
-            d[3 * w] = q[w].x;
-            d[3 * w + 1] = q[w].y;
-            d[3 * w + 2] = q[w].z;
+    auto overlap = [](const double* a, const double* b) {
+        return a[1] >= b[0] && b[1] >= a[0] && a[3] >= b[2] && b[3] >= a[2];
+    };
+    auto record = [&](const PairEnds& I, const PairEnds& J, const PairClass& pc, int id_i, int id_j, bool swap) {
+        const int slot = atomicAdd(&A.status->events, 1);
+        if (slot < A.event_cap) {
+            pair_record(A.events + slot, I, J, pc, hm1, id_i, id_j, swap);
+            A.event_step[slot] = 0;
+        } else {
+            atomicOr(&A.status->overflow, 1);
         }
-        d[12] = A.rcebig[k];
-        d[13] = A.rphysbig[k];
-    }
-    // pairs within the massive set: i Big, i < j < nsplit
-    const int npair_max = nb * (N - 1);
-    for (int q = threadIdx.x; q < npair_max; q += blockDim.x) {
-        const int i = 1 + q / (N - 1), j = 1 + q % (N - 1);
-        if (j <= i) continue;
-        double bi[4], bj[4];
-        box(i, bi);
-        box(j, bj);
-        if (!(bi[1] >= bj[0] && bj[1] >= bi[0] && bi[3] >= bj[2] && bj[3] >= bi[2])) continue;
-        PairClass pc;
-        const PairEnds I = ends(i), J = ends(j);
-        if (pair_classify(I, J, A.rcebig[i], A.rcebig[j], A.rphysbig[i], A.rphysbig[j], h, pc)) {
-            const int slot = atomicAdd(&A.status->events, 1);
-            if (slot < A.event_cap) {
-                pair_record(A.events + slot, I, J, pc, hm1, i + 1, j + 1, A.mbig[j] > A.mbig[i] && j < A.nbig);
-                A.event_step[slot] = A.step;
-            } else {
-                atomicOr(&A.status->overflow, 1);
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(128) screen_particle_kernel(ScreenArgs A) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x, S = A.npcap, nb = A.nbig - 1;
+    };
+    auto central = [&](const PairEnds& E, double m, int id) {
+        double temp = 0.0;
+        if (central_impact(E.x0, E.v0, E.x1, E.v1, A.m0, m, h, A.rcen, temp))
+            central_record(A.events, A.event_step, A.event_cap, A.status, id, temp, A.rcen, 0);
+    };
     const bool ok = p < A.np;
-    double3 x0, v0, x1, v1;
-    double lo_x = 0, hi_x = 0, lo_y = 0, hi_y = 0, rce = 0, rphys = 0;
+    PairEnds J{};
+    double bp[4], rce = 0.0, rphys = 0.0, mj = 0.0;
     if (ok) {
-        x0 = make_double3(A.p0[p], A.p0[S + p], A.p0[2 * S + p]);
-        v0 = make_double3(A.p0[3 * S + p], A.p0[4 * S + p], A.p0[5 * S + p]);
-        x1 = make_double3(A.p1[p], A.p1[S + p], A.p1[2 * S + p]);
-        v1 = make_double3(A.p1[3 * S + p], A.p1[4 * S + p], A.p1[5 * S + p]);
+        J = ends_of(A.p0, A.p1, S, p);
+        mj = A.pconst[p];
         rce = A.pconst[S + p];
         rphys = A.pconst[2 * (size_t)S + p];
-        const double pad = rce * 1.2;
-        box_extent(x0.x, x1.x, v0.x, v1.x, A.h, lo_x, hi_x);
-        box_extent(x0.y, x1.y, v0.y, v1.y, A.h, lo_y, hi_y);
-        lo_x -= pad; hi_x += pad; lo_y -= pad; hi_y += pad;
+        box(J, rce, bp);
     }
-    for (int b = 0; b < nb; ++b) {
-        const double* bx = A.boxes + 4 * b;
-        const bool cand = ok && bx[1] >= lo_x && hi_x >= bx[0] && bx[3] >= lo_y && hi_y >= bx[2];
-        const unsigned mask = __ballot_sync(FULLMASK, cand);
-        if (!mask) continue;
-        const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
-        int base = 0;
-        if (lane == leader) base = atomicAdd(&A.status->cands, __popc(mask));
-        base = __shfl_sync(FULLMASK, base, leader);
-        if (!cand) continue;
-        const int slot = base + __popc(mask & ((1u << lane) - 1u));
-        if (slot >= A.cand_cap) {
-            atomicOr(&A.status->overflow, 2);
+    for (int b0 = 0; b0 < nb; b0 += SCREEN_BODIES) {
+        const int count = min(nb - b0, SCREEN_BODIES);
+        __syncthreads();
+        for (int k = threadIdx.x; k < count; k += blockDim.x) {
+            const int g = 1 + b0 + k;
+            const PairEnds E = ends_of(A.b0, A.b1, N, g);
+            box(E, A.rcebig[g], sbox[k]);
+            const double3 q[4] = {E.x0, E.v0, E.x1, E.v1};
+            for (int w = 0; w < 4; ++w) {
+                sdet[k][3 * w] = q[w].x;
+                sdet[k][3 * w + 1] = q[w].y;
+                sdet[k][3 * w + 2] = q[w].z;
+            }
+            sdet[k][12] = A.rcebig[g];
+            sdet[k][13] = A.rphysbig[g];
+        }
+        __syncthreads();
+        for (int k = 0; ok && k < count; ++k) {
+            if (!overlap(sbox[k], bp)) continue;
+            const double* d = sdet[k];
+            const PairEnds I{make_double3(d[0], d[1], d[2]), make_double3(d[3], d[4], d[5]),
+                             make_double3(d[6], d[7], d[8]), make_double3(d[9], d[10], d[11])};
+            PairClass pc;
+            if (pair_classify(I, J, d[12], rce, d[13], rphys, h, pc))
+                record(I, J, pc, b0 + k + 2, N + A.perm[p] + 1, false);
+        }
+    }
+    if (ok) central(J, mj, N + A.perm[p] + 1);
+    // the massive set: pairs of a Big body i and i < j < nsplit, then impacts
+    // (from the last block, which has no particles of its own)
+    const long long pairs = (long long)nb * (N - 1), stride = (long long)gridDim.x * blockDim.x;
+    const long long first = (long long)(gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
+    for (long long q = first; q < pairs + N - 1; q += stride) {
+        if (q >= pairs) {
+            const int k = 1 + (int)(q - pairs);
+            central(ends_of(A.b0, A.b1, N, k), A.mbig[k], k + 1);
             continue;
         }
-        EncounterCandidate* c = A.cands + slot;
-        c->slot = p; c->body = b; c->step = 0; c->id = A.nsplit + A.perm[p] + 1;
-        c->rce = rce; c->rphys = rphys;
-        c->x0[0] = x0.x; c->x0[1] = x0.y; c->x0[2] = x0.z;
-        c->v0[0] = v0.x; c->v0[1] = v0.y; c->v0[2] = v0.z;
-        c->x1[0] = x1.x; c->x1[1] = x1.y; c->x1[2] = x1.z;
-        c->v1[0] = v1.x; c->v1[1] = v1.y; c->v1[2] = v1.z;
+        const int i = 1 + (int)(q / (N - 1)), j = 1 + (int)(q % (N - 1));
+        if (j <= i) continue;
+        const PairEnds I = ends_of(A.b0, A.b1, N, i), K = ends_of(A.b0, A.b1, N, j);
+        double bi[4], bj[4];
+        box(I, A.rcebig[i], bi);
+        box(K, A.rcebig[j], bj);
+        if (!overlap(bi, bj)) continue;
+        PairClass pc;
+        if (pair_classify(I, K, A.rcebig[i], A.rcebig[j], A.rphysbig[i], A.rphysbig[j], h, pc))
+            record(I, K, pc, i + 1, j + 1, A.mbig[j] > A.mbig[i] && j < A.nbig);
     }
 }
 
@@ -748,8 +760,7 @@ void launch_force_all(const ForceAllArgs& a, cudaStream_t s) {
 }
 
 void launch_screen(const ScreenArgs& a, cudaStream_t s) {
-    screen_massive_kernel<<<1, 256, 0, s>>>(a);
-    if (a.np > 0 && a.nbig > 1) screen_particle_kernel<<<nblocks(a.np, 128), 128, 0, s>>>(a);
+    screen_kernel<<<nblocks(a.np, 128) + 1, 128, 0, s>>>(a);
 }
 
 }  // namespace mb200

@@ -65,12 +65,11 @@ struct ForceAllArgs {
 };
 void launch_force_all(const ForceAllArgs& a, cudaStream_t s);
 
-// Generic encounter screen between the states before (x0,v0) and after
-// (x1,v1) a step, for every pair (Big i, j > i): Big/massive pairs by one CTA,
-// particle pairs as candidates finished by the classify pass.
+// Both screens between the states before (x0, v0) and after (x1, v1) a step:
+// mce_stat for every pair (Big i, j > i) and mce_cent for every body.
 struct ScreenArgs {
     int nbig, nsplit, np, npcap;
-    double h;
+    double h, m0, rcen;
     const double* b0;      // [9][nsplit] previous buffer
     const double* b1;      // [9][nsplit] current buffer
     const double* mbig, *rcebig, *rphysbig;
@@ -78,15 +77,10 @@ struct ScreenArgs {
     const double* p1;
     const double* pconst;  // m, rce, rphys, ...
     const int* perm;
-    double* boxes;         // [nbig-1][4]
-    double* detail;        // [nbig-1][TAB_DETAIL]
     MercuryEvent* events;
     int* event_step;
     int event_cap;
-    EncounterCandidate* cands;
-    int cand_cap;
     DeviceStatus* status;
-    int step;              // event_step of this screen's records
 };
 void launch_screen(const ScreenArgs& a, cudaStream_t s);
 
