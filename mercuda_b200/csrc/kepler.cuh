@@ -313,8 +313,10 @@ __device__ __forceinline__ bool drift_near(double mu, double rmu, double3& p, do
 // (1.6 % at the start of the 1M-particle workload, 5 % after 4,600 steps), but
 // a warp of them takes several times an ordinary warp's time and, started
 // first, still ends a launch of 16 to 31 steps last: what counts here is the
-// length of the chain. False where drift_kepmd applies, an operand is out of
-// range or Laguerre's iteration fails: drift_dan then decides.
+// length of the chain. Undecided (state untouched) where drift_kepmd applies or
+// an operand is out of range: drift_dan then decides. Failed, as drift_dan would
+// be with the same iterates, where Laguerre's 401 passes do not converge.
+enum : int { DRIFT_FAILED = -1, DRIFT_UNDECIDED = 0, DRIFT_DONE = 1 };
 // stumpff with the number of quarterings taken from the exponent (|x| 4^-n is
 // exact either way), for |x| below 2^200.
 __device__ __forceinline__ void stumpff_near(double x, double& c0, double& c1, double& c2, double& c3) {
@@ -344,17 +346,17 @@ __device__ __forceinline__ void stumpff_near(double x, double& c0, double& c1, d
         c0 = 2.0 * c0 * c0 - 1.0;
     }
 }
-__device__ __forceinline__ bool drift_universal(double mu, double3& p, double3& w, double dt) {
+__device__ __forceinline__ int drift_universal(double mu, double3& p, double3& w, double dt) {
     const double rr = p.x * p.x + p.y * p.y + p.z * p.z;
     double r0, yr;
     sqrt_recip(rr, r0, yr);
     const double v0s = w.x * w.x + w.y * w.y + w.z * w.z;
     const double u = p.x * w.x + p.y * w.y + p.z * w.z;
     const double alpha = quotient(2.0 * mu, r0, yr) - v0s;
-    if (!(narrow_range(rr) && narrow_range(mu))) return false;
+    if (!(narrow_range(rr) && narrow_range(mu))) return DRIFT_UNDECIDED;
     double s;
     if (alpha > 0.0) {
-        if (!narrow_range(alpha)) return false;
+        if (!narrow_range(alpha)) return DRIFT_UNDECIDED;
         const double a = quotient(mu, alpha, recip_near(alpha));
         const double asq = a * a;
         const double acu = a * asq;
@@ -367,7 +369,7 @@ __device__ __forceinline__ bool drift_universal(double mu, double3& p, double3& 
         const double turn = dt * en;
         const double dm = turn - double(int(quotient(turn, TWOPI_SWIFT, 1.0 / TWOPI_SWIFT))) * TWOPI_SWIFT;
         dt = quotient(dm, en, yen);
-        if (!((dm * dm > 0.16) || (esq > 0.36)) && esq * dm * dm < 0.0016) return false;
+        if (!((dm * dm > 0.16) || (esq > 0.36)) && esq * dm * dm < 0.0016) return DRIFT_UNDECIDED;
         const double lead = quotient(dt, r0, yr);
         if (lead <= 0.4) {
             const double d = 2.0 * r0 * r0 * r0;
@@ -377,7 +379,7 @@ __device__ __forceinline__ bool drift_universal(double mu, double3& p, double3& 
             const double esg = quotient(u, d, recip_near(d));
             double y = en * dt - esg, e, ye;
             const double e2 = ec * ec + esg * esg;
-            if (!mid_range(e2)) return false;
+            if (!mid_range(e2)) return DRIFT_UNDECIDED;
             sqrt_near(e2, e, ye);
             // mco_sine (fmod leaves an angle within one turn as it is)
             const double pi = 3.141592653589793, twopi = 2.0 * pi;
@@ -395,7 +397,7 @@ __device__ __forceinline__ bool drift_universal(double mu, double3& p, double3& 
         // NaN comes here too and fails below
         if (!kepu_cubic_seed(dt, r0, mu, alpha, u, s)) s = quotient(dt, r0, yr);
     }
-    if (!mid_magnitude(dt)) return false;
+    if (!mid_magnitude(dt)) return DRIFT_UNDECIDED;
     const double ydt = recip_near(dt), tol = DANBYB * DANBYB;
     double fp = 0.0, c0, c1 = 0.0, c2 = 0.0, c3 = 0.0;
     const double st = s, mra = mu - r0 * alpha;
@@ -419,7 +421,7 @@ __device__ __forceinline__ bool drift_universal(double mu, double3& p, double3& 
         ds = -quotient(f, d3, recip_near(d3));
         // z below 2^200, divisors and numerators of moderate size
         if (!(fabs(z) < 1e60 && fabs(f) < 1e60 && mid_magnitude(fp) && mid_magnitude(d2) && mid_magnitude(d3)))
-            return false;
+            return DRIFT_UNDECIDED;
         s = s + ds;
         const double fdt = quotient(f, dt, ydt);
         done = fdt * fdt < tol;
@@ -444,14 +446,14 @@ __device__ __forceinline__ bool drift_universal(double mu, double3& p, double3& 
             double sq, ysq;
             sqrt_near(q, sq, ysq);
             const double d = fp + copysign(1.0, fp) * sq;
-            if (!(fabs(z) < 1e60 && fabs(f) < 1e60 && mid_range(q) && mid_magnitude(d))) return false;
+            if (!(fabs(z) < 1e60 && fabs(f) < 1e60 && mid_range(q) && mid_magnitude(d))) return DRIFT_UNDECIDED;
             s = s - quotient(ln * f, d, recip_near(d));
             const double fdt = quotient(f, dt, ydt);
             done = fdt * fdt < tol;
         }
-        if (!done) return false;
+        if (!done) return DRIFT_FAILED;
     }
-    if (!mid_magnitude(fp)) return false;
+    if (!mid_magnitude(fp)) return DRIFT_UNDECIDED;
     const double yfp = recip_near(fp);
     const double d = fp * r0;
     const double f = 1.0 - quotient(mu, r0, yr) * c2;
@@ -462,34 +464,39 @@ __device__ __forceinline__ bool drift_universal(double mu, double3& p, double3& 
     const double3 w1 = make_double3(p.x * fdot + w.x * gdot, p.y * fdot + w.y * gdot, p.z * fdot + w.z * gdot);
     p = p1;
     w = w1;
-    return true;
+    return DRIFT_DONE;
 }
 
 // drift_one: the drift, else ten substeps of dt/10 (stopping at a failed one).
 // The flag is discarded by all MVS/HYBRID callers (mdt_mvs, mdt_hy, mco_mvs2h).
-// Written as one loop so that drift_dan is instantiated once: attempt 0 is the
-// whole step, attempts 1..10 the substeps.
+// Written as one loop so that each solver is there once: attempt 0 is the whole
+// step, attempts 1..10 the substeps. An orbit whose solves fail takes up to
+// eleven rounds of 401 passes in every step, alone: one such among 1M particles
+// made a run of 457 steps take 458 ms with drift_dan for every round behind a
+// failed first one, 161 as here (runs without such an orbit 32 to 38).
 struct DriftState {
     double3 p, w;
+    int done;
 };
 static __device__ __noinline__ DriftState drift_plain(double mu, DriftState z, double dt) {
-    const double sub = dt / 10.0;
-#pragma unroll 1
-    for (int attempt = 0; attempt <= 10; ++attempt) {
-        const bool ok = drift_dan(mu, z.p, z.w, attempt == 0 ? dt : sub);
-        if (attempt == 0 ? ok : !ok) break;
-    }
+    z.done = drift_dan(mu, z.p, z.w, dt) ? DRIFT_DONE : DRIFT_FAILED;
     return z;
 }
 static __device__ __noinline__ DriftState drift_general(double mu, DriftState z, double dt) {
-    if (drift_universal(mu, z.p, z.w, dt)) return z;
-    return drift_plain(mu, z, dt);
+#pragma unroll 1
+    for (int attempt = 0; attempt <= 10; ++attempt) {
+        z.done = drift_universal(mu, z.p, z.w, dt);
+        if (z.done == DRIFT_UNDECIDED) z = drift_plain(mu, z, dt);
+        if (attempt == 0) dt = dt / 10.0;
+        if ((z.done == DRIFT_DONE) == (attempt == 0)) break;
+    }
+    return z;
 }
 // With rr = |p|^2 at hand and rmu ~ 1/mu. The general solver is a call, so
 // that its registers do not count against the straight-line path.
 __device__ __forceinline__ void drift_one(double mu, double rmu, double3& p, double3& w, double dt, double rr) {
     if (drift_near(mu, rmu, p, w, dt, rr)) return;
-    const DriftState z = drift_general(mu, DriftState{p, w}, dt);
+    const DriftState z = drift_general(mu, DriftState{p, w, 0}, dt);
     p = z.p;
     w = z.w;
 }
