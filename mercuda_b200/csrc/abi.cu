@@ -2556,7 +2556,7 @@ int mercury_b200_mvs_advance(double time, double h, int nsteps, double rcen, int
         const int nb = c.nbig - 1;
         int K = steps_per_launch > 0 ? steps_per_launch : (c.steps_per_launch > 0 ? c.steps_per_launch : 0);
         const bool auto_K = K <= 0;
-        if (K <= 0) K = mvs_max_steps_per_launch(nb);
+        if (K <= 0) K = mvs_usual_steps_per_launch(nb);
         K = std::min(K, mvs_max_steps_per_launch(nb));
         K = std::max(1, std::min(K, nsteps));
         // launch sizes: K steps each; with the automatic choice the first launch

@@ -1225,19 +1225,26 @@ size_t mvs_particle_smem(int nb, int nsteps, int reset, int threads, bool ngf) {
                              (size_t)Cols::STRIDE * Cols::count(ngf));
 }
 
-// Steps fused per launch: 18 KB of tables in global memory (24 steps of eight
-// planets; what a CTA stages of them is 11 KB). Fewer launches re-order the
-// slots and wait for their slowest tile less often, more sort particles that
-// change path sooner. 457 steps of 1M particles take 30.0 ms with 16 steps a
-// launch, 28.7 with 24 to 31, 29.0 with 40; of 10k 0.72, 0.71 to 0.75 and 0.80.
-int mvs_max_steps_per_launch(int nb) {
-    const size_t budget = 18 * 1024;
-    const size_t row = sizeof(double) * (size_t)tab_stride(nb);
-    long k = (long)(budget / row) - 1;
-    if (k < 1) k = 1;
-    if (k > 64) k = 64;
-    return (int)k;
+namespace {
+// Rows of 18 KB less the one for a fresh start's force, 1 to 64.
+int steps_of_rows(int row_doubles) {
+    const int k = (int)(18 * 1024 / (sizeof(double) * (size_t)row_doubles)) - 1;
+    return k < 1 ? 1 : k > 64 ? 64 : k;
 }
+}  // namespace
+
+// The most steps a launch takes: as many as there are rows {head, 8 doubles a
+// body} in 18 KB, whatever else a table row holds: 31 steps of eight planets, 56
+// of four (a CTA stages 14 KB of them).
+int mvs_max_steps_per_launch(int nb) { return steps_of_rows(TAB_HEAD + TAB_BODY * nb); }
+
+// The steps of a launch where the caller leaves it open: 18 KB of whole table
+// rows, 25 steps of eight planets, 47 of four. Fewer launches re-order the slots
+// and wait for their slowest tile less often, more sort particles that change
+// path sooner. 457 steps of 1M particles take 30.0 ms with 16 steps a launch,
+// 28.7 with 24 to 31, 29.0 with 40; a whole pass of 46 steps of 10,000 takes
+// 0.81 ms with 25 (launches of 5, 25 and 16) and 0.84 with 31 (7, 31 and 8).
+int mvs_usual_steps_per_launch(int nb) { return steps_of_rows(tab_stride(nb)); }
 
 void launch_mvs_corrector(const MvsBigArgs& big, const CorrectorArgs& a, cudaStream_t s) {
     const int N = big.nmass > big.nbig ? big.nmass : big.nbig;

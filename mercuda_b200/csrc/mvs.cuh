@@ -200,5 +200,6 @@ void launch_mvs_big(const MvsBigArgs& a, cudaStream_t s);
 void launch_mvs_particles(const MvsParticleArgs& a, cudaStream_t s, int threads);
 size_t mvs_particle_smem(int nb, int nsteps, int reset, int threads, bool ngf);
 int mvs_max_steps_per_launch(int nb);
+int mvs_usual_steps_per_launch(int nb);
 
 }  // namespace mb200
