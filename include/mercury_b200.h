@@ -195,10 +195,12 @@ void mercury_b200_batch_free(void);
  * arrays: x0/v0 (np,3) rows, yar[np] or NULL for none) advance nsteps MVS
  * steps of h, exactly as the MVS path steps them; the final states go to the
  * device arrays x_final/v_final (np,3). The state every checkpoint_every
- * steps is kept for the backward call (9 doubles per particle per
- * checkpoint, plus 12 per particle per step of one segment). The device
- * inputs must stay unchanged until the backward call. No oblateness and no
- * non-gravitational term other than yar. */
+ * steps is kept for the backward call (9 doubles and an int per particle per
+ * checkpoint, plus 12 doubles per particle per step of two segments; of four,
+ * where a segment's take at most 1 GiB and the third and fourth at most a
+ * quarter of the device's free memory). The device inputs must stay unchanged
+ * until the backward call. No oblateness and no non-gravitational term other
+ * than yar. */
 int mercury_b200_adjoint_forward(int nbig, const double* mbig, const double* xbig, const double* vbig, int np,
                                  const double* x0, const double* v0, const double* yar, double h, int nsteps,
                                  int checkpoint_every, double* x_final, double* v_final);

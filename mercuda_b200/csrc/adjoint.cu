@@ -313,8 +313,9 @@ struct Adjoint {
     // Record buffers: a recomputation ends with its slowest particle's serial
     // steps, but segments can be recomputed side by side from their
     // checkpoints: up to three run ahead of the walk (one, where a buffer takes
-    // more than REC_BYTES). 100,000 particles, 20 segments of 50 steps:
-    // backward 17.7 ms with one ahead, 12.2 with three.
+    // more than REC_BYTES or the third and fourth would take more than a quarter
+    // of the free memory). 100,000 particles, 20 segments of 50 steps: backward
+    // 17.7 ms with one ahead, 12.2 with three.
     static constexpr int MAX_REC = 4;
     static constexpr size_t REC_BYTES = (size_t)1 << 30;
     int nrec = 2;
@@ -412,22 +413,46 @@ int mercury_b200_adjoint_forward(int nbig, const double* mbig, const double* xbi
         J.yar = yar;
         J.has_yar = yar != nullptr;
         const int nb = nbig - 1, nseg = (nsteps + J.K - 1) / J.K;
-        for (int k = 0; k < 2; ++k) J.bigstate[k].reserve((size_t)9 * nbig);
-        J.mbig.reserve(nbig);
-        J.zeros.reserve(nbig);
-        J.tab.reserve((size_t)(nsteps + 1) * tab_stride(nb));
-        J.detail.reserve((size_t)nsteps * std::max(1, nb) * TAB_DETAIL);
-        J.ckpt.reserve((size_t)nseg * 9 * np);
         const size_t rec_el = (size_t)J.K * REC * np;
-        J.nrec = std::min(nseg, sizeof(double) * rec_el > Adjoint::REC_BYTES ? 2 : Adjoint::MAX_REC);
-        for (int k = 0; k < J.nrec; ++k) J.rec[k].reserve(rec_el);
+        auto reserve = [&] {
+            for (int k = 0; k < 2; ++k) J.bigstate[k].reserve((size_t)9 * nbig);
+            J.mbig.reserve(nbig);
+            J.zeros.reserve(nbig);
+            J.tab.reserve((size_t)(nsteps + 1) * tab_stride(nb));
+            J.detail.reserve((size_t)nsteps * std::max(1, nb) * TAB_DETAIL);
+            J.ckpt.reserve((size_t)nseg * 9 * np);
+            for (int k = 0; k < std::min(nseg, 2); ++k) J.rec[k].reserve(rec_el);
+            J.lam.reserve((size_t)10 * np);
+            J.events.reserve(4096);
+            J.event_step.reserve(4096);
+            J.status.reserve(1);
+            J.perm.reserve((size_t)nseg * np);
+            J.nslow.reserve((size_t)2 * nseg);
+        };
+        // two record buffers are what a run needs; more of them, an earlier
+        // run's or this one's, only where there is room
+        try {
+            reserve();
+        } catch (const CudaError&) {
+            cudaGetLastError();
+            for (int k = 2; k < Adjoint::MAX_REC; ++k) J.rec[k].release();
+            reserve();
+        }
+        J.nrec = std::min(nseg, 2);
+        if (sizeof(double) * rec_el <= Adjoint::REC_BYTES && nseg > 2) {
+            const int want = std::min(nseg, Adjoint::MAX_REC);
+            size_t more = 0, free_b = 0, total_b = 0;
+            for (int k = 2; k < want; ++k)
+                if (J.rec[k].n < rec_el) more += sizeof(double) * rec_el;
+            if (more == 0 || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && more <= free_b / 4)) {
+                try {
+                    for (; J.nrec < want; ++J.nrec) J.rec[J.nrec].reserve(rec_el);
+                } catch (const CudaError&) {
+                    cudaGetLastError();
+                }
+            }
+        }
         J.ensure_events(nseg);
-        J.lam.reserve((size_t)10 * np);
-        J.events.reserve(4096);
-        J.event_step.reserve(4096);
-        J.status.reserve(1);
-        J.perm.reserve((size_t)nseg * np);
-        J.nslow.reserve((size_t)2 * nseg);
         // Big bodies: SoA [9][nbig] from the host rows, a(3) zero (reset)
         std::vector<double> b(9 * (size_t)nbig, 0.0);
         for (int k = 0; k < nbig; ++k)
