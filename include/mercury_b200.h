@@ -158,7 +158,9 @@ int mercury_b200_fp64_peak(double* tflops, double* ms);
  * (n,3) rows, rce/rphys per body), its central body first, then nbig[s]-1 Big
  * bodies, then massless Small bodies; h[s] is its step. No non-gravitational
  * forces, no oblateness; nbig[s] <= 32. The upload replaces any previous
- * batch and resets every system's cached acceleration. */
+ * batch and resets every system's cached acceleration; the previous batch's
+ * device buffers are kept for one of about its size
+ * (mercury_b200_batch_free gives them back). */
 int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig, const double* h,
                               const double* m, const double* x, const double* v, const double* rce,
                               const double* rphys);

@@ -41,13 +41,14 @@ struct Batch {
     DBuf<double> prce, prphys;
     DBuf<int> plocal;
     DBuf<double> tab[2], det[2];
-    DBuf<double> stage;              // the host arrays as they are: x, v (3 a body), m, rce, rphys
     size_t tab_size = 0, det_size = 0;
     DBuf<MercuryEvent> events;
     DBuf<int> event_step, event_sys;
     DBuf<EncounterCandidate> cands;
     DBuf<DeviceStatus> status;
     DeviceStatus* status_host = nullptr;
+    // the run's starting state; between runs the host arrays' rows as they are
+    // (x, v, 3 a body, m, rce, rphys: the same size)
     DBuf<double> snap;
     int cur = 0;
     bool reset = true;
@@ -67,8 +68,15 @@ struct Batch {
     std::vector<int> host_sys, host_step;
 
     void release() {
+        release_buffers();
+        nsys = nbody = npcap = ntiles = 0;
+        host_events.clear();
+        host_sys.clear();
+        host_step.clear();
+    }
+    void release_buffers() {
         DBuf<double>* d[] = {&bigbuf[0], &bigbuf[1], &bm, &brce, &brphys, &pstate[0], &pstate[1],
-                             &prce, &prphys, &tab[0], &tab[1], &det[0], &det[1], &snap, &stage};
+                             &prce, &prphys, &tab[0], &tab[1], &det[0], &det[1], &snap};
         for (auto* b : d) b->release();
         d_sys.release();
         d_body_end.release();
@@ -81,11 +89,31 @@ struct Batch {
         cands.release();
         status.release();
         drop_graph();
-        nsys = nbody = npcap = ntiles = 0;
-        host_events.clear();
-        host_sys.clear();
-        host_step.clear();
         ++epoch;
+    }
+    int record_cap() const { return (int)std::min({events.n, event_step.n, event_sys.n}); }
+    // Room for that many records and candidates; what there was where it
+    // cannot be had (the records' three arrays are always of one size).
+    void room_for(size_t records, size_t candidates) {
+        const size_t r0 = events.n, c0 = cands.n;
+        auto reserve = [&](size_t r, size_t c) {
+            events.reserve(r);
+            event_step.reserve(r);
+            event_sys.reserve(r);
+            cands.reserve(c);
+        };
+        ++epoch;
+        try {
+            reserve(std::max(records, r0), candidates);
+        } catch (const CudaError&) {
+            cudaGetLastError();
+            events.release();
+            event_step.release();
+            event_sys.release();
+            cands.release();
+            reserve(r0, c0);
+            throw;
+        }
     }
     void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -125,6 +153,7 @@ constexpr int BATCH_CHUNK = 1024;
 struct BatchRows {
     const BatchSys* sys;
     const int* body_end;      // first row past each system
+    int row0;                 // the first system's first row
     double *x, *v;            // rows, 3 a body
     const double *m, *rce, *rphys;
     double* big;
@@ -138,7 +167,7 @@ template <bool GATHER> __global__ void __launch_bounds__(128) batch_rows_kernel(
     const int n = A.body_end[blockIdx.x] - S.body;
     const int j1 = min(n, (int)(blockIdx.y + 1) * BATCH_CHUNK);
     for (int j = blockIdx.y * BATCH_CHUNK + threadIdx.x; j < j1; j += blockDim.x) {
-        const size_t row = S.body + j;
+        const size_t row = (size_t)(S.body - A.row0) + j;
         double* x = A.x + 3 * row;
         double* v = A.v + 3 * row;
         const bool is_big = j < S.nbig;
@@ -168,11 +197,12 @@ template <bool GATHER> __global__ void __launch_bounds__(128) batch_rows_kernel(
     }
 }
 template <bool GATHER> void launch_batch_rows(Batch& B) {
-    const size_t n = B.nbody;
+    const size_t n = B.nbody - B.body_off[0];
     BatchRows a{};
     a.sys = B.d_sys.p;
     a.body_end = B.d_body_end.p;
-    a.x = B.stage.p;
+    a.row0 = B.body_off[0];
+    a.x = B.snap.p;
     a.v = a.x + 3 * n;
     a.m = a.v + 3 * n;
     a.rce = a.m + n;
@@ -205,11 +235,24 @@ void layout_tables(Batch& B, int K) {
     if (t > (size_t)INT32_MAX || d > (size_t)INT32_MAX) throw std::runtime_error("batched tables too large");
     B.tab_size = t;
     B.det_size = d;
-    for (int k = 0; k < 2; ++k) {
-        const size_t n0 = B.tab[k].n, n1 = B.det[k].n;
-        B.tab[k].reserve(t);
-        B.det[k].reserve(d);
-        if (B.tab[k].n != n0 || B.det[k].n != n1) ++B.epoch;
+    auto reserve = [&] {
+        for (int k = 0; k < 2; ++k) {
+            if (t > B.tab[k].n || d > B.det[k].n) ++B.epoch;
+            B.tab[k].reserve(t);
+            B.det[k].reserve(d);
+        }
+    };
+    try {
+        reserve();
+    } catch (const CudaError&) {
+        // the room for candidates may be an earlier run's guess
+        cudaGetLastError();
+        const size_t least = std::max(16384, B.npcap / 2);
+        if (B.cands.n <= least) throw;
+        B.cands.release();
+        ++B.epoch;
+        B.cands.reserve(least);
+        reserve();
     }
     B.K = K;
     h2d(B.d_sys.p, B.sys.data(), sizeof(BatchSys) * B.nsys, B.stream);
@@ -230,7 +273,7 @@ BatchBigArgs big_chunk(Batch& B, int ch, int ks, int reset, int central, int s0,
     a.events = B.events.p;
     a.event_step = B.event_step.p;
     a.event_sys = B.event_sys.p;
-    a.event_cap = (int)B.events.n;
+    a.event_cap = B.record_cap();
     a.status = B.status.p;
     return a;
 }
@@ -257,7 +300,7 @@ BatchParticleArgs particle_chunk(Batch& B, int ch, int ks, int reset, int centra
     a.events = B.events.p;
     a.event_step = B.event_step.p;
     a.event_sys = B.event_sys.p;
-    a.event_cap = (int)B.events.n;
+    a.event_cap = B.record_cap();
     a.cands = B.cands.p;
     a.cand_cap = (int)B.cands.n;
     a.status = B.status.p;
@@ -379,18 +422,22 @@ void sort_batch_events(Batch& B) {
 
 // Room for a run's records and one chunk's candidates, so that a run need not
 // be made again: the package's workloads give up to 8 records and 400
-// candidates per 10,000 particle-steps (the first is capped at 4M records;
-// an overflow still grows the buffers and redoes the run).
+// candidates per 10,000 particle-steps. Only a guess (the records are capped at
+// 4M), so made out of a quarter of the free memory or not at all: an overflow
+// still grows the buffers and redoes the run.
 void size_records(Batch& B, int nsteps, int K) {
     const long long slots = B.npcap;
     const size_t records = (size_t)std::min<long long>(4 << 20, slots * nsteps / 1000);
     const size_t cands = (size_t)std::min<long long>(INT32_MAX / 2, slots * K / 25);
-    if (records > B.events.n || cands > B.cands.n) {
-        B.events.reserve(records);
-        B.event_step.reserve(B.events.n);
-        B.event_sys.reserve(B.events.n);
-        B.cands.reserve(cands);
-        ++B.epoch;
+    if (records <= B.events.n && cands <= B.cands.n) return;
+    size_t more = 0, free_b = 0, total_b = 0;
+    if (records > B.events.n) more += records * (sizeof(MercuryEvent) + 2 * sizeof(int));
+    if (cands > B.cands.n) more += cands * sizeof(EncounterCandidate);
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || more > free_b / 4) return;
+    try {
+        B.room_for(records, cands);
+    } catch (const CudaError&) {
+        cudaGetLastError();
     }
 }
 
@@ -407,8 +454,8 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
     try {
         if (nsys < 1) throw std::runtime_error("batch needs at least one system");
         B.ensure_streams();
-        // the buffers of an earlier batch stay (batch_free gives them back);
-        // its graph, records and sizes do not
+        // the buffers of an earlier batch may stay (below); its graph, records
+        // and sizes do not
         B.drop_graph();
         B.host_events.clear();
         B.host_sys.clear();
@@ -457,33 +504,47 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
         B.npcap = std::max(1, slots);
         B.ntiles = (int)tiles.size();
         B.nbigs = bigs;
-        B.d_sys.reserve(nsys);
-        B.d_tiles.reserve(std::max(1, B.ntiles));
-        B.d_proto.reserve(nsys);
-        for (int k = 0; k < 2; ++k) {
-            B.bigbuf[k].reserve((size_t)9 * bigs);
-            B.pstate[k].reserve((size_t)9 * B.npcap);
+        auto reserve = [&] {
+            B.d_sys.reserve(nsys);
+            B.d_tiles.reserve(std::max(1, B.ntiles));
+            B.d_proto.reserve(nsys);
+            for (int k = 0; k < 2; ++k) {
+                B.bigbuf[k].reserve((size_t)9 * bigs);
+                B.pstate[k].reserve((size_t)9 * B.npcap);
+            }
+            B.bm.reserve(bigs);
+            B.brce.reserve(bigs);
+            B.brphys.reserve(bigs);
+            B.prce.reserve(B.npcap);
+            B.prphys.reserve(B.npcap);
+            B.plocal.reserve(B.npcap);
+            B.room_for(std::max(4096, B.npcap / 64), std::max(16384, B.npcap / 2));
+            B.status.reserve(1);
+            B.snap.reserve((size_t)9 * B.npcap + (size_t)9 * bigs);
+            B.d_body_end.reserve(nsys);
+            layout_tables(B, B.forced_K > 0 ? B.forced_K : 31);   // copies the systems' records
+        };
+        // An earlier batch's buffers stay for one of about its size (until
+        // batch_free, or until room is short): programs upload batch after batch,
+        // and allocating some hundred MB takes as long as copying them
+        const size_t spare = (size_t)1 << 20;
+        if (B.pstate[0].n > (size_t)9 * B.npcap / 4 * 5 + spare || B.bigbuf[0].n > (size_t)9 * bigs / 4 * 5 + spare)
+            B.release_buffers();
+        B.nsys = nsys;
+        try {
+            reserve();
+        } catch (const CudaError&) {
+            cudaGetLastError();
+            B.release_buffers();
+            reserve();
         }
-        B.bm.reserve(bigs);
-        B.brce.reserve(bigs);
-        B.brphys.reserve(bigs);
-        B.prce.reserve(B.npcap);
-        B.prphys.reserve(B.npcap);
-        B.plocal.reserve(B.npcap);
-        B.events.reserve(std::max(4096, slots / 64));
-        B.event_step.reserve(B.events.n);
-        B.event_sys.reserve(B.events.n);
-        B.cands.reserve(std::max(16384, slots / 2));
-        B.status.reserve(1);
-        B.snap.reserve((size_t)9 * B.npcap + (size_t)9 * bigs);
         // every host array in one round of copies; layout on the device
-        const size_t n = B.nbody;
-        B.stage.reserve(9 * n);
-        B.d_body_end.reserve(nsys);
+        const size_t o = B.body_off[0], n = B.nbody - o;
+        auto rows = [&](size_t at, const double* a, size_t width) {
+            return HostSpan{B.snap.p + at * n, const_cast<double*>(a) + width * o, sizeof(double) * width * n};
+        };
         std::vector<HostSpan> spans = {
-            {B.stage.p, const_cast<double*>(xx), 24 * n},        {B.stage.p + 3 * n, const_cast<double*>(vv), 24 * n},
-            {B.stage.p + 6 * n, const_cast<double*>(m), 8 * n},  {B.stage.p + 7 * n, const_cast<double*>(rce), 8 * n},
-            {B.stage.p + 8 * n, const_cast<double*>(rphys), 8 * n},
+            rows(0, xx, 3), rows(3, vv, 3), rows(6, m, 1), rows(7, rce, 1), rows(8, rphys, 1),
             {B.d_body_end.p, B.body_off.data() + 1, sizeof(int) * nsys}};
         if (B.ntiles) spans.push_back({B.d_tiles.p, tiles.data(), sizeof(BatchTile) * B.ntiles});
         copy_in(spans, B.stream);
@@ -506,9 +567,7 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
             }
         }
         h2d(B.d_proto.p, proto.data(), sizeof(MvsBigArgs) * nsys, B.stream);
-        B.nsys = nsys;
         B.cur = 0;
-        layout_tables(B, B.forced_K > 0 ? B.forced_K : 31);   // copies the systems' records
         launch_batch_rows<false>(B);
         check(cudaMemsetAsync(B.bigbuf[1].p, 0, sizeof(double) * 9 * bigs, B.stream), "upload");
         check(cudaMemsetAsync(B.pstate[1].p, 0, sizeof(double) * 9 * B.npcap, B.stream), "upload");
@@ -519,6 +578,7 @@ int mercury_b200_batch_upload(int nsys, const int* body_offset, const int* nbig,
         B.tuned_threads = 128;
         return 0;
     } catch (const std::exception& e) {
+        B.nsys = 0;
         return report(e);
     }
 }
@@ -570,16 +630,11 @@ int mercury_b200_batch_advance(double time, int nsteps, double rcen, int* nevent
             if (B.status_host->fault) throw std::runtime_error("MVS force failed");
             if (!B.status_host->overflow) break;
             if (attempt > 8) throw std::runtime_error("event buffer growth failed");
-            if (B.status_host->overflow & 1) {
-                const size_t n = std::max(2 * B.events.n, (size_t)B.status_host->events + 1024);
-                B.events.reserve(n);
-                B.event_step.reserve(n);
-                B.event_sys.reserve(n);
-            }
-            if (B.status_host->overflow & 2) B.cands.reserve(2 * B.cands.n + 4096);
-            ++B.epoch;
             copy(B.pstate[B.cur].p, B.snap.p, sizeof(double) * 9 * B.npcap);
             copy(B.bigbuf[B.cur].p, B.snap.p + 9 * (size_t)B.npcap, sizeof(double) * 9 * bigs);
+            const int over = B.status_host->overflow;
+            B.room_for(over & 1 ? std::max(2 * B.events.n, (size_t)B.status_host->events + 1024) : 0,
+                       over & 2 ? 2 * B.cands.n + 4096 : 0);
         }
         check(cudaEventElapsedTime(&B.last_ms, B.t0, B.t1), "timer");
         B.last_launches = launches;
@@ -637,11 +692,9 @@ int mercury_b200_batch_download(double* xx, double* vv) {
     Batch& B = batch();
     try {
         if (B.nsys < 1) throw std::runtime_error("no batch uploaded");
-        const size_t n = B.nbody;
+        const size_t o = B.body_off[0], n = B.nbody - o;   // rows before the first system are not the batch's
         launch_batch_rows<true>(B);
-        const size_t o = B.body_off[0];   // rows before the first system are not the batch's
-        copy_out({{B.stage.p + 3 * o, xx + 3 * o, 24 * (n - o)}, {B.stage.p + 3 * (n + o), vv + 3 * o, 24 * (n - o)}},
-                 B.stream);
+        copy_out({{B.snap.p, xx + 3 * o, 24 * n}, {B.snap.p + 3 * n, vv + 3 * o, 24 * n}}, B.stream);
         return 0;
     } catch (const std::exception& e) {
         return report(e);

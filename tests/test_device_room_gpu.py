@@ -3,10 +3,12 @@ is not asked for, and the results do not depend on it. The sizes below leave
 each call what it must have, and a quarter of that on top."""
 import contextlib
 
+import numpy as np
 import pytest
 import torch
 
 from mercuda_b200.adjoint import mvs_trajectory
+from mercuda_b200.backend import Batch
 from mercuda_b200.system import make_system
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +51,35 @@ def test_adjoint_record_buffers(cuda_lib):
     with little_room(cuda_lib, int(1.25 * needs)):
         tight = run()
     assert all(torch.equal(a, b) for a, b in zip(roomy, tight))
+
+
+def batch_run(systems, nsteps):
+    b = Batch(systems, np.full(len(systems), 8.0))
+    b.set(threads=128, steps_per_launch=64)
+    ev, sy, st = b.advance(0.0, nsteps, 0.005)
+    return ev.tobytes(), sy.tolist(), st.tolist(), b.download()
+
+
+def test_batch_candidates(cuda_lib):
+    """A million particles in four systems, 64 steps a launch: 302 bytes a
+    particle is what an upload asks for, 2.56 candidates a particle (328 bytes)
+    only a guess that saves making a run twice."""
+    systems = [make_system(seed=20 + k, n_particles=250_000, nplanets=1) for k in range(4)]
+    roomy = batch_run(systems, 64)
+    with little_room(cuda_lib, int(1.25 * 302 * 1_000_000)):
+        tight = batch_run(systems, 64)
+        cuda_lib.mercury_b200_batch_free()
+    cuda_lib.mercury_b200_batch_set(0, 0, -1)
+    assert roomy[:3] == tight[:3]
+    assert all(np.array_equal(p, q) for a, c in zip(roomy[3], tight[3]) for p, q in zip(a, c))
+
+
+def test_large_batch_gives_way_to_a_small_one(cuda_lib):
+    little = [make_system(seed=5, n_particles=1000, nplanets=1)]
+    Batch(little, np.full(1, 8.0)).free()
+    free0 = torch.cuda.mem_get_info()[0]
+    Batch([make_system(seed=6, n_particles=500_000, nplanets=1)], np.full(1, 8.0))
+    assert free0 - torch.cuda.mem_get_info()[0] > 500_000 * 302
+    b = Batch(little, np.full(1, 8.0))
+    assert free0 - torch.cuda.mem_get_info()[0] < 32 << 20
+    b.free()
