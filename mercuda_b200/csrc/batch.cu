@@ -146,14 +146,15 @@ Batch& batch() {
 }
 
 // Between the host arrays' rows (staged on the device) and the batch's
-// layout, one block per system and BATCH_CHUNK bodies of it: Big bodies to
+// layout, one block per system and BATCH_CHUNK bodies of it (systems of more
+// than a million bodies: several chunks a block): Big bodies to
 // [9][nbig] at 9 big_off, particles to their slots. GATHER takes positions and
 // velocities back to rows.
-constexpr int BATCH_CHUNK = 1024;
+constexpr int BATCH_CHUNK = 1024, BATCH_CHUNK_BLOCKS = 1024;
 struct BatchRows {
     const BatchSys* sys;
     const int* body_end;      // first row past each system
-    int row0;                 // the first system's first row
+    int row0, nchunks;        // the first system's first row; BATCH_CHUNKs of the largest system
     double *x, *v;            // rows, 3 a body
     const double *m, *rce, *rphys;
     double* big;
@@ -165,8 +166,7 @@ struct BatchRows {
 template <bool GATHER> __global__ void __launch_bounds__(128) batch_rows_kernel(BatchRows A) {
     const BatchSys S = A.sys[blockIdx.x];
     const int n = A.body_end[blockIdx.x] - S.body;
-    const int j1 = min(n, (int)(blockIdx.y + 1) * BATCH_CHUNK);
-    for (int j = blockIdx.y * BATCH_CHUNK + threadIdx.x; j < j1; j += blockDim.x) {
+    auto move = [&](int j) {
         const size_t row = (size_t)(S.body - A.row0) + j;
         double* x = A.x + 3 * row;
         double* v = A.v + 3 * row;
@@ -184,7 +184,7 @@ template <bool GATHER> __global__ void __launch_bounds__(128) batch_rows_kernel(
                 d[(6 + c) * st] = 0.0;
             }
         }
-        if (GATHER) continue;
+        if (GATHER) return;
         if (is_big) {
             A.bm[S.big_off + j] = A.m[row];
             A.brce[S.big_off + j] = A.rce[row];
@@ -194,6 +194,12 @@ template <bool GATHER> __global__ void __launch_bounds__(128) batch_rows_kernel(
             A.prphys[slot] = A.rphys[row];
             A.local[slot] = q;
         }
+    };
+    for (int c = blockIdx.y; c < A.nchunks; c += gridDim.y) {
+        const int j0 = c * BATCH_CHUNK;
+        if (j0 >= n) break;
+        const int count = min(n - j0, BATCH_CHUNK);
+        for (int j = threadIdx.x; j < count; j += blockDim.x) move(j0 + j);
     }
 }
 template <bool GATHER> void launch_batch_rows(Batch& B) {
@@ -202,6 +208,7 @@ template <bool GATHER> void launch_batch_rows(Batch& B) {
     a.sys = B.d_sys.p;
     a.body_end = B.d_body_end.p;
     a.row0 = B.body_off[0];
+    a.nchunks = (int)(((long long)B.max_body + BATCH_CHUNK - 1) / BATCH_CHUNK);
     a.x = B.snap.p;
     a.v = a.x + 3 * n;
     a.m = a.v + 3 * n;
@@ -216,7 +223,7 @@ template <bool GATHER> void launch_batch_rows(Batch& B) {
     a.prce = B.prce.p;
     a.prphys = B.prphys.p;
     a.local = B.plocal.p;
-    const dim3 grid(B.nsys, (B.max_body + BATCH_CHUNK - 1) / BATCH_CHUNK);
+    const dim3 grid(B.nsys, std::min(a.nchunks, BATCH_CHUNK_BLOCKS));
     batch_rows_kernel<GATHER><<<grid, 128, 0, B.stream>>>(a);
     check(cudaGetLastError(), "batch rows");
 }
