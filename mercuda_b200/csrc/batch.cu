@@ -234,12 +234,11 @@ void layout_tables(Batch& B, int K) {
     size_t t = 0, d = 0;
     for (int s = 0; s < B.nsys; ++s) {
         const int nb = B.nbig[s] - 1;
-        B.sys[s].tab_off = (int)t;
-        B.sys[s].det_off = (int)d;
+        B.sys[s].tab_off = t;
+        B.sys[s].det_off = d;
         t += (size_t)(K + 1) * tab_stride(nb);
         d += (size_t)K * std::max(1, nb) * TAB_DETAIL;
     }
-    if (t > (size_t)INT32_MAX || d > (size_t)INT32_MAX) throw std::runtime_error("batched tables too large");
     B.tab_size = t;
     B.det_size = d;
     auto reserve = [&] {

@@ -131,8 +131,8 @@ struct BatchSys {
     double mu, h;
     int nbig, nb;
     int first_slot, np;   // the system's particle slots
-    int tab_off;          // doubles into a table set: [K + 1][tab_stride(nb)]
-    int det_off;          // doubles into a detail set: [K][nb][TAB_DETAIL]
+    size_t tab_off;       // doubles into a table set: [K + 1][tab_stride(nb)]
+    size_t det_off;       // doubles into a detail set: [K][nb][TAB_DETAIL]
     int body, big_off;    // the system's first row of the host arrays and Big-body entry
 };
 struct BatchTile {
