@@ -91,9 +91,17 @@ struct BigSmem {
     __device__ double* QT(int c, int k) const { return PT(3 + c, k); }
     __device__ double* RT(int c) const { return PT(6, 0) + c * np(); }
 };
-__host__ __device__ inline size_t big_smem_doubles(int N) {
+constexpr size_t big_smem_doubles(int N) {
     return (size_t)(17 * 3 + 5) * N + (N <= BIG_PAIR_MAX ? (size_t)(6 * N + 3) * term_row(N) + 1 : 0);
 }
+// For a launch of systems of up to N bodies: one of 33, with its pair terms, takes
+// more than one of 34 to 183 without.
+constexpr size_t big_smem_doubles_up_to(int N) {
+    const size_t largest = big_smem_doubles(N), pairs = big_smem_doubles(N < BIG_PAIR_MAX ? N : BIG_PAIR_MAX);
+    return largest > pairs ? largest : pairs;
+}
+// 512 bodies are the most that an upload takes
+static_assert(sizeof(double) * big_smem_doubles_up_to(512) <= 227 * 1024, "shared memory of a CTA");
 
 // Bodies held by the Big-body CTA (Big, then massive Small bodies).
 __device__ __forceinline__ int big_count(const MvsBigArgs& A) { return A.nmass > A.nbig ? A.nmass : A.nbig; }
@@ -1264,7 +1272,7 @@ void launch_mvs_corrector(const MvsBigArgs& big, const CorrectorArgs& a, cudaStr
 }
 
 void launch_mvs_big_batch(const BatchBigArgs& a, int nsys, int max_nbig, cudaStream_t s) {
-    const size_t smem = sizeof(double) * big_smem_doubles(max_nbig);
+    const size_t smem = sizeof(double) * big_smem_doubles_up_to(max_nbig);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(mvs_big_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (nsys > 0) mvs_big_batch_kernel<<<nsys, 32, smem, s>>>(a);
