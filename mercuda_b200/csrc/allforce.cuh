@@ -57,7 +57,7 @@ __device__ __forceinline__ Radius radius_of(const double3 x) {
     Radius R;
     R.r2 = x.x * x.x + x.y * x.y + x.z * x.z;
     sqrt_recip(R.r2, R.r, R.ri);
-    R.mid = mid_range(R.r2);
+    R.mid = root_range(R.r2);
     return R.mid ? R : radius_plain(R.r2);
 }
 

@@ -174,7 +174,7 @@ __device__ __forceinline__ double3 hkce_member_force(const BsArgs& A, int g, int
         const double q2 = q * q, q3 = q * q2, q4 = q2 * q2, q5 = q2 * q3;
         const double K = (1.0 - 10.0 * q3 + 15.0 * q4 - 6.0 * q5) * s_3;
         const double faci = (s2 <= 0.01 * rc2 ? s_3 : K) * row[3];
-        if (mid_range(s2) && mid_range(d)) {
+        if (root_range(s2) && mid_range(d)) {
             if (s2 < rc2) a = make_double3(a.x - faci * dx, a.y - faci * dy, a.z - faci * dz);
             q0 = 1;
         }
@@ -196,7 +196,7 @@ __device__ __forceinline__ double3 hkce_member_force(const BsArgs& A, int g, int
             const int i = A.adj[e].x;
             term(i, fmax(A.rcrit[i], rcrit_p));
         }
-    if (!mid_range(sc)) return hkce_central(a, x, A.f.m0);
+    if (!root_range(sc)) return hkce_central(a, x, A.f.m0);
     const double tmp2 = A.f.m0 * c_1 * c_1 * c_1;
     return make_double3(a.x - tmp2 * x.x, a.y - tmp2 * x.y, a.z - tmp2 * x.z);
 }

@@ -75,12 +75,21 @@ __device__ __forceinline__ void sqrt_near(double x, double& s, double& y) {
     const double g = x * y;
     s = fma(fma(-g, g, x), half_of(y), g);
 }
-// s = sqrt(x) rounded and r = 1/s rounded: the two roundings of 1.0 / sqrt(x).
+// s = sqrt(x) rounded and r = 1/s rounded: the two roundings of 1.0 / sqrt(x),
+// for x inside root_range().
 __device__ __forceinline__ void sqrt_recip(double x, double& s, double& r) {
     double y;
     sqrt_near(x, s, y);
     r = recip_fix(s, y);
 }
+
+// mid_range less the operands whose significand ends in 32 ones. One in 2^53
+// of them, 4^k (1 - 2^-53), has a root whose reciprocal recip_fix gets wrong: the
+// significand of the root is all ones, and the residual correction ends in the
+// middle of two doubles. The other reciprocals that lie as close to a middle as
+// the correction's error (the 53-bit factors of 2^106 - 16 .. 2^106 + 16) were
+// worked through one by one and come out right.
+__device__ __forceinline__ bool root_range(double x) { return mid_range(x) && __double2loint(x) != -1; }
 
 // The same for any operands: what is out of range takes the plain statements,
 // by a call (their code then stays out of the way of the code around).
@@ -88,7 +97,7 @@ static __device__ __noinline__ double sqrt_plain(double x) { return sqrt(x); }
 static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
 __device__ __forceinline__ void sqrt_recip_any(double x, double& s, double& r) {
     sqrt_recip(x, s, r);
-    if (!mid_range(x)) {
+    if (!root_range(x)) {
         s = sqrt_plain(x);
         r = div_plain(1.0, s);
     }

@@ -279,7 +279,7 @@ __device__ void big_force_terms(const MvsBigArgs& A, BigSmem& S, const double* V
         double s, r, rj;
         sqrt_recip(r2, s, r);
         sqrt_recip(rj2, s, rj);
-        const bool fast = mid_range(r2) && mid_range(rj2);
+        const bool fast = root_range(r2) && root_range(rj2);
         if (!fast) {
             r = div_plain(1.0, sqrt_plain(r2));
             rj = div_plain(1.0, sqrt_plain(rj2));

@@ -334,6 +334,7 @@ __device__ __forceinline__ double3 direct_terms(const double3 x, const double* r
                                                 bool* coincident = nullptr) {
     double3 a3 = make_double3(0.0, 0.0, 0.0);
     unsigned bad = 0;   // each high word less 2^-511's, ORed: below 2^30 when every s2 is within 2^-511 .. 2^513
+    unsigned low = 0;   // the largest low word (root_range)
     auto term = [&](const double* row) {
         const double2 r01 = *reinterpret_cast<const double2*>(row), r23 = *reinterpret_cast<const double2*>(row + 2);
         const double dx = x.x - r01.x, dy = x.y - r01.y, dz = x.z - r23.x;
@@ -341,6 +342,7 @@ __device__ __forceinline__ double3 direct_terms(const double3 x, const double* r
         double s, s_1;
         sqrt_recip(s2, s, s_1);
         bad |= (unsigned)__double2hiint(s2) - 0x20000000u;
+        low = max(low, (unsigned)__double2loint(s2));
         const double s_3 = s_1 * s_1 * s_1;
         const double faci = r23.y * s_3;
         return make_double3(faci * dx, faci * dy, faci * dz);
@@ -361,7 +363,7 @@ __device__ __forceinline__ double3 direct_terms(const double3 x, const double* r
     }
 #pragma unroll 1
     for (; b < nb; ++b) take(term(rows + b * ROW));
-    if (bad >= 0x40000000u) {
+    if (bad >= 0x40000000u || low == 0xffffffffu) {
         bool zero = false;
         a3 = direct_terms_plain<ROW>(x, rows, nb, &zero);
         if (coincident) *coincident = zero;
