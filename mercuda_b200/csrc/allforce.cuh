@@ -104,7 +104,7 @@ __device__ __forceinline__ double3 finish_force(double3 a, const double3 x, cons
         if (!(mj != 0.0 || g[3] == 0.0)) {
             const double sw = 0.3, yc = 1.0 / c;
             const double vr = quotient(x.x * v.x + x.y * v.y + x.z * v.z, R.r, ri);
-            const double ff = quotient(K2 * g[3], R.r * R.r, ri * ri);
+            const double ff = quotient_of(K2 * g[3], R.r * R.r, ri * ri);
             const double rad = 1.0 - quotient((1.0 + sw) * vr, c, yc);
             pr.x = ff * (quotient(rad * x.x, R.r, ri) - quotient((1.0 + sw) * v.x, c, yc));
             pr.y = ff * (quotient(rad * x.y, R.r, ri) - quotient((1.0 + sw) * v.y, c, yc));

@@ -1,9 +1,11 @@
 // Shared definitions of the B200 test-particle library.
 //
 // Every translation unit is compiled with --fmad=false and IEEE division and
-// square root, so each FP64 statement rounds exactly as the Fortran reference
-// (built with -ffp-contract=off) rounds it; the statement order of each routine
-// follows the Fortran routine it restates (cited at each function).
+// square root, and the hot paths' quotients and roots are those of fp64.cuh,
+// which round the same (its head says how far that is proven), so each FP64
+// statement rounds as the Fortran reference (built with -ffp-contract=off)
+// rounds it; the statement order of each routine follows the Fortran routine it
+// restates (cited at each function). Gradients are not bound to those roundings.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -1,5 +1,6 @@
-// Correctly rounded FP64 quotients, square roots and reciprocals without
-// branches, for operands whose exponents are known to be moderate.
+// FP64 quotients, square roots and reciprocals, rounded as IEEE division and
+// square root round them, without branches, for operands whose exponents are
+// known to be moderate.
 //
 // The compiler's IEEE division and square root are calls that begin with a
 // range test and end in a branch to a slow path; a particle-step of the MVS
@@ -12,16 +13,20 @@
 // third-order step to half an ulp, then one correction by the exact residual.
 // The value before the last rounding is within 2^-103 of the true one, so the
 // result is the IEEE one unless the true value lies that close to the middle
-// of two doubles (an exact quotient or root always comes out exact). 2^36
-// random operands and 400,000 quotients and roots made to lie next to a middle
-// gave no difference; of 14,218 operands made so for 1/sqrt one did, by an ulp.
+// of two doubles (an exact quotient or root always comes out exact). What is
+// known of those: 2^36 random operands gave no difference; the reciprocals of
+// roots that lie so close are a finite list, worked through (root_range);
+// quotients made to lie there come out right where the reciprocal is known to
+// half an ulp, and one in a hundred of them did not where it was a product of
+// reciprocals, which therefore takes one more step (quotient_of). A quotient so
+// small that its residual falls below the normal range may be an ulp off.
 // A denominator that several quotients share pays for its reciprocal once,
 // and sqrt and 1/sqrt share one seed.
 //
-// Operands must lie inside FP64_MID (about 1e-60 .. 1e60 in magnitude), so that no
-// product or residual leaves the normal range; mid_range() is the test, one
-// integer subtraction and compare. Zero, subnormal, infinite and NaN operands
-// fail it: callers then run the plain statements.
+// Operands must lie inside mid_range() (about 1e-60 .. 1e60 in magnitude), so that
+// no product or residual leaves the normal range: one integer subtraction and
+// compare. Zero, subnormal, infinite and NaN operands fail it: callers then run
+// the plain statements.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -53,12 +58,18 @@ __device__ __forceinline__ double recip_near(double b) {
 // One residual correction of y ~ 1/b (within a few ulp): 1/b rounded.
 __device__ __forceinline__ double recip_fix(double b, double y) { return fma(fma(-b, y, 1.0), y, y); }
 
-// a/b rounded, from y ~ 1/b (within a few ulp).
+// a/b rounded, from y = 1/b to half an ulp (and 2^-60): with y rounded this is
+// Markstein's theorem, and the other y that recip_near and sqrt_near leave give
+// no difference on quotients made to lie next to a middle.
 __device__ __forceinline__ double quotient(double a, double b, double y) {
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
-// a/b rounded, from an approximation q of it and y ~ 1/b.
+// a/b rounded, from y ~ 1/b (within a few ulp: a product of reciprocals). Without
+// the step on y one in a hundred quotients made to lie next to a middle is an
+// ulp off.
+__device__ __forceinline__ double quotient_of(double a, double b, double y) { return quotient(a, b, recip_fix(b, y)); }
+// a/b rounded, from a quotient q of it within an ulp and y as quotient()'s.
 __device__ __forceinline__ double quotient_fix(double a, double b, double y, double q) {
     return fma(fma(-b, q, a), y, q);
 }

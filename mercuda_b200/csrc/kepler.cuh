@@ -240,8 +240,9 @@ __device__ __forceinline__ bool drift_dan(double mu, double3& p, double3& w, dou
 // others. rr = |p|^2 and rmu ~ 1/mu (within an ulp) come from the caller. False
 // (state untouched) where drift_dan takes another branch, drift_kepmd does not
 // converge or an operand is out of range; the caller then runs drift_dan.
-// 253 FP64 and 85 other instructions against about 560 in all for the calls;
-// what bounds it is the issue of those and the length of its chain.
+// What bounds it is the issue of its FP64 instructions and the length of its
+// chain. Five of the reciprocals are products and take a step more to be known to
+// half an ulp: ten instructions, 2.59 -> 2.62 ms for 100 steps of 300,000 particles.
 __device__ __forceinline__ bool narrow_range(double x) {   // positive, exponent -100 .. 99
     return (unsigned)__double2hiint(x) - ((1023u - 100u) << 20) < (200u << 20);
 }
@@ -261,10 +262,10 @@ __device__ __forceinline__ bool drift_near(double mu, double rmu, double3& p, do
     const double asq = a * a;
     const double acu = a * asq;
     double en, yen;
-    sqrt_near(quotient(mu, acu, recip_near(acu)), en, yen);
-    const double ya = alpha * rmu;
+    sqrt_recip(quotient(mu, acu, recip_near(acu)), en, yen);
+    const double ya = recip_fix(a, alpha * rmu);
     const double ec = 1.0 - quotient(r0, a, ya);
-    const double es = quotient(u, en * asq, yen * (ya * ya));
+    const double es = quotient_of(u, en * asq, yen * (ya * ya));
     const double esq = ec * ec + es * es;
     // dt en: beyond one turn it fails the next test, and within one the whole
     // turns drift_dan takes off are none
@@ -272,7 +273,7 @@ __device__ __forceinline__ bool drift_near(double mu, double rmu, double3& p, do
     if (!(!((dm * dm > 0.16) || (esq > 0.36)) && esq * dm * dm < 0.0016)) return false;
     const double dt = quotient_fix(dm, en, yen, dt0);
     const double b = 1.0 - ec;   // r0 / a but for its rounding
-    const double fac1 = recip_fix(b, a * yr);
+    const double fac1 = recip_fix(b, recip_fix(b, a * yr));
     const double q = fac1 * dm;
     const double fac2 = es * es * fac1 - quotient(ec, 3.0, 1.0 / 3.0);
     double x = q * (1.0 - 0.5 * fac1 * q * (es - q * fac2));
@@ -298,7 +299,7 @@ __device__ __forceinline__ bool drift_near(double mu, double rmu, double3& p, do
     const double yfp = recip_near(fp);
     const double f = quotient(a, r0, yr) * (c - 1.0) + 1.0;
     const double g = dt + quotient(s - x, en, yen);
-    const double fdot = -quotient(a, r0 * fp, yr * yfp) * en * s;
+    const double fdot = -quotient_of(a, r0 * fp, yr * yfp) * en * s;
     const double gdot = quotient(c - 1.0, fp, yfp) + 1.0;
     const double3 p1 = make_double3(p.x * f + w.x * g, p.y * f + w.y * g, p.z * f + w.z * g);
     const double3 w1 = make_double3(p.x * fdot + w.x * gdot, p.y * fdot + w.y * gdot, p.z * fdot + w.z * gdot);
@@ -361,10 +362,10 @@ __device__ __forceinline__ int drift_universal(double mu, double3& p, double3& w
         const double asq = a * a;
         const double acu = a * asq;
         double en, yen;
-        sqrt_near(quotient(mu, acu, recip_near(acu)), en, yen);
+        sqrt_recip(quotient(mu, acu, recip_near(acu)), en, yen);
         const double ya = recip_near(a);
         const double ec = 1.0 - quotient(r0, a, ya);
-        const double es = quotient(u, en * asq, yen * (ya * ya));
+        const double es = quotient_of(u, en * asq, yen * (ya * ya));
         const double esq = ec * ec + es * es;
         const double turn = dt * en;
         const double dm = turn - double(int(quotient(turn, TWOPI_SWIFT, 1.0 / TWOPI_SWIFT))) * TWOPI_SWIFT;
@@ -390,7 +391,7 @@ __device__ __forceinline__ int drift_universal(double mu, double3& p, double3& w
             const double sigma = copysign(1.0, esg * cy + ec * sy);
             const double x = y + sigma * 0.85 * e;
             double sa, ysa;
-            sqrt_near(alpha, sa, ysa);
+            sqrt_recip(alpha, sa, ysa);
             s = quotient(x, sa, ysa);
         }
     } else {
@@ -458,7 +459,7 @@ __device__ __forceinline__ int drift_universal(double mu, double3& p, double3& w
     const double d = fp * r0;
     const double f = 1.0 - quotient(mu, r0, yr) * c2;
     const double g = dt - mu * c3;
-    const double fdot = -quotient(mu, d, yfp * yr) * c1;
+    const double fdot = -quotient_of(mu, d, yfp * yr) * c1;
     const double gdot = 1.0 - quotient(mu, fp, yfp) * c2;
     const double3 p1 = make_double3(p.x * f + w.x * g, p.y * f + w.y * g, p.z * f + w.z * g);
     const double3 w1 = make_double3(p.x * fdot + w.x * gdot, p.y * fdot + w.y * gdot, p.z * fdot + w.z * gdot);

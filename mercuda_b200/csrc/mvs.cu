@@ -288,7 +288,7 @@ __device__ void big_force_terms(const MvsBigArgs& A, BigSmem& S, const double* V
         const double fac0 = m[k] * r3;
         const double fac12 = m[0] * rj3;
         const double f2 = m[k] * fac12, dr = (r2 - rj2) * 0.5, mi = S.MI()[k];
-        double fac2 = quotient(f2, mi, S.TH()[k]), u = quotient(dr, rj2, rj * rj);
+        double fac2 = quotient(f2, mi, S.TH()[k]), u = quotient_of(dr, rj2, rj * rj);
         if (!(fast && mid_magnitude(mi) && (mid_magnitude(f2) || f2 == 0.0) && (mid_magnitude(dr) || dr == 0.0))) {
             fac2 = div_plain(f2, mi);
             u = div_plain(dr, rj2);

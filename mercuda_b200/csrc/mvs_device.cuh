@@ -108,8 +108,8 @@ __device__ __forceinline__ bool nongrav_near(const double3 p, const double3 u, d
     const double t2 = tx * tx + ty * ty + tz * tz;
     double tn, yt;
     sqrt_near(t2, tn, yt);
-    const double f = quotient(g[4], r2 * tn, y2 * yt);
-    if (yar_only && mid_range(r2) && mid_range(t2)) {
+    const double f = quotient_of(g[4], r2 * tn, y2 * yt);
+    if (yar_only && mid_range(r2) && mid_range(t2) && mid_magnitude(g[4])) {
         a = make_double3(f * tx, f * ty, f * tz);
         return true;
     }
