@@ -149,6 +149,38 @@ MB200_HD inline bool universal_anomaly(double r0, double sig0, double alpha, dou
     return fabs(F) <= 1e-13 * scale;
 }
 
+// The universal anomaly s of the drift of (x, v) by dt that ended at x1, and its
+// G functions. Returns 0 if it did not converge, 1 if it was iterated, 2 if one
+// step from the guess sufficed.
+MB200_HD inline int drift_anomaly(const double x[3], const double v[3], const double x1[3], double r0, double ir0,
+                                  double sig0, double alpha, double mu, double imu, double dt, double& s,
+                                  double G[6]) {
+    s = anomaly_guess(x, v, x1, r0, ir0, sig0, alpha, mu, imu, dt);
+    gfuncs(s, alpha, G);
+    // One Newton step, and the G functions moved along it by dG_k/ds = G_{k-1}
+    // to second order, where its own remainder F'' ds^2 / 2F' is below a rounding
+    // of s and the third order is too: the usual guess is that good. A poor one
+    // (orbits that are nearly radial) goes through the iteration.
+    const double F = fma(r0, G[1], fma(sig0, G[2], fma(mu, G[3], -dt)));
+    const double F1 = fma(r0, G[0], fma(sig0, G[1], mu * G[2]));
+    const double F2 = fma(sig0, G[0], fma(-alpha, r0, mu) * G[1]);
+    const double ds = -F * adj_recip(F1);
+    if (fabs(ds) <= 1e-7 * fabs(s) && fabs(F2 * ds) * fabs(ds) <= 2e-16 * fabs(F1 * s)) {
+        const double d2 = 0.5 * ds * ds, Gm1 = -alpha * G[1], Gm2 = -alpha * G[0];
+        G[5] += fma(ds, G[4], d2 * G[3]);
+        G[4] += fma(ds, G[3], d2 * G[2]);
+        G[3] += fma(ds, G[2], d2 * G[1]);
+        G[2] += fma(ds, G[1], d2 * G[0]);
+        G[1] += fma(ds, G[0], d2 * Gm1);
+        G[0] += fma(ds, Gm1, d2 * Gm2);
+        s += ds;
+        return 2;
+    }
+    if (!universal_anomaly(r0, sig0, alpha, mu, dt, s)) return 0;
+    gfuncs(s, alpha, G);
+    return 1;
+}
+
 // lx = d(x')/dx ^T lx1 + d(v')/dx ^T lv1, lv likewise, for the drift of
 // (x, v) by dt about mu that ended at x1. Returns false if the anomaly did not
 // converge.
@@ -164,27 +196,8 @@ MB200_HD inline bool drift_vjp(double mu, const double x[3], const double v[3], 
 #endif
     const double imu = adj_recip(mu);
     const double alpha = fma(2.0 * mu, ir0, -dot3(v, v));
-    double s = anomaly_guess(x, v, x1, r0, ir0, sig0, alpha, mu, imu, dt);
-    double G[6];
-    gfuncs(s, alpha, G);
-    // one Newton step, and the G functions moved along it by dG_k/ds = G_{k-1}
-    // to second order: with the usual guess the third is far below a rounding;
-    // a poor one goes through the iteration
-    const double F = fma(r0, G[1], fma(sig0, G[2], fma(mu, G[3], -dt)));
-    const double ds = -F * adj_recip(fma(r0, G[0], fma(sig0, G[1], mu * G[2])));
-    if (fabs(ds) <= 1e-7 * fabs(s)) {
-        const double d2 = 0.5 * ds * ds, Gm1 = -alpha * G[1], Gm2 = -alpha * G[0];
-        G[5] += fma(ds, G[4], d2 * G[3]);
-        G[4] += fma(ds, G[3], d2 * G[2]);
-        G[3] += fma(ds, G[2], d2 * G[1]);
-        G[2] += fma(ds, G[1], d2 * G[0]);
-        G[1] += fma(ds, G[0], d2 * Gm1);
-        G[0] += fma(ds, Gm1, d2 * Gm2);
-        s += ds;
-    } else {
-        if (!universal_anomaly(r0, sig0, alpha, mu, dt, s)) return false;
-        gfuncs(s, alpha, G);
-    }
+    double s, G[6];
+    if (!drift_anomaly(x, v, x1, r0, ir0, sig0, alpha, mu, imu, dt, s, G)) return false;
     const double r = fma(r0, G[0], fma(sig0, G[1], mu * G[2]));
     const double ir = adj_recip(r), irr = ir * ir0;
     const double f = fma(-mu * G[2], ir0, 1.0);
