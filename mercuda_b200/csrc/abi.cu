@@ -2560,9 +2560,11 @@ int mercury_b200_mvs_advance(double time, double h, int nsteps, double rcen, int
         K = std::min(K, mvs_max_steps_per_launch(nb));
         K = std::max(1, std::min(K, nsteps));
         // launch sizes: K steps each; with the automatic choice the first launch
-        // is short, so that its Big-body steps (one CTA, serial, ~20 us a step)
-        // hold up the particles briefly and the next launch's Big-body steps run
-        // beside its particles
+        // is short, so that its Big-body steps (one CTA, serial, 5.2 us a step of
+        // eight planets) hold up the particles briefly and the next launch's
+        // Big-body steps run beside its particles. 20 steps of 1M particles: 1.16 ms
+        // without a short launch, 1.11 with a tenth of K, 1.10 with a fifth, 1.16
+        // with a third; 100 steps of 300,000: 2.62, 2.55, 2.51 and 2.58.
         std::vector<int>& ksz = c.launch_steps;
         ksz.clear();
         {

@@ -31,7 +31,12 @@
 namespace mb200 {
 namespace {
 
-constexpr int ADJ_CTAS = 6;  // of 128 threads an SM (80 registers): 100,000 particles in one wave
+// CTAs of 128 threads an SM (80 registers). What a segment ends with is its
+// slowest particle's serial chain, and a smaller bound shortens that while the
+// rest fits anyway: forward and backward of 100,000 particles, 1,000 steps, 9.8 +
+// 10.4 ms with 4, 10.5 + 10.7 with 6, 11.0 + 10.7 with 8; of 400,000, 300 steps,
+// 6.8 + 12.0, 6.6 + 11.9 and 6.8 + 11.9.
+constexpr int ADJ_CTAS = 6;
 constexpr int REC = 12;  // per step of a segment: x, v after the kick (drift input), x, v after the drift
 
 struct AdjArgs {

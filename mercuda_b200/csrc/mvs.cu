@@ -734,7 +734,10 @@ __device__ __forceinline__ unsigned overlap_mask(const int4* keys, int n, int kx
             : "+r"(mask)
             : "r"(k.y), "r"(kxlo), "r"(kxhi), "r"(k.x), "r"(k.w), "r"(kylo), "r"(kyhi), "r"(k.z), "r"(bit));
     };
-    if (n == 8) {   // the usual planetary system, without a loop
+    // the usual planetary system without a loop, whose counter and branches are
+    // 2.5 % of the kernel (1M particles, 160 steps: 8.78 ms so, 9.00 with the loop,
+    // 8.90 with it unrolled by four)
+    if (n == 8) {
 #pragma unroll
         for (int b = 0; b < 8; ++b) test(b, 1u << b);
     } else {
@@ -1218,11 +1221,10 @@ void launch_variant(const MvsParticleArgs& a, cudaStream_t s, int threads) {
         room.smem = smem;
         room.slots = sms * (per_sm < 1 ? 1 : per_sm);
     }
-    // One CTA slot fewer than the device holds, so that the Big-body CTA of
-    // the next chunk (another stream) can start beside this persistent grid.
-    int slots = room.slots - 1;
-    if (slots < 1) slots = 1;
-    const int grid = tiles < slots ? tiles : slots;
+    // All of them: the Big-body CTA of the next launch (another stream) needs
+    // 38,912 registers, so it starts as these drain, and leaving one slot free
+    // for it changes nothing (1M particles, 160 steps: 8.78 ms with, 8.79 without).
+    const int grid = tiles < room.slots ? tiles : room.slots;
     if (grid > 0) kern<<<grid, threads, smem, s>>>(a);
 }
 
