@@ -359,14 +359,18 @@ void particles_and_events(const MvsParticleArgs& pa, const double* detail, cudaS
     if (!fresh) check(cudaMemsetAsync(&pa.status->cands, 0, sizeof(int), s), "memset");
 }
 
-// Candidate room for a launch of `steps` steps: box overlaps run at 2-4 % of
-// the particles per step on a system with 1 % of its particles near planets,
-// so steps x np / 25, kept from one run to the next (not with a fixed
-// starting capacity set for tests, which exercise the overflow path).
+// Candidate room for a launch of `steps` steps: box overlaps run at 2 to 4.3 %
+// of the particles per step on systems with 1 % of their particles near planets,
+// so 5 % a step, up to the 4 % that a launch of the most steps needs on average;
+// kept from one run to the next (not with a fixed starting capacity set for
+// tests, which exercise the overflow path). With 4 % of 25 steps, one first run
+// in three of 1M particles overflowed and was made again (28 ms of 457 steps).
 void ensure_candidates(int steps) {
     Context& c = ctx();
     if (g_event_cap > 0) return;
-    const size_t want = (size_t)std::max(1, steps) * (size_t)c.np / 25 + 16384;
+    const size_t np = (size_t)c.np;
+    const size_t want = std::min((size_t)std::max(1, steps) * np / 20,
+                                 (size_t)mvs_max_steps_per_launch(c.nbig - 1) * np / 25) + 16384;
     if (c.cands.n < want) c.cands.reserve(want);
 }
 
