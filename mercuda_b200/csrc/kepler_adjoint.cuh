@@ -176,7 +176,15 @@ MB200_HD inline int drift_anomaly(const double x[3], const double v[3], const do
         s += ds;
         return 2;
     }
-    if (!universal_anomaly(r0, sig0, alpha, mu, dt, s)) return 0;
+    // The guess of a radial orbit is a quotient of roundings (x x v is not zero with
+    // fused products where v is a power of two times x) and may lie too far off.
+    bool found = false;
+#pragma unroll 1
+    for (int start = 0; start < 2 && !found; ++start) {
+        if (start == 1) s = dt * ir0;
+        found = universal_anomaly(r0, sig0, alpha, mu, dt, s);
+    }
+    if (!found) return 0;
     gfuncs(s, alpha, G);
     return 1;
 }
