@@ -44,6 +44,8 @@ def test_adjoint_record_buffers(cuda_lib):
         g = torch.autograd.grad((xf ** 2).sum() + (vf ** 2).sum(), t)
         return [q.detach().cpu() for q in (xf, vf, *g)]
 
+    cuda_lib.mercury_b200_adjoint_free()   # what an earlier test's run left
+    torch.cuda.empty_cache()
     free0 = torch.cuda.mem_get_info()[0]
     roomy = run()
     assert free0 - torch.cuda.mem_get_info()[0] > 4 * 8 * 12 * 8 * 300_000
