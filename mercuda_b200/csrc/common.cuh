@@ -66,8 +66,8 @@ __device__ __forceinline__ void raise_fault(DeviceStatus* st, int bit) { atomicO
 // choice, 3568-3596): the BS2 attempt kernels read the trial step h0 here;
 // the post-attempt kernel takes each attempt's decision, advances the local
 // clock into the next attempt's copy (two copies alternate), and commits and
-// screens only after an acceptance. The host reads it back every few dozen
-// attempts.
+// screens only after an acceptance. The host watches a progress word and reads
+// this back once, at the end.
 struct EncCtl {
     double h0;          // trial step of the next attempt
     double hdid;        // step of the last accepted substep

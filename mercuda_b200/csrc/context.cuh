@@ -209,8 +209,8 @@ struct Context {
     // already (head_count records)
     bool head_ready = false;
     int head_count = 0;
-    // the encounter subsystem's step control, read back once per block of
-    // attempts
+    // the encounter subsystem's step control as it begins, and read back once
+    // at the end
     EncCtl* enc_host = nullptr;
     int2* enc_progress = nullptr;   // written by the device, read by the host
     // the encounter subsystem's step control on the device (two copies that

@@ -759,12 +759,10 @@ __device__ __forceinline__ unsigned overlap_mask(const int4* keys, int n, int kx
 // key(b) - 1), and x at the step's start, |x|^2 and x.v come from the step
 // before. What passes is tested with mce_box's and mce_cent's own statements.
 // The kernel issues an FP64 instruction every other cycle and another kind in
-// between (on particles that all take drift_kepmd's path it fits 1.8 cycles
-// for each FP64 instruction and 1.4 for any other), so both kinds count. Per
-// warp-step, 8 planets: 563 FP64 of 1,138 instructions with exact boxes
-// compared on the FP64 pipe and IEEE division calls, 497 of 944 so; 1M
-// particles, 16 steps: 1.19 ms a launch before, 0.75 now, and with the
-// benchmark's mixture of orbits 1.52 ms and 0.89.
+// between, so both kinds count. Per warp-step of the benchmark's mixture of
+// orbits, 8 planets: 729 FP64 of 1,535 instructions with exact boxes compared on
+// the FP64 pipe and IEEE division calls, 564 of 1,116 so; 1M particles, 16 steps:
+// 1.45 ms a launch before, 0.93 now.
 template <bool NGF, bool OBL, bool CENTRAL, int ROW, class Cols, class Found, class Struck>
 __device__ __forceinline__ void particle_step(Particle& P, bool ok, const Cols& cols, const double* T,
                                               const double* G, const StepEnv& E, const double* jcen,
