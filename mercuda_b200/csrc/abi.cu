@@ -402,7 +402,7 @@ void grow_after_overflow() {
 //
 // The Big bodies never feel the particles, so the Big-body step after the
 // speculative one runs on a third stream beside the speculative particles
-// (in the CTA slot the particle grid leaves free), and the next speculative
+// (where their grid leaves room, or as it drains), and the next speculative
 // step starts from its output: the particles' step is then the only kernel
 // on the critical path of a step.
 //

@@ -207,7 +207,7 @@ static __device__ void row_head(const double* X, const double* m, const ForceCfg
 // nothing depends on which bodies act on which); one thread per body finishes
 // with the central terms. The same roundings in the same order as the loops
 // above. Eight planets, a call of RADAU: 4.6 us with sums in one thread and
-// division calls, 2.1 us so.
+// division calls, 1.9 us so.
 constexpr int MASSIVE_PAR_MAX = 32;
 __host__ __device__ constexpr int massive_rows_doubles(int N) {
     return N <= MASSIVE_PAR_MAX ? (3 * N + 6) * term_row(N) + 5 * N + 1 : 0;

@@ -370,7 +370,7 @@ template <bool STAGED> __global__ void __launch_bounds__(256) ra15_massive_kerne
 // coordinate) keeps its B, G, a1, x1 and v1 in registers for the whole
 // sequence, and each force call is massive_rows_call. What bounds it is the
 // chain of 15 (43 at a start) force calls; the particles wait for it. Eight
-// planets: 70 us a sequence by the kernel above, 31 us so.
+// planets: 70 us a sequence by the kernel above, 28 us so.
 __global__ void __launch_bounds__(256) ra15_massive_rows_kernel(const __grid_constant__ Ra15Args A) {
     extern __shared__ double sm[];
     const ForceCfg& f = A.f;
@@ -439,8 +439,8 @@ __global__ void __launch_bounds__(256) ra15_massive_rows_kernel(const __grid_con
 // Three CTAs of 128 per SM (at most 168 registers, a few spilled words): 12
 // warps per SM hide the FP64 dependency chains better than the 8 the
 // unbounded 194-register build fits (0.361 -> 0.322 ms per step at 100k). With
-// the branch-free force the kernel takes 113 us a sequence (149 with division
-// calls); 2 CTAs 114, 4 CTAs 148.
+// the branch-free force the kernel takes 96 us a sequence (149 with division
+// calls); when it took 113, 2 CTAs took 114 and 4 CTAs 148.
 constexpr int RA15_PARTICLE_THREADS = 128;
 __global__ void __launch_bounds__(RA15_PARTICLE_THREADS, 3) ra15_particle_kernel(Ra15Args A) {
     const ForceCfg& f = A.f;
